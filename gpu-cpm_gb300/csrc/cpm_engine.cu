@@ -141,6 +141,12 @@ struct cpm_handle {
   int graph_launches = 1;  // sweep kernels per replay (2 for hybrid)
   cudaStream_t graph_stream = nullptr;
 
+  // Scratch of the synchronous seeding and measuring calls, grown on demand
+  // and freed with the handle (an allocation per call costs more than their
+  // kernels on small lattices).
+  char* d_scratch = nullptr;
+  size_t scratch_cap = 0;
+
   uint64_t seed = 0;
   uint32_t stream_id = 0;
   uint64_t tick = 0;
@@ -212,6 +218,7 @@ void free_all(cpm_handle* h) {
   cudaFree(h->d_hyb_prefix);
   cudaFree(h->d_rep_order);
   cudaFree(h->d_tick);
+  cudaFree(h->d_scratch);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
 }
@@ -615,6 +622,18 @@ int set_adhesion(cpm_handle* h, int r, int type, int other, float J, int sym) {
     p.J[type * kMaxTypes + other] = J;
     if (sym) p.J[other * kMaxTypes + type] = J;
   });
+}
+
+// At least `bytes` of scratch at h->d_scratch.  Its users wait for the stream
+// before they return, so nothing in flight holds the old one.
+int ensure_scratch(cpm_handle* h, size_t bytes) {
+  if (bytes <= h->scratch_cap) return CPM_OK;
+  cudaFree(h->d_scratch);
+  h->d_scratch = nullptr;
+  h->scratch_cap = 0;
+  CPM_CUDA(h, cudaMalloc((void**)&h->d_scratch, bytes));
+  h->scratch_cap = bytes;
+  return CPM_OK;
 }
 
 int read_error_word(cpm_handle* h, uint32_t* word) {
@@ -1578,20 +1597,30 @@ int cpm_observe_heterotypic(cpm_handle* h, float* out_host) {
   CPM_BIND(h);
   if (h->ndim != 2) return h->fail(CPM_ERR_UNSUPPORTED, "2D engines only");
   if (!out_host) return h->fail(CPM_ERR_INVALID, "out_host is NULL");
-  unsigned long long* counts = nullptr;
-  CPM_CUDA(h, cudaMallocAsync((void**)&counts, sizeof(unsigned long long) * 2 * h->nrep,
-                              h->stream));
-  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * 2 * h->nrep, h->stream);
+  // [nrep + 1] first tasks, then [2 nrep] counts, in one buffer
+  std::vector<long long> start(h->nrep + 1, 0);
+  for (int r = 0; r < h->nrep; ++r) {
+    const DevReplica& R = h->reps[r];
+    start[r + 1] = start[r] + ((R.nx + 31LL) / 32) * ((R.ny + kObserveRows - 1LL) / kObserveRows);
+  }
+  const size_t start_b = sizeof(long long) * (h->nrep + 1),
+               counts_b = sizeof(unsigned long long) * 2 * h->nrep;
+  if (int rc = ensure_scratch(h, start_b + counts_b)) return rc;
+  char* buf = h->d_scratch;
+  unsigned long long* counts = reinterpret_cast<unsigned long long*>(buf + start_b);
+  cudaError_t e = cudaMemcpyAsync(buf, start.data(), start_b, cudaMemcpyHostToDevice, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, counts_b, h->stream);
   if (e == cudaSuccess)
-    e = launch_observe_heterotypic(h->d_lat, h->d_reps, h->nrep, h->total_sites, counts,
-                                   h->stream);
+    e = launch_observe_heterotypic(h->d_lat, h->d_reps, h->nrep,
+                                   reinterpret_cast<const long long*>(buf), start[h->nrep],
+                                   counts, h->stream);
   h->launches += 1;
   std::vector<unsigned long long> c(2 * h->nrep);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(c.data(), counts, sizeof(unsigned long long) * 2 * h->nrep,
-                        cudaMemcpyDeviceToHost, h->stream);
-  cudaFreeAsync(counts, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    e = cudaMemcpyAsync(c.data(), counts, counts_b, cudaMemcpyDeviceToHost, h->stream);
+  // (also on an error: the copies read and write this frame's vectors)
+  const cudaError_t e2 = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_observe_heterotypic");
   for (int r = 0; r < h->nrep; ++r)
     out_host[r] = c[2 * r] ? (float)((double)c[2 * r + 1] / (double)c[2 * r]) : 0.0f;
@@ -1625,19 +1654,30 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   const double sites = (double)n[0] * n[1] * n[2];
   const double side = std::pow(2.0 * sites / npoints, 1.0 / nd);
   long long G = 1;
-  double wmin = 1e300;
+  double wmin = 1e300, wmax = 0.0, w[3];
   vg.rmax = 0;
+  int nmax = 1;
   for (int a = 0; a < 3; ++a) {
     vg.n[a] = n[a];
     int g = a < nd ? (int)std::lround((double)n[a] / side) : 1;
     g = std::max(1, std::min(g, n[a]));
     vg.g[a] = g;
-    vg.w[a] = (double)n[a] / g;
-    if (a < nd) wmin = std::min(wmin, vg.w[a]);
+    w[a] = (double)n[a] / g;
+    vg.wf[a] = (float)w[a];
+    vg.inv_w[a] = (float)(1.0 / w[a]);
+    if (a < nd) {
+      wmin = std::min(wmin, w[a]);
+      wmax = std::max(wmax, w[a]);
+      nmax = std::max(nmax, n[a]);
+    }
     vg.rmax = std::max(vg.rmax, g / 2 + 1);
     G *= g;
   }
-  vg.lb_scale = wmin;
+  vg.lb_scale = (float)wmin;
+  // Coordinates and differences of up to nmax, each rounded to FP32 (relative
+  // 2^-24): at most 8 roundings per axis, up to sqrt(3) of it in a distance,
+  // and a few more of the squares and the square root.
+  vg.ferr = (float)(24.0 * nmax * 0x1p-24);
   if (G > (1LL << 30))
     return h->fail(CPM_ERR_INVALID, "cpm_seed_voronoi_r: too many buckets");
   // Counting sort of the points by bucket (host; O(npoints)).
@@ -1645,7 +1685,7 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   for (int k = 0; k < npoints; ++k) {
     long long b = 0;
     for (int a = nd - 1; a >= 0; --a) {
-      int ba = (int)std::floor(points[(size_t)k * nd + a] / vg.w[a]);
+      int ba = (int)std::floor(points[(size_t)k * nd + a] / w[a]);
       ba = std::max(0, std::min(ba, vg.g[a] - 1));
       b = b * vg.g[a] + ba;
     }
@@ -1656,42 +1696,55 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   // Work bound.  A site's search ends within about (d + 1) sqrt(ndim)
   // max(w) / min(w) + 1 rings, d the Chebyshev distance (in buckets, wrapped)
   // from its bucket to the nearest occupied one; d comes from a breadth-first
-  // search over the bucket grid.  Point sets clustered so much that the
-  // search would run for seconds are refused instead of launched.
+  // search over the bucket grid (its first step from the empty buckets, which
+  // are the fewer: of evenly spread points one bucket in eight is empty).
+  // Point sets clustered so much that the search would run for seconds are
+  // refused instead of launched.
   {
     std::vector<int> dist(G, -1), frontier, next;
+    auto neighbours = [&](int b, auto&& f) {  // f(b2) for the wrapped neighbours
+      const int bx = b % vg.g[0], by = (b / vg.g[0]) % vg.g[1], bz = b / (vg.g[0] * vg.g[1]);
+      for (int dz = (nd == 3 ? -1 : 0); dz <= (nd == 3 ? 1 : 0); ++dz)
+        for (int dy = -1; dy <= 1; ++dy)
+          for (int dx = -1; dx <= 1; ++dx) {
+            const int x2 = (bx + dx + vg.g[0]) % vg.g[0], y2 = (by + dy + vg.g[1]) % vg.g[1],
+                      z2 = (bz + dz + vg.g[2]) % vg.g[2];
+            f((z2 * vg.g[1] + y2) * vg.g[0] + x2);
+          }
+    };
     for (long long b = 0; b < G; ++b)
-      if (start[b + 1] > start[b]) {
-        dist[b] = 0;
-        frontier.push_back((int)b);
-      }
-    for (int d = 1; !frontier.empty(); ++d) {
+      if (start[b + 1] > start[b]) dist[b] = 0;
+    for (long long b = 0; b < G; ++b) {
+      if (dist[b] >= 0) continue;
+      bool near = false;
+      neighbours((int)b, [&](int b2) { near = near || dist[b2] == 0; });
+      if (near) frontier.push_back((int)b);
+    }
+    for (int b : frontier) dist[b] = 1;
+    for (int d = 2; !frontier.empty(); ++d) {
       next.clear();
-      for (int b : frontier) {
-        const int bx = b % vg.g[0], by = (b / vg.g[0]) % vg.g[1], bz = b / (vg.g[0] * vg.g[1]);
-        for (int dz = (nd == 3 ? -1 : 0); dz <= (nd == 3 ? 1 : 0); ++dz)
-          for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-              const int x2 = (bx + dx + vg.g[0]) % vg.g[0], y2 = (by + dy + vg.g[1]) % vg.g[1],
-                        z2 = (bz + dz + vg.g[2]) % vg.g[2];
-              const int b2 = (z2 * vg.g[1] + y2) * vg.g[0] + x2;
-              if (dist[b2] < 0) {
-                dist[b2] = d;
-                next.push_back(b2);
-              }
-            }
-      }
+      for (int b : frontier)
+        neighbours(b, [&](int b2) {
+          if (dist[b2] < 0) {
+            dist[b2] = d;
+            next.push_back(b2);
+          }
+        });
       frontier.swap(next);
     }
-    double wmax = 0.0;
-    for (int a = 0; a < nd; ++a) wmax = std::max(wmax, vg.w[a]);
     const double per_bucket_sites = sites / (double)G;
     const double per_bucket_points = (double)npoints / (double)G;
-    double work = 0.0;  // estimated distance evaluations
+    std::vector<long long> at_dist;  // buckets at each distance
     for (long long b = 0; b < G; ++b) {
-      const double rings =
-          std::min((double)vg.rmax, (dist[b] + 1) * std::sqrt((double)nd) * wmax / wmin + 1.0);
-      work += per_bucket_sites * std::pow(2.0 * rings + 1.0, nd) * std::max(1.0, per_bucket_points);
+      if ((size_t)dist[b] >= at_dist.size()) at_dist.resize(dist[b] + 1, 0);
+      ++at_dist[dist[b]];
+    }
+    double work = 0.0;  // estimated distance evaluations
+    for (size_t d = 0; d < at_dist.size(); ++d) {
+      const double rings = std::min(
+          (double)vg.rmax, ((double)d + 1.0) * std::sqrt((double)nd) * wmax / wmin + 1.0);
+      work += (double)at_dist[d] * per_bucket_sites * std::pow(2.0 * rings + 1.0, nd) *
+              std::max(1.0, per_bucket_points);
     }
     if (work > 5e11)
       return h->fail(CPM_ERR_INVALID,
@@ -1699,40 +1752,37 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
                      "search (about %.3g distance evaluations); spread them more evenly or "
                      "label the lattice on the host", work);
   }
-  std::vector<double> pts((size_t)npoints * 3, 0.0);
-  std::vector<int> idx(npoints), fill(start.begin(), start.end() - 1);
+  // One upload: FP32 points, double points, original indices, values, starts.
+  const size_t np = (size_t)npoints;
+  const size_t off_p = sizeof(float4) * np, off_i = off_p + sizeof(double) * 3 * np,
+               off_v = off_i + sizeof(int) * np, off_s = off_v + sizeof(uint32_t) * np,
+               bytes = off_s + sizeof(int) * (size_t)(G + 1);
+  std::vector<char> up(bytes);
+  float4* fpts = reinterpret_cast<float4*>(up.data());
+  double* pts = reinterpret_cast<double*>(up.data() + off_p);
+  int* idx = reinterpret_cast<int*>(up.data() + off_i);
+  std::vector<int> fill(start.begin(), start.end() - 1);
   for (int k = 0; k < npoints; ++k) {
     const int slot = fill[bucket_of[k]]++;
-    for (int a = 0; a < nd; ++a) pts[(size_t)slot * 3 + a] = points[(size_t)k * nd + a];
+    double c[3] = {0.0, 0.0, 0.0};
+    for (int a = 0; a < nd; ++a) c[a] = points[(size_t)k * nd + a];
+    for (int a = 0; a < 3; ++a) pts[(size_t)slot * 3 + a] = c[a];
+    fpts[slot] = make_float4((float)c[0], (float)c[1], (float)c[2], 0.0f);
     idx[slot] = k;
   }
-  double* d_pts = nullptr;
-  int *d_idx = nullptr, *d_start = nullptr;
-  uint32_t* d_val = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_pts, sizeof(double) * pts.size(), h->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_idx, sizeof(int) * npoints, h->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_val, sizeof(uint32_t) * npoints, h->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_start, sizeof(int) * (G + 1), h->stream);
+  std::memcpy(up.data() + off_v, values, sizeof(uint32_t) * np);
+  std::memcpy(up.data() + off_s, start.data(), sizeof(int) * (size_t)(G + 1));
+  if (int rc = ensure_scratch(h, bytes)) return rc;
+  char* dev = h->d_scratch;
+  cudaError_t e = cudaMemcpyAsync(dev, up.data(), bytes, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_pts, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice,
-                        h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_idx, idx.data(), sizeof(int) * npoints, cudaMemcpyHostToDevice,
-                        h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_val, values, sizeof(uint32_t) * npoints, cudaMemcpyHostToDevice,
-                        h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_start, start.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice,
-                        h->stream);
-  if (e == cudaSuccess)
-    e = launch_voronoi(h->d_lat + R.lat_off, vg, d_pts, d_idx, d_val, d_start, h->stream);
+    e = launch_voronoi(h->d_lat + R.lat_off, vg, reinterpret_cast<const double*>(dev + off_p),
+                       reinterpret_cast<const float4*>(dev),
+                       reinterpret_cast<const int*>(dev + off_i),
+                       reinterpret_cast<const uint32_t*>(dev + off_v),
+                       reinterpret_cast<const int*>(dev + off_s), h->stream);
   h->launches += 1;
-  cudaFreeAsync(d_pts, h->stream);
-  cudaFreeAsync(d_idx, h->stream);
-  cudaFreeAsync(d_val, h->stream);
-  cudaFreeAsync(d_start, h->stream);
-  // the host vectors are read by the copies: wait before they go
+  // the host buffer is read by the copy: wait before it goes
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_seed_voronoi_r");
   if (e2 != cudaSuccess) return h->cuda_fail(e2, "cpm_seed_voronoi_r");
@@ -1753,24 +1803,19 @@ int cpm_observe_boundaries(cpm_handle* h, int ntypes, uint64_t* out_host) {
   }
   const long long ntiles = tile_start[h->nrep];
   const size_t nc = (size_t)h->nrep * ntypes * ntypes;
-  unsigned long long* counts = nullptr;
-  long long* d_ts = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&counts, sizeof(unsigned long long) * nc, h->stream);
+  const size_t ts_b = sizeof(long long) * (h->nrep + 1), counts_b = sizeof(uint64_t) * nc;
+  if (int rc = ensure_scratch(h, ts_b + counts_b)) return rc;
+  long long* d_ts = reinterpret_cast<long long*>(h->d_scratch);
+  unsigned long long* counts = reinterpret_cast<unsigned long long*>(h->d_scratch + ts_b);
+  cudaError_t e = cudaMemsetAsync(counts, 0, counts_b, h->stream);
   if (e == cudaSuccess)
-    e = cudaMallocAsync((void**)&d_ts, sizeof(long long) * (h->nrep + 1), h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(unsigned long long) * nc, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_ts, tile_start.data(), sizeof(long long) * (h->nrep + 1),
-                        cudaMemcpyHostToDevice, h->stream);
+    e = cudaMemcpyAsync(d_ts, tile_start.data(), ts_b, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess)
     e = launch_observe_boundaries(h->ndim, h->d_lat, h->d_reps, h->nrep, d_ts, ntiles, ntypes,
                                   counts, h->stream);
   h->launches += 1;
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(out_host, counts, sizeof(unsigned long long) * nc,
-                        cudaMemcpyDeviceToHost, h->stream);
-  cudaFreeAsync(counts, h->stream);
-  cudaFreeAsync(d_ts, h->stream);
+    e = cudaMemcpyAsync(out_host, counts, counts_b, cudaMemcpyDeviceToHost, h->stream);
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_observe_boundaries");
   if (e2 != cudaSuccess) return h->cuda_fail(e2, "cpm_observe_boundaries");

@@ -294,24 +294,31 @@ cudaError_t launch_persist_update(double* prefdir, double* hist, int H, int slot
                                   const int* ctype, const DevParams* params,
                                   const DevReplica* reps, int nrep, long long rows,
                                   cudaStream_t s);
+// Pair counts of 2D replicas; start: per replica its first task of 32 columns
+// by kObserveRows rows (nrep + 1 entries, device memory), ntasks = start[nrep].
+constexpr int kObserveRows = 16;
 cudaError_t launch_observe_heterotypic(const uint32_t* lat, const DevReplica* reps,
-                                       int nrep, long long total_sites,
+                                       int nrep, const long long* start, long long ntasks,
                                        unsigned long long* counts, cudaStream_t s);
 // Periodic Voronoi seeding of one lattice region (nx*ny*nz sites at `lat`):
 // every site takes values[k] of its nearest point (min-image Euclidean
 // distance in double, ties to the lowest k).  Points are binned in a
 // g[0]*g[1]*g[2] bucket grid of widths w[] (bucket-major order: pts[k*3+a],
-// idx[k] their original index, start[b]..start[b+1] bucket b's points).
+// idx[k] their original index, start[b]..start[b+1] bucket b's points; fpts[k]
+// the same coordinates in FP32).
 struct VoronoiGrid {
   int n[3];         // lattice sides (n[2] = 1 in 2D)
   int g[3];         // buckets per axis
-  double w[3];      // bucket widths n / g
-  double lb_scale;  // min(w): ring r bounds unscanned points at r * min(w)
+  float inv_w[3];   // buckets per unit length, g / n
+  float wf[3];      // bucket widths n / g
+  float lb_scale;   // min(w): ring r bounds unscanned points at r * min(w)
+  float ferr;       // bound on the error of a distance (and of a position) in FP32
   int ndim;
   int rmax;         // rings to scan at most (covers every bucket)
 };
 cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, const double* pts,
-                           const int* idx, const uint32_t* values, const int* start,
+                           const float4* fpts, const int* idx, const uint32_t* values,
+                           const int* start,
                            cudaStream_t s);
 // Boundary counts per replica and unordered type pair: Moore pairs (each
 // once) of sites with different values, counts[r*T*T + a*T + b] for a <= b

@@ -1174,38 +1174,91 @@ __global__ void persist_update_kernel(double* prefdir, double* hist, int H, int 
 // Per replica: number of Moore neighbour pairs (each pair once) of two
 // different non-medium cells, and how many of them join cells of different
 // types.  counts[2 r] = all such pairs, counts[2 r + 1] = heterotypic ones.
-__global__ void observe_heterotypic_kernel(const uint32_t* __restrict__ lat,
-                                           const DevReplica* __restrict__ reps, int nrep,
-                                           long long total,
-                                           unsigned long long* counts) {
-  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (long long)gridDim.x * blockDim.x) {
-    const int r = find_site_replica(reps, nrep, g);
-    const DevReplica R = reps[r];
-    const long long local = g - R.lat_off;
-    const int x = (int)(local % R.nx), y = (int)((local / R.nx) % R.ny);
-    const uint32_t v = lat[g];
-    unsigned pairs = 0, hetero = 0;
-    if (v & 0xFFFFFFu) {
-      // forward half of the Moore neighbourhood: (0,1), (1,-1), (1,0), (1,1)
-      const int dys[4] = {0, 1, 1, 1}, dxs[4] = {1, -1, 0, 1};
+//
+// A warp takes tasks of 32 columns x kObserveRows rows of one replica (`start`:
+// tasks before each replica): a lane walks its column, so the row below's
+// three loads are the next row's centre and right neighbour.  Bound: reading
+// the lattice.  Counts stay in registers from task to task, then in shared
+// memory for the block's first replica (its tasks are one contiguous run),
+// so a block issues two global atomics per replica it meets.  (One 64-bit
+// atomic pair per counted site, on two addresses per replica, took 1.18 ms on
+// a 2048^2 tissue and ~10 ms on 256 replicas of 45.5 M sites together.)
+__global__ void __launch_bounds__(256)
+    observe_heterotypic_kernel(const uint32_t* __restrict__ lat,
+                               const DevReplica* __restrict__ reps, int nrep,
+                               const long long* __restrict__ start,
+                               unsigned long long* counts) {
+  __shared__ unsigned long long s_sum[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  if (threadIdx.x < 2) s_sum[threadIdx.x] = 0ull;
+  __syncthreads();
+  const long long ntasks = __ldg(start + nrep);
+  const long long per = (ntasks + gridDim.x - 1) / gridDim.x;
+  const long long t0 = (long long)blockIdx.x * per, t1 = min(ntasks, t0 + per);
+  auto find = [&](long long t, int lo) {  // the replica of task t, at or after lo
+    int hi = nrep - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(start + mid) <= t) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+  };
+  const int rep0 = t0 < t1 ? find(t0, 0) : 0;
+  int r = rep0;
+  unsigned long long pairs = 0, hetero = 0;  // this lane's counts of replica r
+  auto flush = [&]() {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        int xx = x + dxs[k], yy = y + dys[k];
-        xx = xx < 0 ? xx + R.nx : (xx >= R.nx ? xx - R.nx : xx);
-        yy = yy >= R.ny ? yy - R.ny : yy;
-        const uint32_t w = lat[R.lat_off + (long long)yy * R.nx + xx];
-        if ((w & 0xFFFFFFu) && w != v) {
-          ++pairs;
-          hetero += (w >> 24) != (v >> 24);
-        }
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      pairs += __shfl_xor_sync(kFull, pairs, o);
+      hetero += __shfl_xor_sync(kFull, hetero, o);
     }
-    if (pairs) {
-      atomicAdd(&counts[2 * r], (unsigned long long)pairs);
-      if (hetero) atomicAdd(&counts[2 * r + 1], (unsigned long long)hetero);
+    if (lane == 0 && pairs) {
+      unsigned long long* dst = r == rep0 ? s_sum : counts + 2LL * r;
+      atomicAdd(dst, pairs);
+      if (hetero) atomicAdd(dst + 1, hetero);
     }
+    pairs = hetero = 0;
+  };
+  for (long long t = t0 + warp; t < t1; t += wpb) {
+    if (t >= __ldg(start + r + 1)) {
+      flush();
+      r = find(t, r);
+    }
+    const int nx = __ldg(&reps[r].nx), ny = __ldg(&reps[r].ny);
+    const uint32_t* L = lat + __ldg(&reps[r].lat_off);
+    const int local = (int)(t - __ldg(start + r)), segs = (nx + 31) >> 5;
+    const int x = (local % segs) * 32 + lane, y0 = (local / segs) * kObserveRows;
+    const int rows = min(kObserveRows, ny - y0);
+    if (x >= nx) continue;
+    const int xl = x ? x - 1 : nx - 1, xr = x + 1 < nx ? x + 1 : 0;
+    const uint32_t* row = L + (long long)y0 * nx;
+    uint32_t v = __ldg(row + x), right = __ldg(row + xr);
+    unsigned np = 0, nh = 0;
+    auto pair = [&](uint32_t w) {
+      const bool p = (v & 0xFFFFFFu) && (w & 0xFFFFFFu) && w != v;
+      np += p;
+      nh += p && (w >> 24) != (v >> 24);
+    };
+#pragma unroll 4
+    for (int k = 0; k < rows; ++k) {
+      // forward half of the Moore neighbourhood: (0,1), (1,-1), (1,0), (1,1)
+      row = y0 + k + 1 < ny ? row + nx : L;
+      const uint32_t l = __ldg(row + xl), c = __ldg(row + x), rr = __ldg(row + xr);
+      pair(right);
+      pair(l);
+      pair(c);
+      pair(rr);
+      v = c;
+      right = rr;
+    }
+    pairs += np;
+    hetero += nh;
   }
+  __syncwarp();
+  flush();
+  __syncthreads();
+  if (threadIdx.x < 2 && s_sum[threadIdx.x])
+    atomicAdd(counts + 2LL * rep0 + threadIdx.x, s_sum[threadIdx.x]);
 }
 
 // ---- periodic Voronoi seeding -------------------------------------------------
@@ -1214,67 +1267,134 @@ __global__ void observe_heterotypic_kernel(const uint32_t* __restrict__ lat,
 // nothing) until the best squared distance is below the squared lower bound
 // r * min(w) of every bucket not yet scanned, so the answer is the exact
 // brute-force nearest point with ties to the lowest index.
+//
+// The rings are scanned in FP32 first, keeping the nearest point and the
+// distance of the second nearest: this chip has 2 FP64 lanes per SM, and a
+// distance takes 11 FP64 operations (all in FP64: 5.96 ms on a 2048^2
+// tissue, the whole seed / recount / measure sequence on it 9.94 ms, now 1.29).  A float distance is off by at most vg.ferr, so a nearest point
+// that leads by more than 2 ferr is the answer; only where the lead is
+// smaller (ties, points midway) are the site's rings scanned in double.
 __device__ __forceinline__ double min_image(double a, double b, int n) {
-  double d = fabs(__dsub_rn(a, b));
+  const double d = fabs(__dsub_rn(a, b));
   const double e = __dsub_rn((double)n, d);
   return e < d ? e : d;
 }
 
-__global__ void voronoi_kernel(uint32_t* lat, VoronoiGrid vg, const double* __restrict__ pts,
-                               const int* __restrict__ idx, const uint32_t* __restrict__ values,
-                               const int* __restrict__ start) {
-  const long long sites = (long long)vg.n[0] * vg.n[1] * vg.n[2];
-  for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < sites;
-       s += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(s % vg.n[0]), y = (int)((s / vg.n[0]) % vg.n[1]),
-              z = (int)(s / ((long long)vg.n[0] * vg.n[1]));
-    const double c[3] = {(double)x, (double)y, (double)z};
-    int b[3];
-    for (int a = 0; a < 3; ++a) {
-      b[a] = (int)floor(__ddiv_rn(c[a], vg.w[a]));
-      b[a] = b[a] < 0 ? 0 : (b[a] >= vg.g[a] ? vg.g[a] - 1 : b[a]);
+// Bucket coordinate b of an axis of g buckets, wrapped.
+__device__ __forceinline__ int wrap_bucket(int b, int g) {
+  if (b < 0) b += g;
+  if (b >= g) b -= g;
+  if (b < 0 || b >= g) {  // (rings wider than this axis)
+    b %= g;
+    b += b < 0 ? g : 0;
+  }
+  return b;
+}
+
+// visit(k0, k1) for the points of every bucket of ring r around bucket b.
+template <int NDIM, class F>
+__device__ __forceinline__ void scan_ring(const VoronoiGrid& vg, const int* __restrict__ start,
+                                          const int (&b)[3], int r, F&& visit) {
+  const int zr = NDIM == 3 ? r : 0;
+  for (int dz = -zr; dz <= zr; ++dz) {
+    const int bz = NDIM == 3 ? wrap_bucket(b[2] + dz, vg.g[2]) : 0;
+    for (int dy = -r; dy <= r; ++dy) {
+      const int row = (bz * vg.g[1] + wrap_bucket(b[1] + dy, vg.g[1])) * vg.g[0];
+      // the shell of ring r: whole rows on its faces, else the two ends
+      const bool face = dy == r || dy == -r || (NDIM == 3 && (dz == r || dz == -r));
+      for (int dx = -r; dx <= r; dx += face || r == 0 ? 1 : 2 * r) {
+        const int bucket = row + wrap_bucket(b[0] + dx, vg.g[0]);
+        visit(__ldg(start + bucket), __ldg(start + bucket + 1));
+      }
     }
-    double best = 1e300;
-    int best_k = 0x7FFFFFFF;
-    uint32_t best_v = 0;
-    const int rz_max = vg.ndim == 3 ? 1 : 0;
-    for (int r = 0; r <= vg.rmax; ++r) {
-      for (int dz = -r * rz_max; dz <= r * rz_max; ++dz)
-        for (int dy = -r; dy <= r; ++dy)
-          for (int dx = -r; dx <= r; ++dx) {
-            const int ax = dx < 0 ? -dx : dx, ay = dy < 0 ? -dy : dy, az = dz < 0 ? -dz : dz;
-            const int cheb = ax > ay ? (ax > az ? ax : az) : (ay > az ? ay : az);
-            if (cheb != r) continue;  // the shell of ring r only
-            int bx = (b[0] + dx) % vg.g[0], by = (b[1] + dy) % vg.g[1],
-                bz = (b[2] + dz) % vg.g[2];
-            bx += bx < 0 ? vg.g[0] : 0;
-            by += by < 0 ? vg.g[1] : 0;
-            bz += bz < 0 ? vg.g[2] : 0;
-            const int bucket = (bz * vg.g[1] + by) * vg.g[0] + bx;
-            const int k1 = __ldg(start + bucket + 1);
-            for (int k = __ldg(start + bucket); k < k1; ++k) {
-              const double ddx = min_image(c[0], __ldg(pts + 3 * k), vg.n[0]);
-              const double ddy = min_image(c[1], __ldg(pts + 3 * k + 1), vg.n[1]);
-              double d2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
-              if (vg.ndim == 3) {
-                const double ddz = min_image(c[2], __ldg(pts + 3 * k + 2), vg.n[2]);
-                d2 = __dadd_rn(d2, __dmul_rn(ddz, ddz));
-              }
-              const int kk = __ldg(idx + k);
-              if (d2 < best || (d2 == best && kk < best_k)) {
-                best = d2;
-                best_k = kk;
-              }
+  }
+}
+
+template <int NDIM>
+__global__ void __launch_bounds__(256)
+    voronoi_kernel(uint32_t* lat, const VoronoiGrid vg, const double* __restrict__ pts,
+                   const float4* __restrict__ fpts, const int* __restrict__ idx,
+                   const uint32_t* __restrict__ values, const int* __restrict__ start) {
+  const unsigned sites = (unsigned)vg.n[0] * vg.n[1] * vg.n[2];  // < 2^31
+  for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < sites;
+       s += gridDim.x * blockDim.x) {
+    const int x = (int)(s % vg.n[0]), yz = (int)(s / vg.n[0]);
+    const int y = NDIM == 3 ? yz % vg.n[1] : yz, z = NDIM == 3 ? yz / vg.n[1] : 0;
+    const int xyz[3] = {x, y, z};
+    int b[3];
+    float edge = 3.0e38f;  // distance to the nearest edge of the site's bucket
+#pragma unroll
+    for (int a = 0; a < NDIM; ++a) {  // (FP32: ferr covers a bucket off at its edge)
+      const float c = (float)xyz[a];
+      b[a] = (int)floorf(c * vg.inv_w[a]);
+      b[a] = min(max(b[a], 0), vg.g[a] - 1);
+      const float lo = c - (float)b[a] * vg.wf[a];
+      edge = fminf(edge, fminf(lo, vg.wf[a] - lo));
+    }
+    if (NDIM == 2) b[2] = 0;
+    const float fx = (float)x, fy = (float)y, fz = (float)z;
+    const float nx = (float)vg.n[0], ny = (float)vg.n[1], nz = (float)vg.n[2];
+    auto dist2 = [&](const float4 p) {
+      float dx = fabsf(fx - p.x), dy = fabsf(fy - p.y);
+      dx = fminf(dx, nx - dx);
+      dy = fminf(dy, ny - dy);
+      float d2 = dx * dx + dy * dy;
+      if (NDIM == 3) {
+        float dz = fabsf(fz - p.z);
+        dz = fminf(dz, nz - dz);
+        d2 = d2 + dz * dz;
+      }
+      return d2;
+    };
+    float best = 3.0e38f, second = 3.0e38f;  // squared, of two different points
+    int best_j = -1;                         // position in bucket order
+    int r = 0;
+    for (; r <= vg.rmax; ++r) {
+      scan_ring<NDIM>(vg, start, b, r, [&](int k0, int k1) {
+        for (int k = k0; k < k1; ++k) {
+          const float d2 = dist2(__ldg(fpts + k));
+          if (k == best_j) continue;
+          second = fminf(second, fmaxf(best, d2));
+          if (d2 < best) {
+            best = d2;
+            best_j = k;
+          }
+        }
+      });
+      // every bucket not scanned yet lies at periodic Chebyshev distance
+      // >= r + 1, so its points are at least r * min(w) + edge away
+      const float lb = (float)r * vg.lb_scale + edge - 3.0f * vg.ferr;
+      if (best_j >= 0 && lb > 0.0f && best < lb * lb) break;
+    }
+    const float lead = sqrtf(best) + 2.0f * vg.ferr, lead2 = lead * lead;
+    uint32_t out = 0;
+    if (best_j >= 0 && second > lead2) {
+      out = __ldg(values + __ldg(idx + best_j));
+    } else {  // the points that may be nearest, in double
+      double dbest = 1e300;
+      int best_k = 0x7FFFFFFF;
+      for (int q = 0; q <= min(r, vg.rmax); ++q) {
+        scan_ring<NDIM>(vg, start, b, q, [&](int k0, int k1) {
+          for (int k = k0; k < k1; ++k) {
+            if (dist2(__ldg(fpts + k)) > lead2) continue;
+            const double ddx = min_image((double)x, __ldg(pts + 3LL * k), vg.n[0]);
+            const double ddy = min_image((double)y, __ldg(pts + 3LL * k + 1), vg.n[1]);
+            double d2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
+            if (NDIM == 3) {
+              const double ddz = min_image((double)z, __ldg(pts + 3LL * k + 2), vg.n[2]);
+              d2 = __dadd_rn(d2, __dmul_rn(ddz, ddz));
+            }
+            const int kk = __ldg(idx + k);
+            if (d2 < dbest || (d2 == dbest && kk < best_k)) {
+              dbest = d2;
+              best_k = kk;
             }
           }
-      // every bucket not scanned yet lies at periodic Chebyshev distance
-      // >= r + 1, so its points are at least r * min(w) away; the margin
-      // covers the rounding of the bucket indices
-      const double lb = __dsub_rn(__dmul_rn((double)r, vg.lb_scale), 1e-6);
-      if (best_k != 0x7FFFFFFF && lb > 0.0 && best < __dmul_rn(lb, lb)) break;
+        });
+      }
+      if (best_k != 0x7FFFFFFF) out = __ldg(values + best_k);
     }
-    if (best_k != 0x7FFFFFFF) best_v = __ldg(values + best_k);
-    lat[s] = best_v;
+    lat[s] = out;
   }
 }
 
@@ -1332,14 +1452,17 @@ __global__ void observe_boundaries_kernel(const uint32_t* __restrict__ lat,
 }  // namespace
 
 cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, const double* pts,
-                           const int* idx, const uint32_t* values, const int* start,
-                           cudaStream_t s) {
+                           const float4* fpts, const int* idx, const uint32_t* values,
+                           const int* start, cudaStream_t s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long sites = (long long)vg.n[0] * vg.n[1] * vg.n[2];
   const int grid = (int)std::max(1LL, std::min<long long>((sites + 255) / 256, (long long)sms * 16));
-  voronoi_kernel<<<grid, 256, 0, s>>>(lat, vg, pts, idx, values, start);
+  if (vg.ndim == 2)
+    voronoi_kernel<2><<<grid, 256, 0, s>>>(lat, vg, pts, fpts, idx, values, start);
+  else
+    voronoi_kernel<3><<<grid, 256, 0, s>>>(lat, vg, pts, fpts, idx, values, start);
   return cudaGetLastError();
 }
 
@@ -1413,14 +1536,14 @@ cudaError_t launch_persist_update(double* prefdir, double* hist, int H, int slot
 }
 
 cudaError_t launch_observe_heterotypic(const uint32_t* lat, const DevReplica* reps,
-                                       int nrep, long long total_sites,
+                                       int nrep, const long long* start, long long ntasks,
                                        unsigned long long* counts, cudaStream_t s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long want = (total_sites + 255) / 256;
-  const int grid = (int)std::max(1LL, std::min<long long>(want, (long long)sms * 8));
-  observe_heterotypic_kernel<<<grid, 256, 0, s>>>(lat, reps, nrep, total_sites, counts);
+  const int grid =
+      (int)std::max(1LL, std::min<long long>((ntasks + 7) / 8, (long long)sms * 8));
+  observe_heterotypic_kernel<<<grid, 256, 0, s>>>(lat, reps, nrep, start, counts);
   return cudaGetLastError();
 }
 
