@@ -22,8 +22,8 @@ NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "--fmad=false",
            "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
            f"-I{INCLUDE}", f"-I{CSRC}"]
 SOURCES = ["cpm_engine.cu", "cpm_kernels.cu", "cpm_sweep2d.cu", "cpm_sweep3d.cu",
-           "cpm_static.cu"]
-HEADERS = ["cpm_internal.h", "cpm_device.cuh", "cpm_sweep_common.cuh", "cpm_rowtile.cuh"]
+           "cpm_cluster.cu", "cpm_static.cu"]
+HEADERS = ["cpm_internal.h", "cpm_device.cuh", "cpm_sweep_common.cuh", "cpm_sweep.cuh"]
 
 
 def _nvcc() -> str:

@@ -14,15 +14,11 @@
 //     __constant__ struct in every setter, src/kernels.cu:50-53);
 //   * every call returns a status and keeps a message (the reference prints
 //     CUDA errors and carries on, src/cpm.cu:52-56).
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -41,6 +37,59 @@ constexpr int kMaxMcsPerLaunch = 1 << 16;
 }  // namespace
 
 void gpucpm::set_thread_error(const char* message) { g_create_error = message; }
+
+namespace {
+constexpr int kWarps2d = 24, kWarpsWide = 20;  // sweep_warps (cpm_sweep.cuh)
+}
+
+// Variant 0.  A slot's 32-column rows of targets are spread over every SM.
+// While a block has at most one row per warp, one row per task: the phase is
+// one warp's chain, and rows side by side would lengthen it.  Up to four rows
+// per warp they are drawn side by side, one task per warp.  Beyond that,
+// 4-row tasks (8-row ones where every warp still gets two or more), claimed
+// until the slot is done.  Measured (us, one / two / four rows side by side):
+// 101 x 75 x 61 box, 20 MCS 2823 / 2827 / 2941; 1001 x 777, 20 MCS 975 / 942 /
+// 1018; 4096^2 tissue, 50 MCS 8755 / 7875 / 7606; 256^3 tissue, 20 MCS 4268 /
+// 3782 / 3658 (8-row tasks: 3614).
+SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int sms, bool wide) {
+  const long long ncx = std::max(1, nx >> 1), ncy = std::max(1, ny >> 1),
+                  ncz = ndim == 3 ? std::max(1, nz >> 1) : 1;
+  const long long tnx = (ncx + 31) / 32, units = tnx * ncy * ncz;
+  const int W = ndim == 2 && !wide ? kWarps2d : kWarpsWide;
+  const long long upb = (units + sms - 1) / sms;  // rows of a block
+  SweepPlan p;
+  switch (variant) {
+    case 1: p.kr = 2, p.rows = 8; break;
+    case 2: p.kr = 4, p.rows = 16; break;
+    case 3: p.kr = 1, p.rows = 1; break;
+    default:
+      p.kr = upb <= W ? 1 : (upb <= 2 * W ? 2 : 4);
+      p.rows = upb > 16 * W ? 8 : p.kr;
+  }
+  if (wide) {
+    p.kr = 2;
+    p.rows = std::max(p.rows, 2);
+  }
+  const long long tasks = tnx * ((ncy + p.rows - 1) / p.rows) * ncz;
+  p.grid = (int)std::min<long long>(sms, tasks);
+  const long long per = (tasks + p.grid - 1) / p.grid;  // of a block
+  p.warps = (int)std::min<long long>(W, per);
+  p.list_cap = 2 * std::min(32LL, ncx) * std::min<long long>(p.rows, ncy) * per;
+  return p;
+}
+
+// Long tasks fill a warp's batches (attempts of different replicas are not
+// evaluated together); small batches need every warp to get a task.
+int gpucpm::batch_rows(int variant, long long total_units, int sms) {
+  switch (variant) {
+    case 1: return 8;
+    case 2: return 32;
+    case 3: return 2;
+    default: break;
+  }
+  const long long per_warp = total_units / ((long long)sms * kWarpsWide);
+  return per_warp >= 32 ? 16 : (per_warp >= 8 ? 8 : (per_warp >= 4 ? 4 : 2));
+}
 
 struct cpm_handle {
   int ndim = 2;
@@ -64,13 +113,15 @@ struct cpm_handle {
   // reference keeps them, device floats; layout of SweepArgs::field
   std::vector<double> h_field;
   float* d_field = nullptr;
-  // act model (allocated on first use): MCS of the last copy into each site,
-  // and the per-block lists of copies deferred to the end of their phase
+  // act model (allocated on first use): MCS of the last copy into each site;
+  // (on the first act run) second copies of lattice and stamps, and the
+  // blocks' lists of the copies of two phases (SweepArgs::lat2, act2, pend)
   std::vector<uint32_t> h_act;
   uint32_t* d_act = nullptr;
-  unsigned long long* d_pend_site = nullptr;
-  uint32_t* d_pend_val = nullptr;
-  long long pend_entries = 0;  // capacity of the pending arrays (all blocks)
+  uint32_t* d_lat2 = nullptr;
+  uint32_t* d_act2 = nullptr;
+  uint4* d_pend = nullptr;
+  long long pend_entries = 0;  // of all blocks' lists
   bool act_active = false;     // some replica's record has an act lambda
   // 3D persistence (allocated on first use): preferred direction per table
   // row, and the ring of the cells' mean coordinates after the last runs
@@ -98,14 +149,12 @@ struct cpm_handle {
   cudaStream_t stream = nullptr;      // stream work is enqueued on
   cudaStream_t own_stream = nullptr;  // created with the handle
   // One launch configuration per tile variant; `variant` is the one runs use
-  // (0 until cpm_autotune picks another).
+  // (0 until cpm_autotune picks another).  For one lattice `plan` is its
+  // sweep's and `wide` that of its extended and score kernels; for a batch
+  // both are grid dispatch's, and `local` is replica dispatch's.
   struct Config {
-    SweepShape shape;
-    int grid = 1;                  // grid dispatch
-    long long list_cap = 0;
-    int grid_local = 1;            // replica dispatch
-    long long list_cap_local = 0;
-    std::vector<int> task_prefix;  // [27][nrep + 1] warp tiles per slot
+    SweepPlan plan, wide, local;
+    std::vector<int> task_prefix;  // (batches) [27][nrep + 1] warp tasks per slot
     std::vector<int> active_slots;
     // hybrid dispatch: the first hyb_ng replicas of rep_order run in grid
     // dispatch (hyb_prefix: [27][hyb_ng + 1], in rep_order), the rest in
@@ -115,21 +164,16 @@ struct cpm_handle {
   } cfg[kTileVariants];
   int variant = 0;
   int dispatch = CPM_DISPATCH_GRID;  // CPM_DISPATCH_*
-  // Single lattices whose width is a multiple of 4 run the row-tile sweeps
-  // (cpm_sweep2d.cu, cpm_sweep3d.cu).  fill: CPM_FILL_PARITY = the parity-split sweep_kernel,
-  // CPM_FILL_VECTOR = row tiles staged with 16-byte loads, CPM_FILL_TMA = row
-  // tiles whose interior tiles are copied by the tensor-map engine (the
-  // default where the maps could be encoded).
+  // CPM_FILL_*: CPM_FILL_CLUSTER runs the cluster sweep (cpm_cluster.cu), the
+  // others the same sweep (cpm_sweep.cuh); row_ok: the shapes that once had
+  // row tiles, which accept CPM_FILL_VECTOR and CPM_FILL_TMA
   int fill = CPM_FILL_PARITY;
-  bool row_ok = false, tma_ok = false;
+  bool row_ok = false;
   // CPM_FILL_CLUSTER: small 2D lattices swept by one thread-block cluster of
   // cl_G blocks, cl_H rows each, dirty lists of cl_cap entries per block
   bool cluster_ok = false;
   int cl_G = 0, cl_H = 0;
   long long cl_cap = 0;
-  struct alignas(64) TileMap {
-    unsigned char bytes[128];  // CUtensorMap of the lattice, box of one variant
-  } tmap[kTileVariants];
   std::vector<unsigned long long> attempts;  // per replica, host-counted
 
   // Graph-captured run (cpm_run_graph): the captured launch reads and
@@ -196,8 +240,9 @@ void free_all(cpm_handle* h) {
   cudaFreeHost(h->h_lat);
   cudaFree(h->d_field);
   cudaFree(h->d_act);
-  cudaFree(h->d_pend_site);
-  cudaFree(h->d_pend_val);
+  cudaFree(h->d_lat2);
+  cudaFree(h->d_act2);
+  cudaFree(h->d_pend);
   cudaFree(h->d_prefdir);
   cudaFree(h->d_hist);
   cudaFree(h->d_lat);
@@ -223,48 +268,25 @@ void free_all(cpm_handle* h) {
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
 }
 
-// Tensor maps of a single lattice for the row-tile sweeps: the lattice as a
-// ny x nx (nz x ny x nx) array of 32-bit words, one box of 72 x (2 CY + 1)
-// (x (2 CZ + 1)) words per tile variant.  cuTensorMapEncodeTiled is reached through the runtime's driver
-// entry point, so the library does not link the driver library itself.
-// False (and no maps) when the entry point or the encoding is unavailable.
-bool encode_tile_maps(cpm_handle* h) {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
-                                         cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  });
-  if (!encode) return false;
-  const DevReplica& R = h->reps[0];
-  for (int v = 0; v < kTileVariants; ++v) {
-    const cuuint64_t dims[3] = {(cuuint64_t)R.nx, (cuuint64_t)R.ny, (cuuint64_t)R.nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)R.nx * 4, (cuuint64_t)R.nx * R.ny * 4};
-    cuuint32_t box[3] = {72u, (cuuint32_t)row_tile_rows(v), 1u};
-    if (h->ndim == 3) {
-      int rows = 0, planes = 0;
-      box_tile_extent(v, &rows, &planes);
-      box[1] = (cuuint32_t)rows;
-      box[2] = (cuuint32_t)planes;
-    }
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    if (encode(reinterpret_cast<CUtensorMap*>(h->tmap[v].bytes), CU_TENSOR_MAP_DATA_TYPE_UINT32,
-               (cuuint32_t)h->ndim, h->d_lat + R.lat_off, dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  }
-  return true;
+// Shapes that accept CPM_FILL_VECTOR and CPM_FILL_TMA.
+bool rows_fit(int ndim, int nx, int ny, int nz) {
+  return ndim == 2 ? row_tiles_fit(nx, ny) : nx % 4 == 0 && nx >= 72 && ny >= 18 && nz >= 18;
 }
 
 void default_params(DevParams& p, float T) {
   std::memset(&p, 0, sizeof p);
   p.temperature = T;
+}
+
+// Whether every target lies where the sweep may compute a constraint's
+// integers in FP32 (DevParams::small_targets).
+bool targets_small(const DevParams& p) {
+  constexpr int kLim = 1 << 21;
+  for (int k = 0; k < kMaxTypes; ++k)
+    if (p.tgt_area[k] <= -kLim || p.tgt_area[k] >= kLim || p.tgt_perim[k] <= -kLim ||
+        p.tgt_perim[k] >= kLim)
+      return false;
+  return true;
 }
 
 bool perim_on(const DevParams& p) {
@@ -321,6 +343,9 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     }
     R.lat_off = sites;
     R.cell_off = rows;
+    R.pad = 0;
+    R.div_nx = fast_div_of((uint32_t)R.nx);
+    R.div_plane = fast_div_of((uint32_t)R.nx * (uint32_t)R.ny);
     sites += ns;
     rows += (long long)R.ncells + 1;
     h->reps.push_back(R);
@@ -370,15 +395,14 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     return e == cudaErrorMemoryAllocation ? CPM_ERR_ALLOC : CPM_ERR_CUDA;
   }
   std::memset(h->h_lat, 0, sizeof(uint32_t) * sites);
-  if (n == 1 && (ndim == 2 ? row_tiles_fit(nx[0], ny[0]) : box_tiles_fit(nx[0], ny[0], nz[0]))) {
+  if (n == 1 && rows_fit(ndim, nx[0], ny[0], nz ? nz[0] : 1)) {
     h->row_ok = true;
-    h->tma_ok = encode_tile_maps(h);
-    h->fill = h->tma_ok ? CPM_FILL_TMA : CPM_FILL_VECTOR;
+    h->fill = CPM_FILL_TMA;
     if (ndim == 2)
       h->cluster_ok = cluster_sweep_plan(nx[0], ny[0], &h->cl_G, &h->cl_H, &h->cl_cap);
   }
 
-  // One launch configuration per tile variant: warp tiles per slot and
+  // One launch configuration per tile variant: warp tasks per slot and
   // replica (prefix over replicas), grid, dirty-list capacity.
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
@@ -394,23 +418,47 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     const DevReplica &X = h->reps[x], &Y = h->reps[y];
     return (long long)X.nx * X.ny * X.nz > (long long)Y.nx * Y.ny * Y.nz;
   });
+  // 32-column rows of targets of replica r's slot
+  auto units = [&](int r, int slot, int rows) -> long long {
+    const DevReplica& R = h->reps[r];
+    const int cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
+    if (ndim == 2 && cz != 0) return 0;
+    const long long ncx = class_count_h(R.nx, cx), ncy = class_count_h(R.ny, cy),
+                    ncz = class_count_h(R.nz, cz);
+    return ((ncx + 31) / 32) * ((ncy + rows - 1) / rows) * ncz;
+  };
+  if (sms < 1) {
+    g_create_error = "cannot place the sweep kernel on this device";
+    free_all(h);
+    delete h;
+    return CPM_ERR_CUDA;
+  }
+  long long total_units = 0;
+  int biggest = order[0];
+  for (int r = 0; r < n; ++r) {
+    total_units += units(r, 0, 1);
+    if (units(r, 0, 1) > units(biggest, 0, 1)) biggest = r;
+  }
+  long long pend_entries = 1;
   for (int v = 0; v < kTileVariants; ++v) {
     cpm_handle::Config& c = h->cfg[v];
-    c.shape = sweep_shape(ndim, v);
+    const DevReplica& B = h->reps[biggest];
+    if (n == 1) {
+      c.plan = plan_sweep(ndim, B.nx, B.ny, B.nz, v, sms, false);
+      c.wide = plan_sweep(ndim, B.nx, B.ny, B.nz, v, sms, true);
+      c.local = c.plan;  // (not used)
+      dlist_entries = std::max(dlist_entries, c.plan.list_cap * 2 * c.plan.grid);
+      dlist_entries = std::max(dlist_entries, c.wide.list_cap * 2 * c.wide.grid);
+      pend_entries = std::max(pend_entries, c.wide.list_cap * c.wide.grid);
+    }
+    const int rows = n == 1 ? c.plan.rows : batch_rows(v, total_units, sms);
     c.task_prefix.assign(27 * (n + 1), 0);
     long long max_tasks = 1;
     for (int slot = 0; slot < 27; ++slot) {
-      const int cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
       long long acc = 0;
       for (int r = 0; r < n; ++r) {
-        c.task_prefix[slot * (n + 1) + r] = (int)acc;
-        const DevReplica& R = h->reps[r];
-        if (ndim == 2 && cz != 0) continue;
-        const long long ncx = class_count_h(R.nx, cx), ncy = class_count_h(R.ny, cy),
-                        ncz = class_count_h(R.nz, cz);
-        if (!ncx || !ncy || !ncz) continue;
-        acc += ((ncx + c.shape.cx - 1) / c.shape.cx) * ((ncy + c.shape.cy - 1) / c.shape.cy) *
-               ((ncz + c.shape.cz - 1) / c.shape.cz);
+        c.task_prefix[slot * (n + 1) + r] = (int)std::min<long long>(acc, INT32_MAX);
+        acc += units(r, slot, rows);
       }
       if (acc >= (1LL << 31)) {
         g_create_error = "batch too large for one launch";
@@ -422,59 +470,31 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
       if (acc > 0) c.active_slots.push_back(slot);
       max_tasks = std::max(max_tasks, acc);
     }
-    const int per_sm = std::min(sweep_max_blocks_per_sm(ndim, true, v),
-                                sweep_max_blocks_per_sm(ndim, false, v));
-    if (per_sm < 1 || sms < 1) {
-      g_create_error = "cannot place the sweep kernel on this device";
-      free_all(h);
-      delete h;
-      return CPM_ERR_CUDA;
+    if (n > 1) {
+      // Grid dispatch: tasks dealt one at a time, at most ceil(tasks / grid)
+      // per block, each attempt touching at most two table rows.
+      c.plan.kr = 2;
+      c.plan.rows = rows;
+      c.plan.warps = 20;
+      c.plan.grid = (int)std::min<long long>(sms, max_tasks);
+      c.plan.list_cap = 2LL * 32 * rows * ((max_tasks + c.plan.grid - 1) / c.plan.grid);
+      c.wide = c.plan;
+      // Replica dispatch: one block per replica at a time.
+      c.local = plan_sweep(ndim, B.nx, B.ny, B.nz, v, 1, false);
+      const SweepPlan w = plan_sweep(ndim, B.nx, B.ny, B.nz, v, 1, true);
+      c.local.list_cap = std::max(c.local.list_cap, w.list_cap);
+      for (int r = 0; r < n; ++r)  // (a narrower replica may have more rows)
+        c.local.list_cap = std::max(c.local.list_cap, 2LL * 32 * c.local.rows *
+                                                          units(r, 0, c.local.rows));
+      c.local.grid = std::min(sms, n);
+      for (const SweepPlan& p : {c.plan, c.local}) {
+        dlist_entries = std::max(dlist_entries, p.list_cap * 2 * p.grid);
+        pend_entries = std::max(pend_entries, p.list_cap * p.grid);
+      }
     }
-    // One block per SM (fewer if the largest slot has fewer warp tiles).
-    const long long blocks_needed = (max_tasks + c.shape.warps - 1) / c.shape.warps;
-    c.grid = (int)std::max(1LL, std::min<long long>((long long)per_sm * sms, blocks_needed));
-    // Per-block dirty lists (two per block, for the running and the previous
-    // phase): a warp works at most ceil(tiles / warps) tiles per slot, each
-    // attempt touching at most two table rows.
-    const long long warps = (long long)c.grid * c.shape.warps;
-    const long long nt = (long long)c.shape.cx * c.shape.cy * c.shape.cz;
-    c.list_cap = 2LL * nt * c.shape.warps * ((max_tasks + warps - 1) / warps);
-    if (ndim == 2) {  // score launches run fewer warps per block (more tiles each)
-      const int sw = sweep_shape(ndim, v, true).warps;
-      const long long swarps = (long long)c.grid * sw;
-      c.list_cap = std::max(c.list_cap, 2LL * nt * sw * ((max_tasks + swarps - 1) / swarps));
-    }
-    if (n == 1 && (ndim == 2 ? row_tiles_fit(nx[0], ny[0])
-                             : box_tiles_fit(nx[0], ny[0], nz[0]))) {
-      // the row-tile sweeps of the one lattice: tiles of 32 x ry (x rz)
-      // targets, dealt to the blocks one at a time; a block gets at most
-      // ceil(tiles / grid) of them
-      int rows = 0, planes = 3;
-      if (ndim == 2)
-        rows = row_tile_rows(v);
-      else
-        box_tile_extent(v, &rows, &planes);
-      const long long ry = rows / 2, rz = planes / 2;
-      const long long tnx = ((nx[0] / 2) + 31) / 32;
-      const long long tiles = tnx * (((ny[0] + 1) / 2 + ry - 1) / ry) *
-                              (ndim == 3 ? (((nz[0] + 1) / 2 + rz - 1) / rz) : 1);
-      const long long per_block = (tiles + c.grid - 1) / c.grid;
-      c.list_cap = std::max(c.list_cap, 2LL * per_block * 32 * ry * rz);
-    }
-    dlist_entries = std::max(dlist_entries, c.list_cap * 2 * c.grid);
-    // Replica dispatch: one block per replica at a time; its dirty list takes
-    // up to two rows per attempt of the replica's largest slot.
-    long long max_rep_tiles = 1;
-    for (int slot = 0; slot < 27; ++slot)
-      for (int r = 0; r < n; ++r)
-        max_rep_tiles = std::max<long long>(
-            max_rep_tiles, c.task_prefix[slot * (n + 1) + r + 1] - c.task_prefix[slot * (n + 1) + r]);
-    c.grid_local = std::min(per_sm * sms, n);
-    c.list_cap_local = n > 1 ? 2LL * nt * max_rep_tiles : 0;  // batches only
-    dlist_entries = std::max(dlist_entries, c.list_cap_local * 2 * c.grid_local);
     // Hybrid split: replica dispatch gets whole rounds of the smallest
     // replicas, grid dispatch the rest.
-    c.hyb_ng = n - (n / c.grid_local) * c.grid_local;
+    c.hyb_ng = n - (n / c.local.grid) * c.local.grid;
     const int ng = c.hyb_ng;
     c.hyb_prefix.assign(27 * (ng + 1), 0);
     for (int slot = 0; slot < 27; ++slot) {
@@ -487,8 +507,9 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
       c.hyb_prefix[slot * (ng + 1) + ng] = acc;
     }
   }
-  // act runs defer one copy per attempt at most: half a dirty list's entries
-  h->pend_entries = dlist_entries / 4 + 1;
+  // act runs list one copy per attempt at most, half of a dirty list's
+  // entries, in two lists per block
+  h->pend_entries = pend_entries;
   e = cudaMalloc((void**)&h->d_dlist, sizeof(uint32_t) * dlist_entries);
   if (e != cudaSuccess) {
     g_create_error = std::string("dirty-list allocation failed: ") + cudaGetErrorString(e);
@@ -501,8 +522,8 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
   // no replica is much larger than a block's fair share of the sites, hybrid
   // when those replicas do not fill whole rounds (the autotuner can change
   // the choice).
-  h->dispatch = (n >= h->cfg[0].grid_local && n >= sms &&
-                 max_sites * (long long)h->cfg[0].grid_local <= 2 * sites)
+  h->dispatch = (n >= h->cfg[0].local.grid && n >= sms &&
+                 max_sites * (long long)h->cfg[0].local.grid <= 2 * sites)
                     ? (h->cfg[0].hyb_ng > 0 ? CPM_DISPATCH_HYBRID : CPM_DISPATCH_REPLICA)
                     : CPM_DISPATCH_GRID;
   e = cudaMemcpyAsync(h->d_reps, h->reps.data(), sizeof(DevReplica) * n,
@@ -675,7 +696,7 @@ int persist_after_run(cpm_handle* h) {
   return CPM_OK;
 }
 
-// The act lattice (zeros) and the pending lists, on first use.
+// The act lattice (zeros), on first use.
 int ensure_act(cpm_handle* h) {
   if (!h->d_act) {
     const size_t n = (size_t)h->total_sites;
@@ -687,11 +708,16 @@ int ensure_act(cpm_handle* h) {
     CPM_CUDA(h, cudaMalloc((void**)&h->d_act, sizeof(uint32_t) * (n ? n : 1)));
     CPM_CUDA(h, cudaMemsetAsync(h->d_act, 0, sizeof(uint32_t) * (n ? n : 1), h->stream));
   }
-  if (!h->d_pend_site) {
-    CPM_CUDA(h, cudaMalloc((void**)&h->d_pend_site,
-                           sizeof(unsigned long long) * h->pend_entries));
-    CPM_CUDA(h, cudaMalloc((void**)&h->d_pend_val, sizeof(uint32_t) * h->pend_entries));
-  }
+  return CPM_OK;
+}
+
+// The act run's second lattice and stamp copies and its lists.
+int ensure_act_run(cpm_handle* h) {
+  if (int rc = ensure_act(h)) return rc;
+  const size_t b = sizeof(uint32_t) * (h->total_sites ? h->total_sites : 1);
+  if (!h->d_lat2) CPM_CUDA(h, cudaMalloc((void**)&h->d_lat2, b));
+  if (!h->d_act2) CPM_CUDA(h, cudaMalloc((void**)&h->d_act2, b));
+  if (!h->d_pend) CPM_CUDA(h, cudaMalloc((void**)&h->d_pend, sizeof(uint4) * h->pend_entries));
   return CPM_OK;
 }
 
@@ -733,6 +759,7 @@ int upload_params(cpm_handle* h) {
     p.persist_on = 0;
     for (int k = 0; k < kMaxTypes; ++k)
       if (p.persist_lambda[k] != 0.0f) p.persist_on = 1;
+    p.small_targets = targets_small(p) ? 1 : 0;
   }
   bool persist = false;
   for (const auto& p : h->psets) persist = persist || (h->ndim == 3 && p.persist_on);
@@ -749,7 +776,7 @@ int upload_params(cpm_handle* h) {
   bool act = false;
   for (const auto& p : h->psets) act = act || p.act_on;
   if (act) {
-    if (int rc = ensure_act(h)) return rc;
+    if (int rc = ensure_act_run(h)) return rc;
   }
   if (act != h->act_active) {  // another kernel, other arguments
     h->act_active = act;
@@ -788,9 +815,8 @@ bool any_perimeter(const cpm_handle* h) {
 }
 
 // Kernel arguments of a sweep with tile variant v and dispatch d (tick0 /
-// mcs filled in by the caller).
-SweepArgs sweep_args(const cpm_handle* h, int v, int d) {
-  if (h->act_active || h->persist_active) v = 0;  // extended-term kernels: variant 0
+// mcs, and what depends on the launch, filled in by the caller).
+SweepArgs sweep_args(const cpm_handle* h, int v) {
   SweepArgs a;
   std::memset(&a, 0, sizeof a);
   a.lat = h->d_lat;
@@ -802,15 +828,15 @@ SweepArgs sweep_args(const cpm_handle* h, int v, int d) {
   }
   const cpm_handle::Config& c = h->cfg[v];
   a.dlist = h->d_dlist;
-  a.block_local = d == CPM_DISPATCH_REPLICA ? 1 : 0;
   a.field = h->d_field;
-  a.act = h->d_act;
   a.act_on = h->act_active ? 1 : 0;
+  if (h->act_active) {
+    a.act = h->d_act;
+    a.lat2 = h->d_lat2;
+    a.act2 = h->d_act2;
+    a.pend = h->d_pend;
+  }
   a.prefdir = h->persist_active ? h->d_prefdir : nullptr;
-  a.pend_site = h->d_pend_site;
-  a.pend_val = h->d_pend_val;
-  a.pend_cap = (d == CPM_DISPATCH_REPLICA ? c.list_cap_local : c.list_cap) / 2;
-  a.list_cap = a.block_local ? c.list_cap_local : c.list_cap;
   a.rep_order = h->d_rep_order;
   a.queue_len = h->nrep;
   a.rep_map = nullptr;
@@ -828,61 +854,69 @@ SweepArgs sweep_args(const cpm_handle* h, int v, int d) {
   return a;
 }
 
-int grid_of(const cpm_handle* h, int v, int d) {
-  if (h->act_active || h->persist_active) v = 0;
-  return d == CPM_DISPATCH_REPLICA ? h->cfg[v].grid_local : h->cfg[v].grid;
+// The plan of a launch with variant v and dispatch d (GRID or REPLICA).
+const SweepPlan& plan_of(const cpm_handle* h, int v, int d, bool scores = false) {
+  const cpm_handle::Config& c = h->cfg[v];
+  if (d == CPM_DISPATCH_REPLICA) return c.local;
+  return scores || h->act_active || h->persist_active ? c.wide : c.plan;
 }
 
-// The launches of one sweep run (`a` from sweep_args with dispatch `d`,
-// times filled in): one launch for GRID and REPLICA, two for HYBRID (grid
-// dispatch over the first hyb_ng replicas of rep_order, then replica
-// dispatch over the rest).  Each launch starts with its barrier words
-// cleared.  Returns the number of launches through *nlaunch.
+int grid_of(const cpm_handle* h, int v, int d) { return plan_of(h, v, d).grid; }
+
+// The launches of one sweep run (`a` from sweep_args, times filled in): one
+// launch for GRID and REPLICA, two for HYBRID (grid dispatch over the first
+// hyb_ng replicas of rep_order, then replica dispatch over the rest).  Each
+// launch starts with its barrier words cleared.  Returns the number of
+// launches through *nlaunch.
 cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a, bool perim,
                           bool scores, int* nlaunch) {
-  if (h->act_active || h->persist_active) v = 0;
   const cpm_handle::Config& c = h->cfg[v];
   *nlaunch = 0;
-  auto one = [&](const SweepArgs& x, int grid) {
+  if (h->act_active) {  // both lattice and stamp copies start equal
+    const size_t b = sizeof(uint32_t) * h->total_sites;
+    cudaError_t e = cudaMemcpyAsync(h->d_lat2, h->d_lat, b, cudaMemcpyDeviceToDevice, h->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(h->d_act2, h->d_act, b, cudaMemcpyDeviceToDevice, h->stream);
+    if (e != cudaSuccess) return e;
+  }
+  auto one = [&](SweepArgs x, const SweepPlan& p, bool batch) {
     cudaError_t e = cudaMemsetAsync(h->d_ctl, 0, sizeof(uint32_t) * kCtlErr, h->stream);
-    const bool row = h->fill != CPM_FILL_PARITY && h->row_ok && !scores && !h->act_active &&
-                     !h->persist_active && x.nrep == 1 && x.rep_map == nullptr &&
-                     !x.block_local;
-    if (e == cudaSuccess && row && h->fill == CPM_FILL_CLUSTER) {
-      SweepArgs xc = x;
-      xc.list_cap = h->cl_cap;
-      e = launch_sweep2d_cluster(perim, v, xc, h->tmap[3].bytes, h->reps[0].nx, h->cl_G,
-                                 h->cl_H, h->stream);
-    } else if (e == cudaSuccess && row)
-      e = (h->ndim == 2 ? launch_sweep2d : launch_sweep3d)(
-          perim, v, x, h->tmap[v].bytes, h->fill == CPM_FILL_TMA ? 1 : 0, grid, c.shape.warps,
-          h->stream);
-    else if (e == cudaSuccess)
-      e = launch_sweep(h->ndim, perim, v, x, grid, h->stream, scores);
+    if (e != cudaSuccess) return e;
+    if (h->fill == CPM_FILL_CLUSTER && !scores && !h->act_active && !h->persist_active) {
+      x.list_cap = h->cl_cap;
+      e = launch_sweep2d_cluster(perim, v, x, h->reps[0].nx, h->cl_G, h->cl_H, h->stream);
+    } else {
+      x.rows = p.rows;
+      x.kr = p.kr;
+      x.list_cap = p.list_cap;
+      x.pend_cap = p.list_cap / 2;
+      e = h->ndim == 2 ? launch_sweep2d(x, batch, scores, p.grid, p.warps, h->stream)
+                       : launch_sweep3d(x, batch, p.grid, p.warps, h->stream);
+    }
     if (e == cudaSuccess) ++*nlaunch;
     return e;
   };
-  if (d != CPM_DISPATCH_HYBRID) return one(a, grid_of(h, v, d));
-  const int ng = c.hyb_ng;
+  if (d == CPM_DISPATCH_GRID) {
+    SweepArgs g = a;
+    g.block_local = 0;
+    return one(g, plan_of(h, v, d, scores), h->nrep > 1);
+  }
+  const int ng = d == CPM_DISPATCH_HYBRID ? c.hyb_ng : 0;
   if (ng > 0) {  // grid dispatch over the largest replicas
     SweepArgs g = a;
     g.block_local = 0;
-    g.list_cap = c.list_cap;
-    g.pend_cap = c.list_cap / 2;
     g.nrep = ng;
     g.task_prefix = h->d_hyb_prefix + (size_t)v * 27 * (h->nrep + 1);
     g.rep_map = h->d_rep_order;
     g.tick_advance = ng < h->nrep ? 0 : 1;
-    if (cudaError_t e = one(g, c.grid)) return e;
+    if (cudaError_t e = one(g, c.plan, true)) return e;
   }
-  if (ng < h->nrep) {  // replica dispatch over the rest, whole rounds
+  if (ng < h->nrep) {  // replica dispatch over the rest
     SweepArgs q = a;
     q.block_local = 1;
-    q.list_cap = c.list_cap_local;
-    q.pend_cap = c.list_cap_local / 2;
     q.rep_order = h->d_rep_order + ng;
     q.queue_len = h->nrep - ng;
-    if (cudaError_t e = one(q, c.grid_local)) return e;
+    if (cudaError_t e = one(q, c.local, false)) return e;
   }
   return cudaSuccess;
 }
@@ -1373,7 +1407,7 @@ int cpm_run(cpm_handle* h, int mcs) {
   if (mcs == 0) return CPM_OK;
   if (int rc = upload_params(h)) return rc;
   const bool any_perim = any_perimeter(h);
-  SweepArgs a = sweep_args(h, h->variant, h->dispatch);
+  SweepArgs a = sweep_args(h, h->variant);
   int left = mcs;
   while (left > 0) {
     const int chunk = std::min(left, kMaxMcsPerLaunch);
@@ -1409,7 +1443,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     }
     // Capture: reset the barrier words, then the persistent sweep reading
     // its start time from (and advancing) the device tick.
-    SweepArgs a = sweep_args(h, h->variant, h->dispatch);
+    SweepArgs a = sweep_args(h, h->variant);
     a.tick_ptr = h->d_tick;
     a.mcs = mcs;
     cudaGraph_t g = nullptr;
@@ -1498,8 +1532,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   // A lattice that one thread-block cluster can hold is also tried in the
   // cluster sweep (every one of its tile heights), unless the caller chose
   // the parity-split sweep.
-  const int row_fill = h->fill == CPM_FILL_CLUSTER ? (h->tma_ok ? CPM_FILL_TMA : CPM_FILL_VECTOR)
-                                                   : h->fill;
+  const int row_fill = h->fill == CPM_FILL_CLUSTER ? CPM_FILL_TMA : h->fill;
   const bool try_cluster = h->cluster_ok && h->fill != CPM_FILL_PARITY;
   if (try_cluster)
     for (int v = 0; v < kTileVariants; ++v) pairs.emplace_back(v, -1);
@@ -1510,7 +1543,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
     const bool cl = pairs[i % npairs].second < 0;
     const int d = cl ? CPM_DISPATCH_GRID : pairs[i % npairs].second;
     h->fill = cl ? CPM_FILL_CLUSTER : row_fill;
-    SweepArgs a = sweep_args(h, v, d);
+    SweepArgs a = sweep_args(h, v);
     a.tick0 = tick;
     a.mcs = probe_mcs;
     e = copy(false);
@@ -1572,7 +1605,7 @@ int cpm_run_scores(cpm_handle* h, int mcs, float* d_scores, uint64_t score_base,
   if (h->act_active || h->persist_active)
     return h->fail(CPM_ERR_UNSUPPORTED, "cpm_run_scores: scores of runs with the act or "
                                         "persistence term are not supported");
-  SweepArgs a = sweep_args(h, h->variant, h->dispatch);
+  SweepArgs a = sweep_args(h, h->variant);
   a.scores = d_scores;
   a.score_base = score_base;
   a.score_len = score_len;
@@ -1862,8 +1895,6 @@ int cpm_set_fill(cpm_handle* h, int fill) {
   if (fill != CPM_FILL_PARITY && !h->row_ok)
     return h->fail(CPM_ERR_UNSUPPORTED, "row tiles need one lattice with nx a multiple of 4 "
                                         "and nx >= 72; in 2D ny >= 66, in 3D ny, nz >= 18");
-  if (fill == CPM_FILL_TMA && !h->tma_ok)
-    return h->fail(CPM_ERR_UNSUPPORTED, "the tensor maps of this lattice could not be encoded");
   h->fill = fill;
   return CPM_OK;
 }
@@ -2029,12 +2060,12 @@ int cpm_info(const cpm_handle* h, int* n_replicas, int* dimensionality,
 int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x, int* tile_y,
                      int* tile_z, int* warps_per_block, int* grid, int* dispatch) {
   if (!h) return CPM_ERR_INVALID;
-  const cpm_handle::Config& c = h->cfg[h->variant];
   if (variant) *variant = h->variant;
-  if (tile_x) *tile_x = c.shape.cx;
-  if (tile_y) *tile_y = c.shape.cy;
-  if (tile_z) *tile_z = c.shape.cz;
-  if (warps_per_block) *warps_per_block = c.shape.warps;
+  const SweepPlan& p = plan_of(h, h->variant, h->dispatch);
+  if (tile_x) *tile_x = 32;
+  if (tile_y) *tile_y = p.rows;
+  if (tile_z) *tile_z = 1;
+  if (warps_per_block) *warps_per_block = p.warps;
   if (grid) *grid = grid_of(h, h->variant, h->dispatch);
   if (dispatch) *dispatch = h->dispatch;
   if (h->fill == CPM_FILL_CLUSTER) {  // one cluster, its own tile heights

@@ -35,70 +35,27 @@
 namespace gpucpm {
 
 constexpr int kMaxTypes = 32;
-// Warps per sweep block (one block per SM): 24 at 80 registers in 2D; 20 at
-// 96 registers in 3D and in score launches, whose attempts would spill at 80.
-constexpr int kMaxSweepWarps = 24;
-constexpr int kMaxSweepWarps3d = 20;
-template <int NDIM, bool SCORE = false>
-constexpr int max_sweep_warps() {
-  return (NDIM == 3 || SCORE) ? kMaxSweepWarps3d : kMaxSweepWarps;
-}
 constexpr int kSweepSmemMax = 227 * 1024;  // usable shared memory per block
 constexpr int kInitThreads = 256;
 
-// Warp tile: CX x CY x CZ targets of one slot, staged with their one-site
-// halo in the warp's own shared memory.  Four compiled variants per
-// dimensionality; the autotuner (cpm_autotune) picks one per engine.  The
-// sweep's result does not depend on the variant.
-//   2D  v0 32 x 6 (66 x 13 sites)   v1 32 x 8      v2 32 x 16     v3 32 x 1
-//   3D  v0 32 x 2 x 2 (66 x 5 x 5)  v1 32 x 4 x 2  v2 32 x 4 x 4  v3 32 x 1 x 1
-// v3 is for lattices too small to give every warp of the GPU a wide tile
-// (256^2 has 85 tiles of 32 x 6 per slot): one row of targets per warp cuts
-// the serial chain of a phase to one iteration of each pass.
+// How the slots of a sweep are cut into warp tasks of 32 target columns x
+// `rows` target rows, `kr` of them drawn side by side.  The sweep's result
+// does not depend on it.  Four variants; the autotuner (cpm_autotune) picks
+// one per engine.  Variant 0 follows from the size (plan_sweep, plan_batch),
+// 1 has 8-row tasks, 2 16-row tasks, 3 one-row tasks.
 constexpr int kTileVariants = 4;
-template <int NDIM, int V>
-struct TileGeom;
-template <>
-struct TileGeom<2, 0> {
-  static constexpr int CX = 32, CY = 6, CZ = 1;
+struct SweepPlan {
+  int kr, rows;
+  int warps;           // per block
+  int grid;            // blocks
+  long long list_cap;  // dirty-list entries of a block and phase
 };
-template <>
-struct TileGeom<2, 1> {
-  static constexpr int CX = 32, CY = 8, CZ = 1;
-};
-template <>
-struct TileGeom<2, 2> {
-  static constexpr int CX = 32, CY = 16, CZ = 1;
-};
-template <>
-struct TileGeom<2, 3> {
-  static constexpr int CX = 32, CY = 1, CZ = 1;
-};
-template <>
-struct TileGeom<3, 0> {
-  static constexpr int CX = 32, CY = 2, CZ = 2;
-};
-template <>
-struct TileGeom<3, 1> {
-  static constexpr int CX = 32, CY = 4, CZ = 2;
-};
-template <>
-struct TileGeom<3, 2> {
-  static constexpr int CX = 32, CY = 4, CZ = 4;
-};
-template <>
-struct TileGeom<3, 3> {
-  static constexpr int CX = 32, CY = 1, CZ = 1;
-};
-
-// Launch shape of one sweep configuration.
-struct SweepShape {
-  int variant;      // tile variant
-  int cx, cy, cz;   // its tile extent in targets
-  int warps;        // warps per block (tiles in flight per block)
-  size_t smem;      // dynamic shared memory per block
-};
-SweepShape sweep_shape(int ndim, int variant, bool scores = false);
+// One lattice over the whole grid.  wide: the extended and score kernels
+// (20 warps per block, two rows side by side).
+SweepPlan plan_sweep(int ndim, int nx, int ny, int nz, int variant, int sms, bool wide);
+// Rows of a batch's tasks (grid dispatch), total_units = 32-column rows of
+// the largest slot.
+int batch_rows(int variant, long long total_units, int sms);
 
 // ctl[] word indices (the barrier counter has a 128-byte line of its own)
 constexpr int kCtlBarrier = 0;
@@ -138,7 +95,7 @@ struct DevParams {
   // persistence (3D, src/kernels3d.cu:327-343, src/kernels.cu:159-212):
   // lambda and diffusion per type
   int persist_on;       // any persist_lambda != 0
-  int pad;
+  int small_targets;    // all target areas and perimeters within (-2^21, 2^21)
   float act_lambda[kMaxTypes];
   int act_max[kMaxTypes];
   float persist_lambda[kMaxTypes];
@@ -146,12 +103,25 @@ struct DevParams {
   int persist_time[kMaxTypes];  // stored for get/set only (not read by any kernel)
 };
 
+// Division of a 31-bit number by a side: n / d = mulhi(n, mul) >> shift, with
+// 2^l >= d, mul = floor(2^(31 + l) / d) + 1 and shift = l - 1 (Granlund and
+// Montgomery, PLDI'94).
+struct FastDiv {
+  uint32_t mul, shift;
+};
+inline FastDiv fast_div_of(uint32_t d) {  // 2 <= d < 2^31
+  uint32_t l = 1;
+  while ((1ull << l) < d) ++l;
+  return {(uint32_t)((1ull << (31 + l)) / d + 1), l - 1};
+}
+
 struct DevReplica {
   int nx, ny, nz, ncells;
   long long lat_off;   // first site of the replica in lat[]
   long long cell_off;  // table row of the replica's id 0
   int pset;            // its parameter record in params[] (shared by replicas)
   int pad;
+  FastDiv div_nx, div_plane;  // by nx and nx * ny
 };
 
 // (area, perimeter) packed in one 64-bit word: area in the low 32 bits (it
@@ -199,7 +169,8 @@ struct SweepArgs {
   unsigned long long* counters;  // [nrep][2]: evaluated, accepted
   const DevReplica* reps;
   const DevParams* params;
-  const int* task_prefix;  // [27][nrep + 1] warp tiles per slot, prefix
+  const int* task_prefix;  // (batches) [27][nrep + 1] warp tasks per slot, prefix
+  int rows, kr;            // target rows of a task, rows drawn side by side
   long long list_cap;      // entries of one dirty list of one block
   // Dispatch: 0 = the tiles of every slot over all replicas go to all warps
   // of the grid, one grid barrier per phase; 1 = each block claims whole
@@ -216,17 +187,21 @@ struct SweepArgs {
   // field[ndim * lat_off + k * sites_r + i] (null when no field exists)
   const float* field;
   // Act model: act[i] = the MCS of the last copy into site i.  With act_on
-  // (some record has an act lambda) every accepted copy is deferred: it goes
-  // to the block's pending list (site, value) and is written, with its act
-  // stamp, after the phase's barrier, so that an attempt's reads around its
-  // source (other targets of the slot) see the phase's starting state.
+  // (some record has an act lambda) an attempt also reads around its source,
+  // other targets of the slot among it, and must see the phase's starting
+  // state.  Lattice and stamps are then double-buffered like the tables: a
+  // phase reads one copy, writes its copies into the other and lists them in
+  // `pend` (two lists per block: site low, site high, value, stamp); the next
+  // phase replays them into the copy they missed.  Both copies are equal
+  // before and after a launch.
   uint32_t* act;
+  uint32_t* lat2;
+  uint32_t* act2;
   int act_on;
   // (3D persistence) preferred direction of each table row, [rows][3]
   const double* prefdir;
-  unsigned long long* pend_site;
-  uint32_t* pend_val;
-  long long pend_cap;  // entries of one block's pending list
+  uint4* pend;
+  long long pend_cap;  // entries of one pending list of one block
   // Monte Carlo time of the first MCS: tick0, or *tick_ptr when tick_ptr is
   // set (graph replays); in the latter case block 0 advances *tick_ptr by
   // mcs when the launch ends.
@@ -251,31 +226,23 @@ struct SweepArgs {
 // Message returned by cpm_last_error(NULL) for calls without a handle.
 void set_thread_error(const char* message);
 
-// Launchers (cpm_kernels.cu).  Each returns the cudaError_t of its launch.
-cudaError_t launch_sweep(int ndim, bool perim, int variant, const SweepArgs& a,
-                         int grid, cudaStream_t s, bool scores = false);
-// The row-tile sweep of one 2D lattice (cpm_sweep2d.cu): tmap points to the
-// 128-byte CUtensorMap of the variant's box (72 x row_tile_rows(variant)
-// words); use_tma = 0 stages every tile with vector loads.  At most
-// warps_cap warps per block.
-cudaError_t launch_sweep2d(bool perim, int variant, const SweepArgs& a, const void* tmap,
-                           int use_tma, int grid, int warps_cap, cudaStream_t s);
-bool row_tiles_fit(int nx, int ny);
-int row_tile_rows(int variant);
-// Cluster mode of the 2D row-tile sweep (small single lattices): plan (G
+// Launchers.  Each returns the cudaError_t of its launch.
+//
+// The sweep (cpm_sweep2d.cu, cpm_sweep3d.cu): batch = grid dispatch over the
+// replicas of a batch (a.task_prefix), else one lattice or, with
+// a.block_local, whole replicas per block.  At most `warps` warps per block.
+cudaError_t launch_sweep2d(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
+                           cudaStream_t s);
+cudaError_t launch_sweep3d(const SweepArgs& a, bool batch, int grid, int warps, cudaStream_t s);
+// Cluster sweep of a small single 2D lattice (cpm_cluster.cu): plan (G
 // blocks of one cluster, H rows per block, dirty-list entries per block)
 // and launch.  The plan is false where no cluster of that shape fits.
+bool row_tiles_fit(int nx, int ny);
 bool cluster_sweep_plan(int nx, int ny, int* G, int* H, long long* list_cap);
-cudaError_t launch_sweep2d_cluster(bool perim, int variant, const SweepArgs& a, const void* tmap,
-                                   int nx, int G, int H, cudaStream_t s);
+cudaError_t launch_sweep2d_cluster(bool perim, int variant, const SweepArgs& a, int nx, int G,
+                                   int H, cudaStream_t s);
 // Target rows per tile of the cluster sweep's variants.
 int cluster_tile_rows(int variant);
-// The 3D row-tile sweep (cpm_sweep3d.cu): boxes of 72 x rows x planes words.
-cudaError_t launch_sweep3d(bool perim, int variant, const SweepArgs& a, const void* tmap,
-                           int use_tma, int grid, int warps_cap, cudaStream_t s);
-bool box_tiles_fit(int nx, int ny, int nz);
-void box_tile_extent(int variant, int* rows, int* planes);
-int sweep_max_blocks_per_sm(int ndim, bool perim, int variant, bool scores = false);
 // checkpoints: host array of ncheck (<= kMaxCheckpoints) MCS counts.
 cudaError_t launch_lr_backward(const float* scores, const float* dl_do,
                                const float* obs, const int* checkpoints, int nrep,

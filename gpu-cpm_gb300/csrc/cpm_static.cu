@@ -172,24 +172,13 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
 
   // Launch geometry, as the engine computes it for a single replica with
   // tile variant 0.
-  const SweepShape sh = sweep_shape(ndim, 0);
-  const int tcx = sh.cx, tcy = sh.cy, tcz = sh.cz;
-  int prefix[27 * 2] = {0};
   SweepArgs a;
   std::memset(&a, 0, sizeof a);
-  long long max_tiles = 1;
   for (int slot = 0; slot < 27; ++slot) {
     const int cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
-    long long tiles = 0;
-    if (!(ndim == 2 && cz != 0)) {
-      const long long ncx = class_count_host(nx, cx), ncy = class_count_host(ny, cy),
-                      ncz = class_count_host(nz, cz);
-      if (ncx && ncy && ncz)
-        tiles = ((ncx + tcx - 1) / tcx) * ((ncy + tcy - 1) / tcy) * ((ncz + tcz - 1) / tcz);
-    }
-    prefix[slot * 2 + 1] = (int)tiles;
-    if (tiles > 0) a.slots[a.nslot_active++] = slot;
-    if (tiles > max_tiles) max_tiles = tiles;
+    if (ndim == 2 && cz != 0) continue;
+    if (class_count_host(nx, cx) && class_count_host(ny, cy) && class_count_host(nz, cz))
+      a.slots[a.nslot_active++] = slot;
   }
   int dev = 0, sms = 0;
   STATIC_CUDA(cudaGetDevice(&dev));
@@ -199,23 +188,12 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
       if (params->lambda_perimeter[k] != 0.0f) return true;
     return false;
   }();
-  const int per_sm = sweep_max_blocks_per_sm(ndim, perim_on, 0);
-  if (per_sm < 1) return fail(CPM_ERR_CUDA, "cpm_sweep_static: cannot place the sweep kernel");
-  const long long blocks_needed = (max_tiles + sh.warps - 1) / sh.warps;
-  const int grid = (int)std::max(1LL, std::min<long long>((long long)per_sm * sms, blocks_needed));
   // Dirty-list space of one block and phase: two table rows per target of
-  // the tiles it sweeps.  The single-lattice sweep gives each block one
-  // contiguous band of at most ceil(tiles / grid) tiles, and a tile holds at
-  // most min(tile extent, class size) targets along each axis, so narrow
-  // lattices (nx far below the tile width) do not pay for empty tile columns.
-  // Over every shape within CPM_STATIC_MAX_SITES the lists of a launch then
-  // need at most 516,096 entries (2D, 66 x 3890) and 337,920 (3D,
-  // 66 x 642 x 6) on 152 SMs, within kListEntries.
-  const long long eff_tile = (long long)std::min(tcx, std::max(1, class_count_host(nx, 0))) *
-                             std::min(tcy, std::max(1, class_count_host(ny, 0))) *
-                             std::min(tcz, std::max(1, class_count_host(nz, 0)));
-  const long long list_cap = 2LL * eff_tile * ((max_tiles + grid - 1) / grid);
-  if (list_cap * 2 * grid > kListEntries)
+  // the tasks it is dealt (narrow lattices do not pay for empty columns).
+  // Over every shape within CPM_STATIC_MAX_SITES the lists of a launch need
+  // at most 544,768 entries in 2D and 272,384 in 3D on 152 SMs, within kListEntries.
+  const SweepPlan plan = plan_sweep(ndim, nx, ny, nz, 0, sms, false);
+  if (plan.list_cap * 2 * plan.grid > kListEntries)
     return fail(CPM_ERR_INVALID,
                 "cpm_sweep_static: lattice shape needs more dirty-list space than the "
                 "fixed working array holds");
@@ -230,7 +208,6 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
   auto* counters = reinterpret_cast<unsigned long long*>(w + kOffCounters);
   auto* rep = reinterpret_cast<DevReplica*>(w + kOffRep);
   auto* dparams = reinterpret_cast<DevParams*>(w + kOffParams);
-  auto* dprefix = reinterpret_cast<int*>(w + kOffPrefix);
 
   // Everything the sweep expects to start at zero (the array keeps the last
   // call's contents, and a failed call may have left deltas behind).
@@ -248,6 +225,8 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
   R.cell_off = 0;
   R.pset = 0;
   R.pad = 0;
+  R.div_nx = fast_div_of((uint32_t)nx);
+  R.div_plane = fast_div_of((uint32_t)nx * (uint32_t)ny);
   DevParams P;
   std::memset(&P, 0, sizeof P);
   std::memcpy(P.J, params->J, sizeof P.J);
@@ -257,6 +236,11 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
   std::memcpy(P.tgt_perim, params->target_perimeter, sizeof P.tgt_perim);
   P.temperature = params->temperature;
   P.perim_on = perim_on ? 1 : 0;
+  P.small_targets = 1;
+  for (int k = 0; k < kMaxTypes; ++k)
+    if (std::abs((long long)P.tgt_area[k]) >= 1 << 21 ||
+        std::abs((long long)P.tgt_perim[k]) >= 1 << 21)
+      P.small_targets = 0;
   std::memcpy(P.stick, params->stickiness, sizeof P.stick);
   for (int k = 0; k < kMaxTypes * kMaxTypes; ++k)
     if (P.stick[k] != 0.0f) P.stick_on = 1;
@@ -264,7 +248,6 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
     if (params->fixed[k]) P.fixed_mask |= 1u << k;
   STATIC_CUDA(cudaMemcpyAsync(rep, &R, sizeof R, cudaMemcpyHostToDevice, s));
   STATIC_CUDA(cudaMemcpyAsync(dparams, &P, sizeof P, cudaMemcpyHostToDevice, s));
-  STATIC_CUDA(cudaMemcpyAsync(dprefix, prefix, sizeof prefix, cudaMemcpyHostToDevice, s));
 
   const int pack_grid = (int)std::min<long long>((rows + 255) / 256, 1024);
   if (recount) {
@@ -306,14 +289,16 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
     a.counters = counters;
     a.reps = rep;
     a.params = dparams;
-    a.task_prefix = dprefix;
-    a.list_cap = list_cap;
+    a.rows = plan.rows;
+    a.kr = plan.kr;
+    a.list_cap = plan.list_cap;
     a.tick0 = tick;
     a.seed = seed;
     a.nrep = 1;
     a.mcs = mcs;
     a.stream0 = stream_id;
-    STATIC_CUDA(launch_sweep(ndim, perim_on, 0, a, grid, s));
+    STATIC_CUDA(ndim == 2 ? launch_sweep2d(a, false, false, plan.grid, plan.warps, s)
+                          : launch_sweep3d(a, false, plan.grid, plan.warps, s));
   }
 
   unpack_tables<<<pack_grid, 256, 0, s>>>(ap0, area, perimeter, rows);

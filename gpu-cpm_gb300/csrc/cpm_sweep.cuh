@@ -1,0 +1,878 @@
+// cpm_sweep.cuh — the checkerboard Metropolis sweep, instantiated for 2D
+// (cpm_sweep2d.cu) and 3D (cpm_sweep3d.cu).
+//
+//   sweep_kernel<NDIM, KR, MODE, BATCH>  persistent over all MCS of a run.
+//                              Replaces copyAttempt (src/kernels2d.cu:44-583)
+//                              and copyAttempt3d (src/kernels3d.cu:51-594).
+//
+// Schedule.  Sites are coloured by their class on every axis (even / odd /
+// last coordinate of an odd axis); one phase ("slot") is one colour, and one
+// MCS runs every non-empty slot in lexicographic (cz, cy, cx) order.  All
+// targets of a slot are >= 2 apart on each axis, so an attempt never reads a
+// site another attempt of the same slot may write; the cell tables are read
+// as they stood when the slot began (double-buffered, see cpm_internal.h) and
+// the integer deltas are exact and order-free.  The result is independent of
+// thread, block and replica order, and the CPU oracle reproduces it bit for
+// bit.
+//
+// A warp takes tasks of 32 target columns x `rows` target rows:
+//   1. draw: KR rows at a time, every lane draws for its targets (KR Philox
+//      chains side by side) and reads the target and the drawn source.  A
+//      source of the target's own value ends the attempt; the others go on
+//      the warp's queue with both values.
+//   2. evaluate: whenever 32 attempts are queued, dH, Metropolis test,
+//      lattice write and table deltas, one attempt per lane.  What a warp has
+//      left when its tasks are done is pooled with the other warps' of the
+//      block, so that even a phase of few targets evaluates full batches.
+//
+// Nothing is staged: sites are read through the L1 cache, which holds what
+// the draws of a task's rows brought in when its attempts are evaluated.  A
+// phase's reads are of sites no other attempt of the phase writes, and the
+// acquire of the phase barrier (which drops the SM's L1 lines) orders them
+// after the writes of the phases before, so plain loads see them.  Against
+// warp tiles staged in shared memory (by cp.async.bulk.tensor, or a load and
+// a store per site), which needed a boundary test of every target before its
+// draw to keep the staging worth its while: 256^3 tissue, 20 MCS, 6.72 ->
+// 3.61 ms; 4096^2 tissue, 50 MCS, 8.44 -> 7.65 ms; a 101 x 75 x 61 box, 20
+// MCS, 5.09 -> 2.84 ms.
+//
+// Bound: instruction issue on large lattices (7 warp instructions per
+// attempt in 2D), the chain of one warp through a phase on small ones: draw,
+// two L2 round trips, ~400 instructions, the grid barrier (2,600 cycles, 3,200
+// with reductions outstanding).
+//
+// Launches (SweepArgs::block_local): grid dispatch deals the tasks of a slot
+// to all blocks, block b taking tasks b, b + G, b + 2G, ..., each row of tasks
+// rotated by its row index; a block's warps claim them from a shared counter.
+// One grid barrier ends each phase.  BATCH kernels do so over all replicas of
+// a batch.  Replica dispatch lets each block claim whole replicas and run all
+// their phases with block barriers.
+#pragma once
+
+#include <cstdint>
+
+#include "cpm_device.cuh"
+#include "cpm_sweep_common.cuh"
+
+namespace gpucpm {
+namespace {
+
+// What a kernel carries besides the plain terms.
+constexpr int kPlain = 0;
+constexpr int kExt = 1;    // act, 3D persistence
+constexpr int kScore = 2;  // likelihood-ratio scores (2D)
+
+// Warps per block (one block per SM): 24 at 80 registers for the plain 2D
+// sweep, 20 at 96 for the others, which would spill at 80.
+template <int NDIM, int MODE, bool BATCH>
+__host__ __device__ constexpr int sweep_warps() {
+  return NDIM == 2 && MODE == kPlain && !BATCH ? 24 : 20;
+}
+
+// An attempt to evaluate: target site, random word (its upper 24 bits) with
+// the source's direction (lower 8), source and target values.
+struct alignas(16) Attempt {
+  uint32_t site, draw, s, t;
+};
+
+template <int KR>
+__host__ __device__ constexpr int queue_len() {
+  return 32 + 32 * KR;
+}
+
+// A type's constraint parameters, one 16-byte shared-memory load.
+struct alignas(16) TypeParams {
+  float lam_area;
+  int tgt_area;
+  float lam_perim;
+  int tgt_perim;
+};
+// Words per row of the shared-memory adhesion matrix: entry (a, b) lies in
+// bank 5 a + b, so that up to five types never meet in one.
+constexpr int kJPitch = 37;
+// Dirty-list entries of a phase kept in shared memory (the rest in global
+// memory): a 4096^2 tissue pushes ~1,000 per block and phase.
+constexpr unsigned kListSmem = 2048;
+
+// What attempts need of their replica, in shared memory (one for the block,
+// in batches one per warp): kept in registers it made every kernel spill.
+struct ReplicaCtx {
+  const DevParams* P;
+  long long lat_off;
+  int rep, ncells;
+  unsigned cell_off;  // (table rows and a replica's sites < 2^31)
+  int nx, ny, nz;
+  FastDiv div_nx, div_plane;
+  float T;
+  unsigned fixed_mask;
+  int stick_on, chemo_on, perim_on, small_targets, act_on, persist_on;
+};
+
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& d) {
+  return __umulhi(n, d.mul) >> d.shift;
+}
+
+// Act model (src/kernels2d.cu:338-473, src/kernels3d.cu:347-470): the
+// geometric mean of max(amax + act[i] - tick, 0) over site (x, y, z) and
+// those of its neighbours that hold `id`, as exp2 of the mean log2 (own
+// log2_pos / exp2_own, summed in neighbour order); 0 when a factor is 0.
+// L and A are the replica's lattice and act stamps as they stood when the
+// phase began.
+template <int NDIM>
+__device__ __forceinline__ float act_mean(const uint32_t* L, const uint32_t* A, int x, int y,
+                                          int z, int nx, int ny, int nz, uint32_t id, int amax,
+                                          long long tick) {
+  auto at = [&](int xx, int yy, int zz) { return ((long long)zz * ny + yy) * nx + xx; };
+  const long long a0 = (long long)amax + (long long)A[at(x, y, z)] - tick;
+  if (a0 <= 0) return 0.0f;
+  float sum = log2_pos((float)a0);
+  int count = 1;
+  const int zlo = NDIM == 3 ? -1 : 0, zhi = NDIM == 3 ? 1 : 0;
+  for (int dz = zlo; dz <= zhi; ++dz)
+    for (int dy = -1; dy <= 1; ++dy)
+      for (int dx = -1; dx <= 1; ++dx) {
+        if (!dz && !dy && !dx) continue;
+        const long long n = at(wrap_coord(x + dx, nx), wrap_coord(y + dy, ny),
+                               NDIM == 3 ? wrap_coord(z + dz, nz) : 0);
+        if (L[n] != id) continue;
+        const long long v = (long long)amax + (long long)A[n] - tick;
+        if (v <= 0) return 0.0f;
+        sum = __fadd_rn(sum, log2_pos((float)v));
+        ++count;
+      }
+  return exp2_own(__fdiv_rn(sum, (float)count));
+}
+
+// Warp-reduces a lane's score partial sums and adds them, by lane 0, to the
+// (replica, MCS) row of the score buffer: J pairs at their index, then
+// lambda_area, lambda_perim and T in that order when enabled.  Clears the
+// partial sums.
+__device__ __forceinline__ void flush_scores(const SweepArgs& a, float* sc, int rep,
+                                             unsigned long long tick) {
+#pragma unroll
+  for (int k = 0; k < kScoreRegs; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sc[k] += __shfl_xor_sync(kFull, sc[k], o);
+  const long long row = (long long)tick - (long long)a.score_base;
+  if ((threadIdx.x & 31) == 0 && rep >= 0 && row >= 0 && row < a.score_len) {
+    float* dst = a.scores + ((long long)rep * a.score_len + row) * kScoreMax;
+    int k = 0;
+#pragma unroll
+    for (int p = 0; p < kScorePairsMax; ++p)
+      if (p < a.score_spec.n_pairs) atomicAdd(dst + k++, sc[p]);
+    if (a.score_spec.lambda_area) atomicAdd(dst + k++, sc[kScorePairsMax]);
+    if (a.score_spec.lambda_perim) atomicAdd(dst + k++, sc[kScorePairsMax + 1]);
+    if (a.score_spec.temperature) atomicAdd(dst + k++, sc[kScorePairsMax + 2]);
+  }
+#pragma unroll
+  for (int k = 0; k < kScoreRegs; ++k) sc[k] = 0.0f;
+}
+
+template <int NDIM, int KR, int MODE, bool BATCH>
+__global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
+    sweep_kernel(const __grid_constant__ SweepArgs a) {
+  constexpr bool EXT = MODE == kExt, SCORE = MODE == kScore;
+  constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
+  constexpr int QLEN = queue_len<KR>();
+  constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
+  // the pooled attempts (32 per warp), then the warps' queues
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t s_list[2][kListSmem];
+  __shared__ float s_J[BATCH ? 1 : kMaxTypes * kJPitch];
+  __shared__ TypeParams s_type[BATCH ? 1 : kMaxTypes];
+  __shared__ ReplicaCtx s_ctx[BATCH ? sweep_warps<NDIM, MODE, BATCH>() : 1];
+  __shared__ int s_ok, s_claim;
+  __shared__ unsigned s_cnt[2], s_next[2], s_pool, s_pend[2];
+  __shared__ unsigned long long s_tick0;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wpb = blockDim.x >> 5;
+  Attempt* const pool = reinterpret_cast<Attempt*>(smem_raw);
+  Attempt* const queue = pool + wpb * 32 + warp * QLEN;
+  const uint32_t k0 = (uint32_t)a.seed, k1 = (uint32_t)(a.seed >> 32);
+  int* err = reinterpret_cast<int*>(&a.ctl[kCtlErr]);
+  // A phase's dirty list: the first kListSmem entries in shared memory, the
+  // others at their index in the block's global list.
+  auto blist = [&](int b) { return a.dlist + (2LL * blockIdx.x + b) * a.list_cap; };
+  unsigned episode = 0;
+  unsigned n_eval = 0, n_acc = 0;  // of replica r, warp-uniform
+  float sc[kScoreRegs];  // (scores) the lane's sums of replica r at the running MCS
+#pragma unroll
+  for (int k = 0; k < kScoreRegs; ++k) sc[k] = 0.0f;
+  if (tid < 2) s_cnt[tid] = s_next[tid] = s_pend[tid] = 0;
+  if (tid == 0) s_pool = 0;
+  // Every block reads *tick_ptr before its first barrier arrival, and block
+  // 0 advances it only after its last barrier, so all blocks see one value.
+  if (tid == 0) s_tick0 = a.tick_ptr ? __ldcg(a.tick_ptr) : a.tick0;
+  __syncthreads();
+
+  // ---- the replica at hand ------------------------------------------------
+  ReplicaCtx& ctx = s_ctx[BATCH ? warp : 0];
+  int r = -1;
+  auto load_replica = [&](int rep) {  // one lane of the warps that share ctx
+    const DevReplica* R = a.reps + rep;
+    const DevParams* P = a.params + __ldg(&R->pset);
+    ctx.P = P;
+    ctx.lat_off = __ldg(&R->lat_off);
+    ctx.rep = rep;
+    ctx.ncells = __ldg(&R->ncells);
+    ctx.cell_off = (unsigned)__ldg(&R->cell_off);
+    ctx.nx = __ldg(&R->nx);
+    ctx.ny = __ldg(&R->ny);
+    ctx.nz = NDIM == 3 ? __ldg(&R->nz) : 1;
+    ctx.div_nx = {__ldg(&R->div_nx.mul), __ldg(&R->div_nx.shift)};
+    ctx.div_plane = {__ldg(&R->div_plane.mul), __ldg(&R->div_plane.shift)};
+    ctx.T = __ldg(&P->temperature);
+    ctx.fixed_mask = __ldg(&P->fixed_mask);
+    ctx.stick_on = __ldg(&P->stick_on);
+    ctx.chemo_on = __ldg(&P->chemo_on);
+    ctx.perim_on = __ldg(&P->perim_on);
+    ctx.small_targets = __ldg(&P->small_targets);
+    ctx.act_on = __ldg(&P->act_on);
+    ctx.persist_on = __ldg(&P->persist_on);
+  };
+  auto flush_counters = [&]() {
+    if (lane == 0 && r >= 0) {
+      if (n_eval) atomicAdd(&a.counters[2 * r], (unsigned long long)n_eval);
+      if (n_acc) atomicAdd(&a.counters[2 * r + 1], (unsigned long long)n_acc);
+    }
+    n_eval = n_acc = 0;
+  };
+
+  // Deltas of the phase with double-buffer index `prv` into the copy it read:
+  // rows of this block's dirty list (each delta is taken with an exchange, so
+  // a row listed twice is replayed once) and, in act runs, its copies.
+  auto replay_phase = [&](int prv, unsigned first) {
+    const unsigned n = min(s_cnt[prv], (unsigned)a.list_cap);  // see kErrListFull
+    unsigned long long* const dap = prv ? a.dap[1] : a.dap[0];
+    unsigned long long* const ap = prv ? a.ap[1] : a.ap[0];
+    unsigned long long* const dcs =
+        reinterpret_cast<unsigned long long*>(prv ? a.dcs[1] : a.dcs[0]);
+    unsigned long long* const cs = reinterpret_cast<unsigned long long*>(prv ? a.cs[1] : a.cs[0]);
+    for (unsigned j = first; j < n; j += blockDim.x) {
+      const long long row = j < kListSmem ? s_list[prv][j] : __ldcg(blist(prv) + j);
+      unsigned long long d[NDIM + 1];  // all exchanges issued before any add
+      d[NDIM] = atomicExch(dap + row, 0ull);
+#pragma unroll
+      for (int k = 0; k < NDIM; ++k) d[k] = atomicExch(dcs + row * NDIM + k, 0ull);
+      if (d[NDIM]) atomicAdd(ap + row, d[NDIM]);
+#pragma unroll
+      for (int k = 0; k < NDIM; ++k)
+        if (d[k]) atomicAdd(cs + row * NDIM + k, d[k]);
+    }
+    if (EXT && a.act_on) {
+      // the copies went into the other lattice copy when they were made;
+      // sites of different phases differ, so this phase's writes commute
+      const unsigned np = min(s_pend[prv], (unsigned)a.pend_cap);
+      const long long base = (2LL * blockIdx.x + prv) * a.pend_cap;
+      uint32_t* const lat = prv ? a.lat2 : a.lat;
+      uint32_t* const act = prv ? a.act2 : a.act;
+      for (unsigned j = first; j < np; j += blockDim.x) {
+        const uint4 e = __ldcg(a.pend + base + j);
+        const unsigned long long site = (unsigned long long)e.x | ((unsigned long long)e.y << 32);
+        lat[site] = e.z;
+        act[site] = e.w;
+      }
+    }
+  };
+
+  // ---- one phase ----------------------------------------------------------------
+  // G blocks share the slot's tasks, this one is number b.
+  auto run_phase = [&](const int slot, const unsigned long long tick, const int step, const int b,
+                       const int G) {
+    const int cur = step & 1;
+    PhaseTables<NDIM> pt;
+    pt.rap = cur ? a.ap[1] : a.ap[0];
+    pt.rcs = cur ? a.cs[1] : a.cs[0];
+    pt.wap = cur ? a.ap[0] : a.ap[1];
+    pt.wcs = cur ? a.cs[0] : a.cs[1];
+    pt.dap = cur ? a.dap[1] : a.dap[0];
+    pt.dcs = cur ? a.dcs[1] : a.dcs[0];
+    // the lattice (act stamps) the phase reads, and the one it writes:
+    // another copy in act runs
+    const bool two = EXT && a.act_on;
+    const uint32_t* const lat_r = two && cur ? a.lat2 : a.lat;
+    uint32_t* const lat_w = two && !cur ? a.lat2 : a.lat;
+    const uint32_t* const act_r = cur ? a.act2 : a.act;
+    uint32_t* const act_w = cur ? a.act : a.act2;
+
+    // ---- evaluate: n <= 32 attempts, one per lane -------------------------------
+    auto evaluate = [&](const Attempt* q, const int n) {
+      const uint32_t* const L = lat_r + ctx.lat_off;
+      bool accepted = false;
+      unsigned push_s = 0xFFFFFFFFu, push_t = 0xFFFFFFFFu;  // table rows this lane changed
+      if (lane < n) {
+        const uint4 e = *reinterpret_cast<const uint4*>(q + lane);
+        const uint32_t site = e.x, s = e.z, t = e.w;
+        const uint32_t is = s & 0xFFFFFFu, it = t & 0xFFFFFFu;
+        if (max(is, it) > (uint32_t)ctx.ncells) {
+          atomicOr(err, kErrBadId);
+        } else {
+          const int kdir = (int)(e.y & 0xFFu);
+          const int ts = (int)(s >> 24) & (kMaxTypes - 1);
+          const int tt = (int)(t >> 24) & (kMaxTypes - 1);
+          const unsigned rs = ctx.cell_off + is, rt = ctx.cell_off + it;
+          // (the medium's row exists; its values are not used)
+          const unsigned long long aps = __ldcg(pt.rap + rs), apt = __ldcg(pt.rap + rt);
+          // centroid sums, needed only on acceptance: in 2D fetched with the
+          // row so that an accepted attempt waits on one L2 round trip; in 3D
+          // (three words a side) on acceptance
+          constexpr bool kEarlyCs = NDIM == 2 && KR < 4;
+          long long cs_s[NDIM], cs_t[NDIM];
+          if constexpr (kEarlyCs) {
+            const longlong2 vs = __ldcg(reinterpret_cast<const longlong2*>(pt.rcs) + rs);
+            const longlong2 vt = __ldcg(reinterpret_cast<const longlong2*>(pt.rcs) + rt);
+            cs_s[0] = vs.x, cs_s[1] = vs.y, cs_t[0] = vt.x, cs_t[1] = vt.y;
+          }
+          const DevParams* const P = ctx.P;
+          const int nx = ctx.nx, ny = ctx.ny, nz = NDIM == 3 ? ctx.nz : 1;
+          const unsigned plane = (unsigned)nx * (unsigned)ny;
+          const int z = NDIM == 3 ? (int)fast_div(site, ctx.div_plane) : 0;
+          const unsigned in_plane = NDIM == 3 ? site - (unsigned)z * plane : site;
+          const int y = (int)fast_div(in_plane, ctx.div_nx),
+                    x = (int)(in_plane - (unsigned)y * nx);
+          // offsets of the neighbouring columns, rows and planes (wrapped)
+          const int xl = x ? -1 : nx - 1, xr = x + 1 < nx ? 1 : 1 - nx;
+          const int yl = y ? -nx : (int)plane - nx, yr = y + 1 < ny ? nx : nx - (int)plane;
+          const int zl = NDIM == 3 ? (z ? -(int)plane : (nz - 1) * (int)plane) : 0;
+          const int zr = NDIM == 3 ? (z + 1 < nz ? (int)plane : -(nz - 1) * (int)plane) : 0;
+          uint32_t nb[NBC];
+  #pragma unroll
+          for (int p = 0; p < (NDIM == 3 ? 3 : 1); ++p)
+  #pragma unroll
+            for (int m = 0; m < 3; ++m) {
+              const uint32_t* c = L + site + (NDIM == 3 ? (p == 0 ? zl : p == 1 ? 0 : zr) : 0) +
+                                  (m == 0 ? yl : m == 1 ? 0 : yr);
+              nb[9 * p + 3 * m] = c[xl];
+              nb[9 * p + 3 * m + 1] = c[0];
+              nb[9 * p + 3 * m + 2] = c[xr];
+            }
+          // Adhesion of both configurations, summed in neighbour order.  Every
+          // value is loaded, so that no load waits on a comparison.
+          float e_old = 0.0f, e_new = 0.0f;
+          int cnt_s = 0, cnt_t = 0;
+          unsigned by_new = 0, by_old = 0;  // (scores) neighbours by type, a byte each
+          auto adhesion = [&](const float* Jt, const float* Js, auto&& load) {
+  #pragma unroll
+            for (int k = 0; k < NBC; ++k) {
+              if (k == NB / 2) continue;  // the target itself
+              const uint32_t v = nb[k];
+              const int tn = (int)(v >> 24) & (kMaxTypes - 1);
+              const float jt = load(Jt + tn), js = load(Js + tn);
+              const bool is_t = v == t, is_s = v == s;
+              e_old = is_t ? e_old : __fadd_rn(e_old, jt);
+              e_new = is_s ? e_new : __fadd_rn(e_new, js);
+              cnt_t += is_t;
+              cnt_s += is_s;
+              if (SCORE && tn < kScoreTypes) {
+                by_new += is_s ? 0u : 1u << (8 * tn);
+                by_old += is_t ? 0u : 1u << (8 * tn);
+              }
+            }
+          };
+          if constexpr (BATCH)
+            adhesion(P->J + tt * kMaxTypes, P->J + ts * kMaxTypes,
+                     [](const float* p) { return __ldg(p); });
+          else
+            adhesion(s_J + tt * kJPitch, s_J + ts * kJPitch, [](const float* p) { return *p; });
+          if (ctx.stick_on) {
+            // stickiness of the old configuration, summed in neighbour order
+            // and added to its adhesion as one term (neighbours read again:
+            // kept past the adhesion sums they cost the other runs spills)
+            float e_st = 0.0f;
+            const float* St = P->stick + tt * kMaxTypes;
+#pragma unroll 1
+            for (int p = 0; p < (NDIM == 3 ? 3 : 1); ++p)
+#pragma unroll 1
+              for (int m = 0; m < 3; ++m) {
+                const uint32_t* c = L + site + (NDIM == 3 ? (p == 0 ? zl : p == 1 ? 0 : zr) : 0) +
+                                    (m == 0 ? yl : m == 1 ? 0 : yr);
+                const uint32_t v3[3] = {c[xl], c[0], c[xr]};
+#pragma unroll
+                for (int k = 0; k < 3; ++k)  // (the target itself holds t)
+                  if (v3[k] != t)
+                    e_st = __fadd_rn(e_st, __ldg(St + ((int)(v3[k] >> 24) & (kMaxTypes - 1))));
+              }
+            e_old = __fadd_rn(e_old, e_st);
+          }
+          float dH = __fsub_rn(e_new, e_old);
+          {
+            // chemotaxis first, as in the reference's sum; lambda of the
+            // source type, of the target type for a medium source
+            float chemo = 0.0f;
+            if (ctx.chemo_on) {
+              const float lam = __ldg(&P->chemo[ts ? ts : tt]);
+              if (lam != 0.0f)
+                chemo = __fmul_rn(-lam, chemo_dot<NDIM>(a.field + NDIM * ctx.lat_off,
+                                                        (long long)plane * nz, x, y, z, kdir, nx,
+                                                        ny, nz));
+            }
+            // persistence next (3D): lambda of the source type (target type for
+            // a medium source), preferred direction of the source cell (of the
+            // target cell for a medium source), src/kernels3d.cu:327-343
+            if (EXT && NDIM == 3 && ctx.persist_on) {
+              const float lam = __ldg(&P->persist_lambda[ts ? ts : tt]);
+              if (lam != 0.0f) {
+                float ux, uy, uz;
+                int sx, sy, sz;
+                unit_dir<NDIM>(kdir, x, y, z, nx, ny, nz, ux, uy, uz, sx, sy, sz);
+                const double* pd = a.prefdir + 3LL * (is ? rs : rt);
+                float c = __fmul_rn(ux, (float)__ldg(pd));
+                c = __fmaf_rn(uy, (float)__ldg(pd + 1), c);
+                c = __fmaf_rn(uz, (float)__ldg(pd + 2), c);
+                chemo = __fadd_rn(chemo, __fmul_rn(-lam, c));
+              }
+            }
+            // act next: lambda and max of the target type, of the source type
+            // for a medium target
+            if (EXT && ctx.act_on) {
+              const int ta = tt ? tt : ts;
+              const float lam = __ldg(&P->act_lambda[ta]);
+              const int amax_a = __ldg(&P->act_max[ta]);
+              if (lam != 0.0f && amax_a != 0) {
+                int sx, sy, sz;
+                source_coords<NDIM>(kdir, x, y, z, nx, ny, nz, sx, sy, sz);
+                const long long tk = (long long)tick;
+                const uint32_t* const A = act_r + ctx.lat_off;
+                const float tgt = t ? act_mean<NDIM>(L, A, x, y, z, nx, ny, nz, t,
+                                                     __ldg(&P->act_max[tt]), tk)
+                                    : 0.0f;
+                const float src = s ? act_mean<NDIM>(L, A, sx, sy, sz, nx, ny, nz, s,
+                                                     __ldg(&P->act_max[ts]), tk)
+                                    : 0.0f;
+                chemo = __fadd_rn(chemo, __fmul_rn(__fdiv_rn(-lam, (float)amax_a),
+                                                   __fsub_rn(src, tgt)));
+              }
+            }
+            dH = __fadd_rn(chemo, dH);
+          }
+          const int dps = NB - 2 * cnt_s;
+          const int dpt = 2 * cnt_t - NB;
+          TypeParams ps, pr;
+          if constexpr (BATCH) {
+            ps = {__ldg(&P->lam_area[ts]), __ldg(&P->tgt_area[ts]), __ldg(&P->lam_perim[ts]),
+                  __ldg(&P->tgt_perim[ts])};
+            pr = {__ldg(&P->lam_area[tt]), __ldg(&P->tgt_area[tt]), __ldg(&P->lam_perim[tt]),
+                  __ldg(&P->tgt_perim[tt])};
+          } else {
+            ps = s_type[ts];
+            pr = s_type[tt];
+          }
+          // The constraints' exact integers, rounded once to FP32.  Where the
+          // tables and targets are below 2^21, all factors are exact in FP32
+          // and so is the rounding of their product; otherwise in 64 bits.
+          float qps, qpt, qas, qat;
+          const int As = unpack_area(aps), At = unpack_area(apt);
+          const int Ps = unpack_perim(aps), Pt = unpack_perim(apt);
+          if (ctx.small_targets && (unsigned)(As | At | Ps | Pt) < (1u << 21)) {
+            qps = __fmul_rn((float)dps, (float)(2 * (Ps - ps.tgt_perim) + dps));
+            qpt = __fmul_rn((float)dpt, (float)(2 * (Pt - pr.tgt_perim) + dpt));
+            qas = (float)(1 + 2 * (As - ps.tgt_area));
+            qat = (float)(1 - 2 * (At - pr.tgt_area));
+          } else {
+            qps = __ll2float_rn((long long)dps * (2LL * (Ps - ps.tgt_perim) + dps));
+            qpt = __ll2float_rn((long long)dpt * (2LL * (Pt - pr.tgt_perim) + dpt));
+            qas = __ll2float_rn(1 + 2LL * (As - ps.tgt_area));
+            qat = __ll2float_rn(1 - 2LL * (At - pr.tgt_area));
+          }
+          if (ctx.perim_on) {
+            dH = s ? __fmaf_rn(ps.lam_perim, qps, dH) : dH;
+            dH = t ? __fmaf_rn(pr.lam_perim, qpt, dH) : dH;
+          }
+          dH = s ? __fmaf_rn(ps.lam_area, qas, dH) : dH;
+          dH = t ? __fmaf_rn(pr.lam_area, qat, dH) : dH;
+          const float T = ctx.T;
+          bool ok;
+          float ex = 1.0f;  // exp(-dH/T) when 0 <= dH and T > 0
+          if (dH < 0.0f) {
+            ok = true;
+          } else if (!(T > 0.0f)) {
+            ok = false;
+          } else {
+            const float u = __fmul_rn(__uint2float_rn((e.y >> 8) | 1u), 0x1p-24f);
+            ex = exp_neg(__fdiv_rn(-dH, T));
+            ok = u < ex;
+          }
+          if (SCORE && dH >= 0.0f && T > 0.0f) {
+            // d log P(decision) / d theta with P(accept) = min(1, exp(-dH/T)):
+            // accept: -g, reject: e/(1-e) g, g = d(dH/T)/d theta.  At
+            // dH = 0 exactly (integer parameters make it common) P has a
+            // kink, slope -g on one side and 0 on the other; the score takes
+            // the mean of the two one-sided derivatives, -g/2.
+            const float xT = dH / T;
+            const float om = xT < 1e-2f
+                                 ? xT * (1.0f - 0.5f * xT * (1.0f - (xT / 3.0f) *
+                                                                        (1.0f - 0.25f * xT)))
+                                 : 1.0f - ex;  // 1 - exp(-x)
+            const float cT = (dH == 0.0f ? -0.5f : (ok ? -1.0f : ex / om)) / T;
+  #pragma unroll
+            for (int p = 0; p < kScorePairsMax; ++p) {
+              if (p < a.score_spec.n_pairs) {
+                const int pa = a.score_spec.pair_a[p], pb = a.score_spec.pair_b[p];
+                int d = 0;
+                if (ts == pa) d += (by_new >> (8 * pb)) & 0xFF;
+                if (pa != pb && ts == pb) d += (by_new >> (8 * pa)) & 0xFF;
+                if (tt == pa) d -= (by_old >> (8 * pb)) & 0xFF;
+                if (pa != pb && tt == pb) d -= (by_old >> (8 * pa)) & 0xFF;
+                sc[p] += cT * (float)d;
+              }
+            }
+            if (a.score_spec.lambda_area) {
+              const int da = (s ? 1 + 2 * (As - ps.tgt_area) : 0) +
+                             (t ? 1 - 2 * (At - pr.tgt_area) : 0);
+              sc[kScorePairsMax] += cT * (float)da;
+            }
+            if (a.score_spec.lambda_perim) {
+              const long long dp =
+                  (s ? (long long)dps * (2LL * (Ps - ps.tgt_perim) + dps) : 0LL) +
+                  (t ? (long long)dpt * (2LL * (Pt - pr.tgt_perim) + dpt) : 0LL);
+              sc[kScorePairsMax + 1] += cT * __ll2float_rn(dp);
+            }
+            if (a.score_spec.temperature) sc[kScorePairsMax + 2] -= cT * xT;
+          }
+          if (ok) {
+            accepted = true;
+            lat_w[ctx.lat_off + site] = s;
+            if (EXT && a.act_on) {  // into this copy in the next phase
+              act_w[ctx.lat_off + site] = (uint32_t)tick;
+              const unsigned j = atomicAdd(&s_pend[cur], 1u);
+              if ((long long)j < a.pend_cap) {
+                const unsigned long long g = (unsigned long long)ctx.lat_off + site;
+                a.pend[(2LL * blockIdx.x + cur) * a.pend_cap + j] =
+                    make_uint4((uint32_t)g, (uint32_t)(g >> 32), s, (uint32_t)tick);
+              } else {
+                atomicOr(err, kErrListFull);  // reported, never written past the end
+              }
+            }
+            const int crd[3] = {x, y, z};
+            const int dim[3] = {nx, ny, nz};
+            long long img[NDIM];
+            if (s) {
+  #pragma unroll
+              for (int k = 0; k < NDIM; ++k)
+                img[k] = nearest_image(
+                    crd[k], dim[k], As,
+                    kEarlyCs ? cs_s[k] : __ldcg(pt.rcs + (long long)rs * NDIM + k));
+              add_delta<NDIM>(pt, rs, 1, dps, img, 1);
+              push_s = rs;
+            }
+            if (t) {
+  #pragma unroll
+              for (int k = 0; k < NDIM; ++k)
+                img[k] = nearest_image(
+                    crd[k], dim[k], At,
+                    kEarlyCs ? cs_t[k] : __ldcg(pt.rcs + (long long)rt * NDIM + k));
+              add_delta<NDIM>(pt, rt, -1, dpt, img, -1);
+              push_t = rt;
+            }
+          }
+        }
+      }
+      n_acc += __popc(__ballot_sync(kFull, accepted));
+      // the changed rows onto the block's dirty list: one shared-memory
+      // atomic per batch
+      const unsigned bs = __ballot_sync(kFull, push_s != 0xFFFFFFFFu);
+      const unsigned bt = __ballot_sync(kFull, push_t != 0xFFFFFFFFu);
+      if (bs | bt) {  // warp-uniform
+        const unsigned npush = (unsigned)(__popc(bs) + __popc(bt));
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&s_cnt[cur], npush);
+        at = __shfl_sync(kFull, at, 0);
+        // The host sizes the lists for two rows per attempt; a list that
+        // would still overflow is reported, never written past its end.
+        if ((long long)at + npush > a.list_cap) {
+          if (lane == 0) atomicOr(err, kErrListFull);
+        } else {
+          auto put = [&](unsigned i, unsigned row) {
+            if (i < kListSmem)
+              s_list[cur][i] = row;
+            else
+              blist(cur)[i] = row;
+          };
+          if (push_s != 0xFFFFFFFFu) put(at + __popc(bs & lanemask_lt()), push_s);
+          if (push_t != 0xFFFFFFFFu) put(at + __popc(bs) + __popc(bt & lanemask_lt()), push_t);
+        }
+      }
+    };
+
+    const int cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
+    const unsigned long long phase = tick * NSLOTS + (unsigned long long)slot;
+    const int rows = a.rows;
+    int nx = 0, ny = 0, nz = 1;
+    unsigned fixed_mask = 0;
+    const uint32_t* L = lat_r;
+    auto enter = [&]() {  // the constants of the replica in ctx
+      r = ctx.rep;
+      nx = ctx.nx;
+      ny = ctx.ny;
+      nz = NDIM == 3 ? ctx.nz : 1;
+      fixed_mask = ctx.fixed_mask;
+      L = lat_r + ctx.lat_off;
+    };
+    if (!BATCH || r >= 0) enter();
+    int ncx = 0, ncy = 0, tnx = 1, tny = 1, ntasks;
+    auto task_grid = [&]() {
+      ncx = class_count(nx, cx);
+      ncy = class_count(ny, cy);
+      tnx = (ncx + 31) >> 5;
+      tny = (ncy + rows - 1) / rows;
+    };
+    const int* pre = nullptr;  // (batches) tasks of the slot before each replica
+    if constexpr (BATCH) {
+      pre = a.task_prefix + slot * (a.nrep + 1);
+      ntasks = __ldg(pre + a.nrep);
+    } else {
+      task_grid();
+      ntasks = tnx * tny * class_count(nz, cz);
+    }
+    unsigned* ctr = &s_next[step & 1];
+    if (tid == 0) s_next[(step + 1) & 1] = 0u;
+    int nq = 0, task = b + warp * G;
+    int j = 0, j1 = -1;  // next target row of the task, its end (-1: no task yet)
+    int x = 0, z = 0;    // the lane's column
+    bool in_x = false;
+    int next_rep = -1;       // (batches) the replica of the task at hand
+    bool rep_ready = !BATCH;  // its constants are loaded
+    int pool_at = -1, pool_n = 0;  // pooled stage: this warp's next batch, all attempts
+    for (;;) {
+      const Attempt* batch = queue;
+      int nbatch = 0;
+      while (pool_at < 0) {
+        if (nq >= 32) {  // the last 32
+          nq -= 32;
+          batch = queue + nq;
+          nbatch = 32;
+          break;
+        }
+        if (j >= j1) {  // the next task
+          if (j1 >= 0) {
+            unsigned v = 0;
+            if (lane == 0) v = atomicAdd(ctr, 1u);
+            task = b + (wpb + (int)__shfl_sync(kFull, v, 0)) * G;
+          }
+          j = 0;
+          j1 = 0;
+          if (task >= ntasks) {
+            if constexpr (BATCH) {  // what is left of the warp's last replica
+              pool_at = 0;
+              pool_n = nq;
+              break;
+            }
+            unsigned at = 0;
+            if (lane == 0 && nq) at = atomicAdd(&s_pool, (unsigned)nq);
+            at = __shfl_sync(kFull, at, 0);
+            if (lane < nq)
+              *reinterpret_cast<uint4*>(pool + at + lane) =
+                  *reinterpret_cast<const uint4*>(queue + lane);
+            __syncthreads();
+            pool_n = (int)s_pool;
+            pool_at = warp * 32;
+            break;
+          }
+          if constexpr (BATCH) {
+            int lo = 0, hi = a.nrep - 1;  // the largest with pre[lo] <= task
+            while (lo < hi) {
+              const int mid = (lo + hi + 1) >> 1;
+              if (__ldg(pre + mid) <= task) lo = mid; else hi = mid - 1;
+            }
+            next_rep = lo;
+            rep_ready = false;
+            j1 = 1;  // a task is at hand
+          }
+        }
+        if constexpr (BATCH) {
+          if (!rep_ready) {
+            const int rep = a.rep_map ? __ldg(a.rep_map + next_rep) : next_rep;
+            if (rep != r) {
+              if (nq > 0) {  // the last replica's attempts first
+                nbatch = nq;
+                nq = 0;
+                break;
+              }
+              if (SCORE && r >= 0) flush_scores(a, sc, r, tick);
+              flush_counters();
+              __syncwarp();
+              if (lane == 0) load_replica(rep);
+              __syncwarp();
+              enter();
+            }
+            task_grid();
+            rep_ready = true;
+            j1 = 0;
+          }
+        }
+        if (j1 == 0) {  // the task's place
+          const int local = BATCH ? task - __ldg(pre + next_rep) : task;
+          const int rest = local / tnx;
+          const int tx = (local - rest * tnx + rest) % tnx;
+          const int tz = NDIM == 3 ? rest / tny : 0, ty = rest - tz * tny;
+          j = ty * rows;
+          j1 = min(ncy, j + rows);
+          in_x = tx * 32 + lane < ncx;
+          x = in_x ? class_coord(nx, cx, tx * 32 + lane) : 0;
+          z = NDIM == 3 ? class_coord(nz, cz, tz) : 0;
+        }
+        const unsigned plane = (unsigned)nx * (unsigned)ny;
+        uint32_t c[KR][4], site[KR], tv[KR], sv[KR];
+        int ys[KR], kd[KR];
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          ys[u] = class_coord(ny, cy, min(j + u, j1 - 1));
+          site[u] = (unsigned)z * plane + (unsigned)ys[u] * (unsigned)nx + (unsigned)x;
+          tv[u] = L[site[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          c[u][0] = site[u];
+          c[u][1] = (uint32_t)phase;
+          c[u][2] = a.stream0 + (uint32_t)r;
+          c[u][3] = (uint32_t)(phase >> 32);
+          philox4x32_10(c[u][0], c[u][1], c[u][2], c[u][3], k0, k1);
+        }
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          kd[u] = (int)__umulhi(c[u][0], (unsigned)NB);
+          int sx, sy, sz;
+          source_coords<NDIM>(kd[u], x, ys[u], z, nx, ny, nz, sx, sy, sz);
+          sv[u] = L[(NDIM == 3 ? (unsigned)sz * plane : 0u) + (unsigned)sy * (unsigned)nx +
+                    (unsigned)sx];
+        }
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          uint32_t s = sv[u];
+          bool keep = in_x && j + u < j1 && s != tv[u];
+          if (fixed_mask && keep) {
+            // a target of a fixed type never changes; a source of a fixed type
+            // proposes the medium instead (src/kernels2d.cu:280-290)
+            if ((fixed_mask >> ((tv[u] >> 24) & (kMaxTypes - 1))) & 1u) {
+              keep = false;
+            } else if ((fixed_mask >> ((s >> 24) & (kMaxTypes - 1))) & 1u) {
+              s = 0u;
+              keep = tv[u] != 0u;
+            }
+          }
+          const unsigned ball = __ballot_sync(kFull, keep);
+          if (keep)
+            *reinterpret_cast<uint4*>(queue + nq + __popc(ball & lanemask_lt())) =
+                make_uint4(site[u], (c[u][1] & 0xFFFFFF00u) | (uint32_t)kd[u], s, tv[u]);
+          nq += __popc(ball);
+          n_eval += __popc(ball);
+        }
+        j += KR;
+        __syncwarp();
+      }
+      if (pool_at >= 0) {
+        if (pool_at >= pool_n) break;
+        batch = (BATCH ? queue : pool) + pool_at;
+        nbatch = min(32, pool_n - pool_at);
+        pool_at += BATCH ? pool_n : wpb * 32;
+      }
+      evaluate(batch, nbatch);
+      __syncwarp();  // the queue is rewritten next
+    }
+    if (SCORE && BATCH && r >= 0) flush_scores(a, sc, r, tick);
+  };
+
+  // All MCS of the launch over the lattice or batch (this block is number b
+  // of G), or over each replica that this block claims (G = 1; block barriers
+  // between its phases).  The first grid barrier of replica dispatch makes
+  // every block read the starting tick before block 0 can advance it.
+  const bool local = !BATCH && a.block_local;
+  const int G = local ? 1 : (int)gridDim.x, b = local ? 0 : (int)blockIdx.x;
+  if (local && !grid_barrier(a.ctl, ++episode, &s_ok)) return;
+  for (;;) {
+    if constexpr (!BATCH) {
+      if (tid == 0) {
+        const int qi = local ? (int)atomicAdd(&a.ctl[kCtlQueue], 1u) : 0;
+        s_claim = qi;
+        if (!local || qi < a.queue_len) load_replica(local ? __ldg(a.rep_order + qi) : 0);
+      }
+      __syncthreads();
+      if (local && s_claim >= a.queue_len) break;  // block-uniform
+      const DevParams* const P = ctx.P;
+      for (int i = tid; i < kMaxTypes * kMaxTypes; i += blockDim.x)
+        s_J[(i / kMaxTypes) * kJPitch + i % kMaxTypes] = __ldg(&P->J[i]);
+      for (int i = tid; i < kMaxTypes; i += blockDim.x)
+        s_type[i] = {__ldg(&P->lam_area[i]), __ldg(&P->tgt_area[i]), __ldg(&P->lam_perim[i]),
+                     __ldg(&P->tgt_perim[i])};
+      __syncthreads();
+    }
+    int step = 0;
+    for (int m = 0; m < a.mcs; ++m) {
+      const unsigned long long tick = s_tick0 + (unsigned long long)m;
+      for (int si = 0; si < a.nslot_active; ++si, ++step) {
+        const int prv = (step & 1) ^ 1;
+        // from the last thread down: the first warps have the first tasks
+        if (step > 0) replay_phase(prv, blockDim.x - 1 - tid);
+        run_phase(a.slots[si], tick, step, b, G);
+        __syncthreads();
+        if (tid == 0) {
+          s_cnt[prv] = s_pend[prv] = 0;
+          s_pool = 0;
+        }
+        if (local)
+          __syncthreads();
+        else if (!grid_barrier(a.ctl, ++episode, &s_ok))
+          return;
+      }
+      if (SCORE && !BATCH) flush_scores(a, sc, r, tick);
+      if (n_eval > (1u << 30)) flush_counters();  // (a phase adds less than 2^31)
+    }
+    // Final replay: the last phase's deltas into the copy it read, so that
+    // both copies agree when the launch ends.
+    if (step > 0) replay_phase((step - 1) & 1, tid);
+    flush_counters();
+    if (!local) break;
+    __syncthreads();
+    if (tid < 2) s_cnt[tid] = s_next[tid] = s_pend[tid] = 0;
+    __syncthreads();
+  }
+  if (a.tick_ptr && a.tick_advance && blockIdx.x == 0 && tid == 0 && a.mcs > 0)
+    *a.tick_ptr = s_tick0 + (unsigned long long)a.mcs;
+}
+
+template <int NDIM, int KR, int MODE, bool BATCH>
+struct SweepFn {
+  static const void* fn() { return (const void*)sweep_kernel<NDIM, KR, MODE, BATCH>; }
+  static size_t smem(int warps) { return sizeof(Attempt) * (size_t)warps * (32 + queue_len<KR>()); }
+};
+
+template <int NDIM, int KR, int MODE, bool BATCH>
+cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_t s) {
+  using F = SweepFn<NDIM, KR, MODE, BATCH>;
+  const int w = warps < sweep_warps<NDIM, MODE, BATCH>() ? warps
+                                                         : sweep_warps<NDIM, MODE, BATCH>();
+  const size_t smem = F::smem(w);
+  const cudaError_t e =
+      cudaFuncSetAttribute(F::fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {const_cast<SweepArgs*>(&a)};
+  return cudaLaunchCooperativeKernel(F::fn(), dim3(grid), dim3(32 * w), args, smem, s);
+}
+
+// One kernel per mode and rows drawn side by side (a.kr; the extended, score
+// and batch kernels have two).
+template <int NDIM>
+cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
+                            cudaStream_t s) {
+  const bool ext = a.act_on || a.prefdir;
+  if (batch) {
+    if (ext) return launch_sweep_as<NDIM, 2, kExt, true>(a, grid, warps, s);
+    if constexpr (NDIM == 2) {
+      if (scores) return launch_sweep_as<NDIM, 2, kScore, true>(a, grid, warps, s);
+    }
+    return launch_sweep_as<NDIM, 2, kPlain, true>(a, grid, warps, s);
+  }
+  if (ext) return launch_sweep_as<NDIM, 2, kExt, false>(a, grid, warps, s);
+  if constexpr (NDIM == 2) {
+    if (scores) return launch_sweep_as<NDIM, 2, kScore, false>(a, grid, warps, s);
+  }
+  switch (a.kr) {
+    case 1: return launch_sweep_as<NDIM, 1, kPlain, false>(a, grid, warps, s);
+    case 4: return launch_sweep_as<NDIM, 4, kPlain, false>(a, grid, warps, s);
+    default: return launch_sweep_as<NDIM, 2, kPlain, false>(a, grid, warps, s);
+  }
+}
+
+}  // namespace
+}  // namespace gpucpm

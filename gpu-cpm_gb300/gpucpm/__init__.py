@@ -27,8 +27,8 @@ Differences from the reference, all deliberate:
     doubles) and the chemotaxis energy is summed in FP32, rounded step by
     step; get_field's array exists whether or not has_field was set.
   * the act model's geometric means use this library's own FP32 log2 /
-    exp2 (the reference uses the fast __powf), and copies of runs with an
-    act lambda are written at the end of their phase (see cpm_set_act).
+    exp2 (the reference uses the fast __powf), and attempts of runs with an
+    act lambda read the phase's starting state (see cpm_set_act).
   * persistence (3D only, as in the reference) draws the initial preferred
     directions from (seed, stream) instead of std::random_device, and its
     energy is summed in FP32 like chemotaxis.  Cpm.run makes one engine run
@@ -500,9 +500,9 @@ class _Engine:
         return v.value, ms.value
 
     def set_variant(self, variant):
-        """Warp tile in targets: 0 = 32x6 (3D 32x2x2), 1 = 32x8 (32x4x2),
-        2 = 32x16 (32x4x4), 3 = 32x1 (32x1x1, for lattices too small to
-        give every warp a wider tile).  The result does not depend on it."""
+        """Target rows of a warp task (32 columns wide): 0 = by the lattice's
+        size, 1 = 8, 2 = 16 (a batch: 32), 3 = 1 (a batch: 2).  The result
+        does not depend on it."""
         self._call("cpm_set_variant", int(variant))
 
     def set_dispatch(self, dispatch):
@@ -559,8 +559,8 @@ class _Engine:
 
     @property
     def fill(self):
-        """How the sweep stages its tiles: FILL_PARITY, FILL_VECTOR, FILL_TMA
-        or FILL_CLUSTER (see cpm_set_fill)."""
+        """The sweep's kernel: FILL_CLUSTER, or FILL_PARITY, FILL_VECTOR or
+        FILL_TMA, which are one (see cpm_set_fill)."""
         f = ctypes.c_int()
         self._call("cpm_get_fill", ctypes.byref(f))
         return f.value

@@ -120,9 +120,9 @@ int cpm_set_adhesion_r(cpm_handle* h, int replica, int type, int other,
  * max(max_act + act - mcs, 0) over the site and its neighbours of the same
  * cell (0 for the medium), act being the MCS of the last copy into a site;
  * here computed as exp2 of the mean log2 with this library's own FP32 log2 /
- * exp2.  Copies of runs with an act lambda are written at the end of their
- * phase, so that every attempt reads the phase's starting state; such runs
- * use tile variant 0 and cannot accumulate scores. */
+ * exp2.  Runs with an act lambda keep two copies of lattice and
+ * stamps, so that every attempt reads the phase's starting state; they cannot
+ * accumulate scores. */
 int cpm_set_act(cpm_handle* h, int type, int max_act, float lambda);
 int cpm_set_act_r(cpm_handle* h, int replica, int type, int max_act, float lambda);
 
@@ -323,14 +323,13 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
                      int* tile_y, int* tile_z, int* warps_per_block,
                      int* grid, int* dispatch);
 
-/* How warp tiles reach shared memory in the sweep of one lattice.  No
- * counterpart in the reference (its tile load is src/kernels2d.cu:109-176).
- *   CPM_FILL_PARITY  the general sweep: scalar loads, even and odd columns
- *                    in separate halves of the tile
- *   CPM_FILL_VECTOR  row-major tiles from 16-byte vector loads
- *   CPM_FILL_TMA     row-major tiles, interior tiles copied by the tensor
- *                    memory accelerator (cp.async.bulk.tensor), tiles on the
- *                    periodic seam from vector loads
+/* The kernel of the sweep of one lattice.  No counterpart in the reference
+ * (its tile load is src/kernels2d.cu:109-176).
+ *   CPM_FILL_PARITY, CPM_FILL_VECTOR, CPM_FILL_TMA
+ *                    the sweep over the whole GPU, which reads sites through
+ *                    the L1 cache; the three names once chose how it staged
+ *                    tiles in shared memory, are still accepted and select
+ *                    the same kernel
  *   CPM_FILL_CLUSTER (small 2D lattices) one thread-block cluster of 16 (or 8)
  *                    blocks holds the lattice in its shared memory, one
  *                    strip of rows per block with copies of its neighbours'
@@ -338,10 +337,9 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
  *                    and the phases end at a barrier inside the cluster.
  *                    cpm_autotune tries it wherever it fits and keeps it
  *                    when it is faster.
- * Row-major tiles need a single lattice with nx a multiple of 4 and
- * nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18); such lattices start
- * in CPM_FILL_TMA (CPM_FILL_VECTOR where the tensor maps cannot be encoded),
- * all others in CPM_FILL_PARITY.
+ * CPM_FILL_VECTOR and CPM_FILL_TMA need a single lattice with nx a multiple of
+ * 4 and nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18); such lattices
+ * start in CPM_FILL_TMA, all others in CPM_FILL_PARITY.
  * The result does not depend on the fill: it selects the kernel only
  * (CPM_ERR_UNSUPPORTED for a fill the lattice cannot use). */
 #define CPM_FILL_PARITY 0

@@ -1,0 +1,57 @@
+"""The sweep at the sizes where its plan changes, against the oracle bit for
+bit: one, two and four rows of targets drawn side by side, several tasks per
+warp, one target per task, lattices one task wide or a few rows high, odd
+sides, every tile variant; and targets so large that a constraint's integers
+no longer fit FP32."""
+import numpy as np
+import pytest
+
+import oracle
+from gpucpm import workloads as W
+from test_gpu_parity import assert_same, finish, make_engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(w, mcs, variant=0, seed=5):
+    e = make_engine(w, seed=seed)
+    e.set_variant(variant)
+    e.run_mcs(mcs)
+    finish(e)
+    sim = oracle.OracleSim(w.lattice, w.ncells, **w.oracle_kwargs(), seed=seed).run(mcs)
+    assert_same(e, sim)
+    assert int(sim.counters[2]) > 0
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("shape,ncells,mcs", [
+    ((3, 5), 2, 40), ((2001, 5), 60, 4), ((5, 2003), 60, 4), ((67, 65), 25, 8),
+    ((4, 6, 3), 3, 30), ((3, 7, 70), 20, 8), ((35, 3, 33), 30, 8),
+])
+def test_narrow_and_odd_shapes(engine_lib, shape, ncells, mcs, variant):
+    _check(W.random_small(shape, ncells, seed=40 + ncells, temperature=12.0), mcs, variant)
+
+
+@pytest.mark.parametrize("shape,mcs", [
+    ((570, 1024), 3),        # two rows side by side
+    ((1301, 1025), 2),       # four rows, one task per warp, odd sides
+    ((4000, 2000), 1),       # 8-row tasks, several per warp
+    ((135, 136, 64), 2),     # 3D, two rows
+    ((200, 201, 63), 1),     # 3D, four rows, odd
+    ((312, 314, 128), 1),    # 3D, 8-row tasks
+])
+def test_plans_by_size(engine_lib, shape, mcs):
+    ncells = int(np.prod(shape)) // (200 if len(shape) == 2 else 800)
+    _check(W.random_small(shape, ncells, ntypes=3, seed=len(shape), temperature=10.0), mcs)
+
+
+@pytest.mark.parametrize("shape", [(40, 50), (16, 14, 18)])
+@pytest.mark.parametrize("target", [2**21 - 1, 2**21, -2**21, 2**24 + 1])
+def test_targets_beyond_fp32_integers(engine_lib, shape, target):
+    w = W.random_small(shape, 20, seed=9, temperature=15.0)
+    w.tgt_area = w.tgt_area.copy()
+    w.tgt_perim = w.tgt_perim.copy()
+    w.lam_area = w.lam_area * np.float32(1e-7)
+    w.lam_perim = w.lam_perim * np.float32(1e-7)
+    w.tgt_area[1], w.tgt_perim[2] = target, target
+    _check(w, 6)
