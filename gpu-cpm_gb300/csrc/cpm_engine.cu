@@ -164,16 +164,16 @@ struct cpm_handle {
   } cfg[kTileVariants];
   int variant = 0;
   int dispatch = CPM_DISPATCH_GRID;  // CPM_DISPATCH_*
-  // CPM_FILL_*: CPM_FILL_CLUSTER runs the cluster sweep (cpm_cluster.cu), the
-  // others the same sweep (cpm_sweep.cuh); row_ok: the shapes that once had
-  // row tiles, which accept CPM_FILL_VECTOR and CPM_FILL_TMA
+  // CPM_FILL_*.  Until the caller or the autotuner chooses one (fill_auto) the
+  // engine runs the cluster sweep (cpm_cluster.cu) on small lattices that fit
+  // it, else the grid sweep (cpm_sweep.cuh); CPM_FILL_CLUSTER asks for the cluster sweep,
+  // the other fills for the grid sweep.  row_ok: the shapes that accept
+  // CPM_FILL_VECTOR and CPM_FILL_TMA; cluster_fill: those that accept
+  // CPM_FILL_CLUSTER.
   int fill = CPM_FILL_PARITY;
-  bool row_ok = false;
-  // CPM_FILL_CLUSTER: small 2D lattices swept by one thread-block cluster of
-  // cl_G blocks, cl_H rows each, dirty lists of cl_cap entries per block
-  bool cluster_ok = false;
-  int cl_G = 0, cl_H = 0;
-  long long cl_cap = 0;
+  bool fill_auto = true;
+  bool row_ok = false, cluster_fill = false;
+  int cluster_blocks = 0;  // blocks of the cluster that holds the lattice (0: none)
   std::vector<unsigned long long> attempts;  // per replica, host-counted
 
   // Graph-captured run (cpm_run_graph): the captured launch reads and
@@ -270,7 +270,19 @@ void free_all(cpm_handle* h) {
 
 // Shapes that accept CPM_FILL_VECTOR and CPM_FILL_TMA.
 bool rows_fit(int ndim, int nx, int ny, int nz) {
-  return ndim == 2 ? row_tiles_fit(nx, ny) : nx % 4 == 0 && nx >= 72 && ny >= 18 && nz >= 18;
+  return nx % 4 == 0 && nx >= 72 && (ndim == 2 ? ny >= 66 : ny >= 18 && nz >= 18);
+}
+// Shapes that accept CPM_FILL_CLUSTER: about 190 KB of rows per block of a
+// 16-block cluster.
+bool cluster_fits(int nx, int ny) {
+  if (!rows_fit(2, nx, ny, 1)) return false;
+  for (int g : {16, 8}) {
+    const long long h = (ny + g - 1) / g;
+    const long long strip = (((h + 2) * (nx + 8) + 31) & ~31LL) * 4;
+    const long long lists = 8 * (64LL * (((nx >> 1) + 31) / 32) * (h / 2 + 8));
+    if (strip + lists + 23040 <= kSweepSmemMax - 1024) return true;
+  }
+  return false;
 }
 
 void default_params(DevParams& p, float T) {
@@ -398,9 +410,9 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
   if (n == 1 && rows_fit(ndim, nx[0], ny[0], nz ? nz[0] : 1)) {
     h->row_ok = true;
     h->fill = CPM_FILL_TMA;
-    if (ndim == 2)
-      h->cluster_ok = cluster_sweep_plan(nx[0], ny[0], &h->cl_G, &h->cl_H, &h->cl_cap);
+    if (ndim == 2) h->cluster_fill = cluster_fits(nx[0], ny[0]);
   }
+  if (n == 1 && ndim == 2) h->cluster_blocks = cluster_sweep_blocks(nx[0], ny[0], ncells[0]);
 
   // One launch configuration per tile variant: warp tasks per slot and
   // replica (prefix over replicas), grid, dirty-list capacity.
@@ -808,12 +820,6 @@ int upload_params(cpm_handle* h) {
   return CPM_OK;
 }
 
-bool any_perimeter(const cpm_handle* h) {
-  for (size_t i = 0; i < h->psets.size(); ++i)
-    if (h->pset_refs[i] > 0 && perim_on(h->psets[i])) return true;
-  return false;
-}
-
 // Kernel arguments of a sweep with tile variant v and dispatch d (tick0 /
 // mcs, and what depends on the launch, filled in by the caller).
 SweepArgs sweep_args(const cpm_handle* h, int v) {
@@ -863,13 +869,25 @@ const SweepPlan& plan_of(const cpm_handle* h, int v, int d, bool scores = false)
 
 int grid_of(const cpm_handle* h, int v, int d) { return plan_of(h, v, d).grid; }
 
+int fill_key(const cpm_handle* h) { return h->fill_auto ? -2 : h->fill; }
+
+// Whether plain runs take the cluster sweep.
+// By itself up to the size where the grid sweep, whose phases take 4.8 us
+// whatever the size, overtakes its 16 SMs (us per MCS, grid / cluster: 350^2
+// 19.5 / 16.7, 400^2 19.2 / 20.4).
+constexpr long long kClusterAutoSites = 140000;
+bool uses_cluster(const cpm_handle* h) {
+  return h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
+         (h->fill_auto ? h->total_sites <= kClusterAutoSites : h->fill == CPM_FILL_CLUSTER);
+}
+
 // The launches of one sweep run (`a` from sweep_args, times filled in): one
 // launch for GRID and REPLICA, two for HYBRID (grid dispatch over the first
 // hyb_ng replicas of rep_order, then replica dispatch over the rest).  Each
 // launch starts with its barrier words cleared.  Returns the number of
 // launches through *nlaunch.
-cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a, bool perim,
-                          bool scores, int* nlaunch) {
+cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a, bool scores,
+                          int* nlaunch) {
   const cpm_handle::Config& c = h->cfg[v];
   *nlaunch = 0;
   if (h->act_active) {  // both lattice and stamp copies start equal
@@ -880,12 +898,13 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
     if (e != cudaSuccess) return e;
   }
   auto one = [&](SweepArgs x, const SweepPlan& p, bool batch) {
-    cudaError_t e = cudaMemsetAsync(h->d_ctl, 0, sizeof(uint32_t) * kCtlErr, h->stream);
-    if (e != cudaSuccess) return e;
-    if (h->fill == CPM_FILL_CLUSTER && !scores && !h->act_active && !h->persist_active) {
-      x.list_cap = h->cl_cap;
-      e = launch_sweep2d_cluster(perim, v, x, h->reps[0].nx, h->cl_G, h->cl_H, h->stream);
+    cudaError_t e;
+    if (uses_cluster(h) && !scores) {  // (no grid barrier, no queue)
+      const DevReplica& R = h->reps[0];
+      e = launch_cluster_sweep(x, R.nx, R.ny, R.ncells, h->cluster_blocks, h->stream);
     } else {
+      e = cudaMemsetAsync(h->d_ctl, 0, sizeof(uint32_t) * kCtlErr, h->stream);
+      if (e != cudaSuccess) return e;
       x.rows = p.rows;
       x.kr = p.kr;
       x.list_cap = p.list_cap;
@@ -1406,7 +1425,6 @@ int cpm_run(cpm_handle* h, int mcs) {
   if (!h->pushed) return h->fail(CPM_ERR_STATE, "run() before a successful push_to_gpu()");
   if (mcs == 0) return CPM_OK;
   if (int rc = upload_params(h)) return rc;
-  const bool any_perim = any_perimeter(h);
   SweepArgs a = sweep_args(h, h->variant);
   int left = mcs;
   while (left > 0) {
@@ -1416,7 +1434,7 @@ int cpm_run(cpm_handle* h, int mcs) {
     // Barrier counter and release flag start at zero in every launch; the
     // sticky error word is left alone until cpm_synchronize reads it.
     int nl = 0;
-    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, any_perim, false, &nl));
+    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, false, &nl));
     h->launches += nl;
     h->tick += (uint64_t)chunk;
     left -= chunk;
@@ -1435,7 +1453,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     return h->fail(CPM_ERR_STATE, "graph runs need a non-default stream");
   if (int rc = upload_params(h)) return rc;
   if (!h->graph_exec || h->graph_mcs != mcs || h->graph_variant != h->variant ||
-      h->graph_dispatch != h->dispatch || h->graph_fill != h->fill ||
+      h->graph_dispatch != h->dispatch || h->graph_fill != fill_key(h) ||
       h->graph_stream != h->stream) {
     if (h->graph_exec) {
       cudaGraphExecDestroy(h->graph_exec);
@@ -1449,7 +1467,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     cudaGraph_t g = nullptr;
     CPM_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int nl = 0;
-    cudaError_t e2 = enqueue_sweep(h, h->variant, h->dispatch, a, any_perimeter(h), false, &nl);
+    cudaError_t e2 = enqueue_sweep(h, h->variant, h->dispatch, a, false, &nl);
     cudaError_t e3 = cudaStreamEndCapture(h->stream, &g);
     if (e2 != cudaSuccess) return h->cuda_fail(e2, "capture of the sweep launch");
     if (e3 != cudaSuccess) return h->cuda_fail(e3, "cudaStreamEndCapture");
@@ -1460,7 +1478,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     h->graph_launches = nl;
     h->graph_variant = h->variant;
     h->graph_dispatch = h->dispatch;
-    h->graph_fill = h->fill;
+    h->graph_fill = fill_key(h);
     h->graph_stream = h->stream;
   }
   if (h->d_tick_stale) {
@@ -1519,7 +1537,6 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   const uint64_t tick = h->tick;
   float best = -1.0f;
   int best_v = h->variant, best_d = h->dispatch;
-  const bool any_perim = any_perimeter(h);
   // Every (tile variant, dispatch) pair, replica dispatch only for batches,
   // timed in three rounds (the fastest run counts): a variant's first launch
   // also loads its module, and clocks may still be rising.
@@ -1530,12 +1547,13 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
       if (d != CPM_DISPATCH_HYBRID || (h->cfg[v].hyb_ng > 0 && h->cfg[v].hyb_ng < h->nrep))
         pairs.emplace_back(v, d);
   // A lattice that one thread-block cluster can hold is also tried in the
-  // cluster sweep (every one of its tile heights), unless the caller chose
-  // the parity-split sweep.
+  // cluster sweep (which has no tile variants), unless the caller chose the
+  // parity fill.
   const int row_fill = h->fill == CPM_FILL_CLUSTER ? CPM_FILL_TMA : h->fill;
-  const bool try_cluster = h->cluster_ok && h->fill != CPM_FILL_PARITY;
-  if (try_cluster)
-    for (int v = 0; v < kTileVariants; ++v) pairs.emplace_back(v, -1);
+  const bool fill_auto = h->fill_auto;
+  h->fill_auto = false;
+  if (h->cluster_blocks > 0 && (fill_auto || h->fill != CPM_FILL_PARITY))
+    pairs.emplace_back(h->variant, -1);
   int best_fill = row_fill;
   const int npairs = (int)pairs.size();
   for (int i = 0; i < 3 * npairs && e == cudaSuccess; ++i) {
@@ -1549,7 +1567,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
     e = copy(false);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], h->stream);
     int nl = 0;
-    if (e == cudaSuccess) e = enqueue_sweep(h, v, d, a, any_perim, false, &nl);
+    if (e == cudaSuccess) e = enqueue_sweep(h, v, d, a, false, &nl);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], h->stream);
     if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
     float ms = 0.0f;
@@ -1563,6 +1581,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
     }
   }
   h->fill = best_fill;
+  h->fill_auto = fill_auto && h->cluster_blocks == 0;
   if (e == cudaSuccess) e = copy(false);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(save);
@@ -1616,7 +1635,7 @@ int cpm_run_scores(cpm_handle* h, int mcs, float* d_scores, uint64_t score_base,
     a.tick0 = h->tick;
     a.mcs = chunk;
     int nl = 0;
-    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, any_perimeter(h), true, &nl));
+    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, true, &nl));
     h->launches += nl;
     h->tick += (uint64_t)chunk;
     left -= chunk;
@@ -1888,7 +1907,7 @@ int cpm_set_fill(cpm_handle* h, int fill) {
       fill != CPM_FILL_CLUSTER)
     return h->fail(CPM_ERR_INVALID, "fill %d is not parity (0), vector (1), tma (2) or "
                                     "cluster (3)", fill);
-  if (fill == CPM_FILL_CLUSTER && !h->cluster_ok)
+  if (fill == CPM_FILL_CLUSTER && !h->cluster_fill)
     return h->fail(CPM_ERR_UNSUPPORTED, "no thread-block cluster holds this lattice (one 2D "
                                         "lattice that fits row tiles and ~190 KB of rows per "
                                         "block of a 16- or 8-block cluster)");
@@ -1896,6 +1915,7 @@ int cpm_set_fill(cpm_handle* h, int fill) {
     return h->fail(CPM_ERR_UNSUPPORTED, "row tiles need one lattice with nx a multiple of 4 "
                                         "and nx >= 72; in 2D ny >= 66, in 3D ny, nz >= 18");
   h->fill = fill;
+  h->fill_auto = false;
   return CPM_OK;
 }
 
@@ -2052,7 +2072,8 @@ int cpm_info(const cpm_handle* h, int* n_replicas, int* dimensionality,
   if (!h) return CPM_ERR_INVALID;
   if (n_replicas) *n_replicas = h->nrep;
   if (dimensionality) *dimensionality = h->ndim;
-  if (sweep_grid) *sweep_grid = grid_of(h, h->variant, h->dispatch);
+  if (sweep_grid)
+    *sweep_grid = uses_cluster(h) ? h->cluster_blocks : grid_of(h, h->variant, h->dispatch);
   if (kernel_launches) *kernel_launches = h->launches;
   return CPM_OK;
 }
@@ -2068,10 +2089,10 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x, int* tile_y
   if (warps_per_block) *warps_per_block = p.warps;
   if (grid) *grid = grid_of(h, h->variant, h->dispatch);
   if (dispatch) *dispatch = h->dispatch;
-  if (h->fill == CPM_FILL_CLUSTER) {  // one cluster, its own tile heights
-    if (tile_y) *tile_y = cluster_tile_rows(h->variant);
-    if (tile_z) *tile_z = 1;
-    if (grid) *grid = h->cl_G;
+  if (uses_cluster(h)) {  // one cluster, targets dealt one per lane
+    if (tile_y) *tile_y = 1;
+    if (warps_per_block) *warps_per_block = cluster_sweep_threads() / 32;
+    if (grid) *grid = h->cluster_blocks;
   }
   return CPM_OK;
 }

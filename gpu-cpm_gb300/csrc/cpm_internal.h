@@ -234,15 +234,12 @@ void set_thread_error(const char* message);
 cudaError_t launch_sweep2d(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
                            cudaStream_t s);
 cudaError_t launch_sweep3d(const SweepArgs& a, bool batch, int grid, int warps, cudaStream_t s);
-// Cluster sweep of a small single 2D lattice (cpm_cluster.cu): plan (G
-// blocks of one cluster, H rows per block, dirty-list entries per block)
-// and launch.  The plan is false where no cluster of that shape fits.
-bool row_tiles_fit(int nx, int ny);
-bool cluster_sweep_plan(int nx, int ny, int* G, int* H, long long* list_cap);
-cudaError_t launch_sweep2d_cluster(bool perim, int variant, const SweepArgs& a, int nx, int G,
-                                   int H, cudaStream_t s);
-// Target rows per tile of the cluster sweep's variants.
-int cluster_tile_rows(int variant);
+// Cluster sweep of a small single 2D lattice (cpm_cluster.cu): blocks of the
+// cluster that can hold it with its tables (0: none), and launch.
+int cluster_sweep_blocks(int nx, int ny, int ncells);
+int cluster_sweep_threads();
+cudaError_t launch_cluster_sweep(const SweepArgs& a, int nx, int ny, int ncells, int G,
+                                 cudaStream_t s);
 // checkpoints: host array of ncheck (<= kMaxCheckpoints) MCS counts.
 cudaError_t launch_lr_backward(const float* scores, const float* dl_do,
                                const float* obs, const int* checkpoints, int nrep,

@@ -80,16 +80,6 @@ __host__ __device__ constexpr int queue_len() {
   return 32 + 32 * KR;
 }
 
-// A type's constraint parameters, one 16-byte shared-memory load.
-struct alignas(16) TypeParams {
-  float lam_area;
-  int tgt_area;
-  float lam_perim;
-  int tgt_perim;
-};
-// Words per row of the shared-memory adhesion matrix: entry (a, b) lies in
-// bank 5 a + b, so that up to five types never meet in one.
-constexpr int kJPitch = 37;
 // Dirty-list entries of a phase kept in shared memory (the rest in global
 // memory): a 4096^2 tissue pushes ~1,000 per block and phase.
 constexpr unsigned kListSmem = 2048;

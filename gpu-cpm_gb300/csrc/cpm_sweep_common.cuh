@@ -1,8 +1,7 @@
 // cpm_sweep_common.cuh — device pieces shared by the sweep kernels
-// (cpm_kernels.cu: every dimensionality, batches, scores, act; cpm_sweep2d.cu:
-// 2D single lattices with TMA-staged row-major tiles): lane masks, source
-// coordinates and chemotaxis, the double-buffered cell tables and their
-// delta replay.
+// (cpm_sweep.cuh, cpm_cluster.cu): lane masks, source coordinates and
+// chemotaxis, the deltas of the double-buffered cell tables, the constraint
+// and Metropolis arithmetic.
 #pragma once
 
 #include <cstdint>
@@ -102,8 +101,6 @@ struct PhaseTables {
   long long* wcs;
   unsigned long long* dap;        // this phase's deltas (replayed next phase)
   long long* dcs;
-  uint32_t* list;                 // this block's dirty list for the phase
-  unsigned* cnt;                  // its length (shared memory)
 };
 
 // One accepted copy's change of one table row: added to the other table
@@ -125,55 +122,71 @@ __device__ __forceinline__ void add_delta(const PhaseTables<NDIM>& pt,
   }
 }
 
-// Replays the deltas of the rows on a block's dirty list into `ap`/`cs`,
-// strided over the block's threads.  A row can be on several lists (or
-// twice on one); taking its delta with an exchange hands it to exactly one
-// of them and leaves the delta table zeroed for the phase after next.  All
-// exchanges of a row are issued before any add, so a row costs one round
-// trip to L2.  SMEM_LIST: the list lives in shared memory (cluster sweep).
-// replay_lanes takes entries first, first + stride, ... (one warp's lanes),
-// U of them per round with all their exchanges in flight together (a single
-// replay warp then waits on one round trip per U x 32 entries).
-template <int NDIM, bool SMEM_LIST = false, int U = 1>
-__device__ __forceinline__ void replay_lanes(const uint32_t* list, unsigned n,
-                                             unsigned long long* dap, long long* dcs,
-                                             unsigned long long* ap, long long* cs,
-                                             unsigned first, unsigned stride) {
-  for (unsigned j0 = first; j0 < n; j0 += U * stride) {
-    uint32_t row[U];
-    unsigned long long d[U], dc[U][NDIM];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const unsigned j = j0 + (unsigned)u * stride;
-      row[u] = 0u;
-      d[u] = 0ull;
-#pragma unroll
-      for (int k = 0; k < NDIM; ++k) dc[u][k] = 0ull;
-      if (j < n) {
-        row[u] = SMEM_LIST ? list[j] : __ldcg(list + j);
-        d[u] = atomicExch(dap + row[u], 0ull);
-#pragma unroll
-        for (int k = 0; k < NDIM; ++k)
-          dc[u][k] = atomicExch(
-              reinterpret_cast<unsigned long long*>(dcs + (long long)row[u] * NDIM + k), 0ull);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (d[u]) atomicAdd(ap + row[u], d[u]);
-#pragma unroll
-      for (int k = 0; k < NDIM; ++k)
-        if (dc[u][k])
-          atomicAdd(reinterpret_cast<unsigned long long*>(cs + (long long)row[u] * NDIM + k),
-                    dc[u][k]);
-    }
+// A type's constraint parameters, one 16-byte shared-memory load.
+struct alignas(16) TypeParams {
+  float lam_area;
+  int tgt_area;
+  float lam_perim;
+  int tgt_perim;
+};
+// Words per row of the shared-memory adhesion matrix: entry (a, b) lies in
+// bank 5 a + b, so that up to five types never meet in one.
+constexpr int kJPitch = 37;
+
+// The integers that the constraints multiply: dp (2 (P - P*) + dp) for a
+// perimeter that changes by dp, 1 +- 2 (A - A*) for an area that changes by
+// +-1 (`sign`), each rounded once to FP32.  Where the tables and targets are
+// below 2^21 (`small` tells of the targets) all factors are exact in FP32 and
+// so is the rounding of their product; otherwise in 64 bits.
+__device__ __forceinline__ void constraint_terms(int area, int perim, int dp, int sign,
+                                                 const TypeParams& p, bool small, float& qp,
+                                                 float& qa) {
+  if (small && (unsigned)(area | perim) < (1u << 21)) {
+    qp = __fmul_rn((float)dp, (float)(2 * (perim - p.tgt_perim) + dp));
+    qa = (float)(1 + sign * 2 * (area - p.tgt_area));
+  } else {
+    qp = __ll2float_rn((long long)dp * (2LL * ((long long)perim - p.tgt_perim) + dp));
+    qa = __ll2float_rn(1 + sign * 2LL * ((long long)area - p.tgt_area));
   }
 }
-template <int NDIM, bool SMEM_LIST = false>
-__device__ __forceinline__ void replay(const uint32_t* list, unsigned n,
-                                       unsigned long long* dap, long long* dcs,
-                                       unsigned long long* ap, long long* cs) {
-  replay_lanes<NDIM, SMEM_LIST>(list, n, dap, dcs, ap, cs, threadIdx.x, blockDim.x);
+
+// Metropolis test.  `draw`: the attempt's random word; ex receives
+// exp(-dH/T) where 0 <= dH and T > 0.
+__device__ __forceinline__ bool metropolis(float dH, float T, uint32_t draw, float& ex) {
+  if (dH < 0.0f) return true;
+  if (!(T > 0.0f)) return false;
+  ex = exp_neg(__fdiv_rn(-dH, T));
+  return __fmul_rn(__uint2float_rn((draw >> 8) | 1u), 0x1p-24f) < ex;
+}
+
+// Paired evaluation: an attempt on two neighbouring lanes, the even one
+// (side 0) with the source cell's values, the odd one (side 1) with the
+// target cell's.  Each sums its own configuration's adhesion e (side 0 the
+// new one's, side 1 the old one's) and its own constraint integers; the
+// energy is put together on both in the order of the one-lane form:
+// adhesion, chemotaxis (and what else `extra` holds), perimeter of source
+// and target, area of source and target.  Where a phase is the chain of one
+// warp through its attempts this halves what a lane does one after the
+// other.  `mask`: the lanes that call, pairs complete.
+__device__ __forceinline__ float pair_energy(unsigned mask, int side, bool has_s, bool has_t,
+                                             float e, float extra, float qp, float qa,
+                                             const TypeParams& p, bool perim_on) {
+  const float e2 = __shfl_xor_sync(mask, e, 1);
+  const float qp2 = __shfl_xor_sync(mask, qp, 1), qa2 = __shfl_xor_sync(mask, qa, 1);
+  const float lp2 = __shfl_xor_sync(mask, p.lam_perim, 1);
+  const float la2 = __shfl_xor_sync(mask, p.lam_area, 1);
+  float dH = __fsub_rn(side ? e2 : e, side ? e : e2);
+  dH = __fadd_rn(extra, dH);
+  if (perim_on) {
+    const float ds = __fmaf_rn(side ? lp2 : p.lam_perim, side ? qp2 : qp, dH);
+    dH = has_s ? ds : dH;
+    const float dt = __fmaf_rn(side ? p.lam_perim : lp2, side ? qp : qp2, dH);
+    dH = has_t ? dt : dH;
+  }
+  const float ds = __fmaf_rn(side ? la2 : p.lam_area, side ? qa2 : qa, dH);
+  dH = has_s ? ds : dH;
+  const float dt = __fmaf_rn(side ? p.lam_area : la2, side ? qa : qa2, dH);
+  return has_t ? dt : dH;
 }
 
 }  // namespace

@@ -331,15 +331,21 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
  *                    tiles in shared memory, are still accepted and select
  *                    the same kernel
  *   CPM_FILL_CLUSTER (small 2D lattices) one thread-block cluster of 16 (or 8)
- *                    blocks holds the lattice in its shared memory, one
- *                    strip of rows per block with copies of its neighbours'
- *                    edge rows, for a whole run; tiles are read in place
- *                    and the phases end at a barrier inside the cluster.
- *                    cpm_autotune tries it wherever it fits and keeps it
- *                    when it is faster.
+ *                    blocks holds the lattice and its tables in its shared
+ *                    memory for a whole run, one strip of rows per block with
+ *                    copies of its neighbours' edge rows, and the phases end
+ *                    at a barrier inside the cluster.  Where lattice and
+ *                    tables do not fit (about 400^2), runs take the other
+ *                    sweep.
+ * Until a fill is set (or cpm_autotune picks one) plain runs of a 2D lattice
+ * of up to 140,000 sites take the cluster sweep where it fits, all others the
+ * sweep over the whole GPU; cpm_get_fill then reports CPM_FILL_TMA or
+ * CPM_FILL_PARITY, by the shape alone.  cpm_autotune also tries the cluster
+ * sweep.
  * CPM_FILL_VECTOR and CPM_FILL_TMA need a single lattice with nx a multiple of
- * 4 and nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18); such lattices
- * start in CPM_FILL_TMA, all others in CPM_FILL_PARITY.
+ * 4 and nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18), for which
+ * CPM_FILL_TMA is reported; CPM_FILL_CLUSTER a 2D one of these with about
+ * 190 KB of rows per block of a 16-block cluster at most.
  * The result does not depend on the fill: it selects the kernel only
  * (CPM_ERR_UNSUPPORTED for a fill the lattice cannot use). */
 #define CPM_FILL_PARITY 0

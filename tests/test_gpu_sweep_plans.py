@@ -9,6 +9,7 @@ import pytest
 import oracle
 from gpucpm import workloads as W
 from test_gpu_parity import assert_same, finish, make_engine
+from test_gpu_rowtiles import _terms
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +56,35 @@ def test_targets_beyond_fp32_integers(engine_lib, shape, target):
     w.lam_perim = w.lam_perim * np.float32(1e-7)
     w.tgt_area[1], w.tgt_perim[2] = target, target
     _check(w, 6)
+
+
+@pytest.mark.parametrize("shape,ncells,terms", [
+    ((3, 5), 2, False),        # more blocks than rows
+    ((61, 53), 30, True), ((17, 4), 3, False), ((4, 600), 40, True),
+    ((31, 32), 12, False), ((33, 67), 20, True),
+    ((256, 256), 640, False),  # two targets per lane, all blocks full
+    ((375, 371), 900, True),   # rounds of draws beyond the first
+    ((600, 100), 2000, False),
+])
+@pytest.mark.parametrize("runs", [(40,), (1, 1, 25, 13)])
+def test_small_lattices_run_in_a_cluster(engine_lib, shape, ncells, terms, runs):
+    """Lattices small enough to start in the cluster sweep, and the same ones
+    in the grid sweep: lattice, tables and counters of the oracle, over one
+    launch and over several (tables go out and come in again), and under a
+    graph."""
+    import gpucpm
+    w = W.random_small(shape, ncells, ntypes=3, seed=70 + ncells, temperature=11.0)
+    if terms:
+        _terms(w, ncells)
+    sim = oracle.OracleSim(w.lattice, w.ncells, **w.oracle_kwargs(), seed=6).run(sum(runs))
+    for fill in (None, gpucpm.FILL_PARITY):
+        e = make_engine(w, seed=6)
+        if fill is not None:
+            e.set_fill(fill)
+        else:
+            # (3 columns are below the cluster sweep's least width)
+            assert (e.sweep_config()["grid"] <= 16) or shape[1] < 4
+        for i, mcs in enumerate(runs):
+            (e.run_graph if i % 2 else e.run_mcs)(mcs)
+        finish(e)
+        assert_same(e, sim)
