@@ -820,6 +820,11 @@ int upload_params(cpm_handle* h) {
   return CPM_OK;
 }
 
+// Whether a sweep looks at every table row instead of keeping dirty lists:
+// with up to a row per eight sites the coalesced scan costs less than the
+// lists.
+bool scans(const cpm_handle* h) { return 8 * h->rows <= h->total_sites; }
+
 // Kernel arguments of a sweep with tile variant v and dispatch d (tick0 /
 // mcs, and what depends on the launch, filled in by the caller).
 SweepArgs sweep_args(const cpm_handle* h, int v) {
@@ -834,6 +839,8 @@ SweepArgs sweep_args(const cpm_handle* h, int v) {
   }
   const cpm_handle::Config& c = h->cfg[v];
   a.dlist = h->d_dlist;
+  a.scan = scans(h) ? 1 : 0;
+  a.scan_rows = (unsigned)h->rows;
   a.field = h->d_field;
   a.act_on = h->act_active ? 1 : 0;
   if (h->act_active) {

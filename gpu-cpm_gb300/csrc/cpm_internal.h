@@ -172,6 +172,8 @@ struct SweepArgs {
   const int* task_prefix;  // (batches) [27][nrep + 1] warp tasks per slot, prefix
   int rows, kr;            // target rows of a task, rows drawn side by side
   long long list_cap;      // entries of one dirty list of one block
+  int scan;                // 1: no dirty lists, every table row is replayed
+  unsigned scan_rows;      // (batches) rows of the tables
   // Dispatch: 0 = the tiles of every slot over all replicas go to all warps
   // of the grid, one grid barrier per phase; 1 = each block claims whole
   // replicas in rep_order and runs all their phases with block barriers.

@@ -63,8 +63,9 @@ constexpr int kExt = 1;    // act, 3D persistence
 constexpr int kScore = 2;  // likelihood-ratio scores (2D)
 
 // Warps per block (one block per SM): 24 at 80 registers for the plain 2D
-// sweep, 20 at 96 for the others, which would spill at 80.
-template <int NDIM, int MODE, bool BATCH>
+// sweep, 20 at 96 for the others, which would spill at 80.  (28 or 32 warps at
+// 72 or 64 registers: 4096^2 tissue 7.96 -> 8.13 or 8.54 ms.)
+template <int NDIM, int KR, int MODE, bool BATCH>
 __host__ __device__ constexpr int sweep_warps() {
   return NDIM == 2 && MODE == kPlain && !BATCH ? 24 : 20;
 }
@@ -78,6 +79,30 @@ struct alignas(16) Attempt {
 template <int KR>
 __host__ __device__ constexpr int queue_len() {
   return 32 + 32 * KR;
+}
+
+// A changed table row: row, target site, the row's area, perimeter change + 64
+// and (bit 8) whether the cell lost the site.
+struct alignas(16) RowChange {
+  uint32_t row, site, area, change;
+};
+constexpr int kChangeLen = 32 + 64;
+
+// Whether a kernel queues the row changes of accepted copies and makes them 32
+// at a time.  Few lanes of a batch accept (one in eight on the tissues), and
+// the ~250 instructions of a copy's row changes ran for every batch: 4096^2
+// tissue, 50 MCS 7.65 -> 7.07 ms.  In the kernels of small lattices a phase is
+// one warp's chain, which a second queue lengthens; it gained nothing in 3D
+// (3.61 ms either way) and lost where many accept (256 ragged replicas 22.9 ->
+// 23.7 ms, scores 31.6 -> 32.4).
+template <int NDIM, int KR, int MODE, bool BATCH>
+__host__ __device__ constexpr bool defers() {
+  return NDIM == 2 && KR == 4 && MODE == kPlain && !BATCH;
+}
+template <int NDIM, int KR, int MODE, bool BATCH>
+__host__ __device__ constexpr int warp_smem() {
+  return (int)sizeof(Attempt) * (32 + queue_len<KR>()) +
+         (defers<NDIM, KR, MODE, BATCH>() ? (int)sizeof(RowChange) * kChangeLen : 0);
 }
 
 // Dirty-list entries of a phase kept in shared memory (the rest in global
@@ -159,18 +184,19 @@ __device__ __forceinline__ void flush_scores(const SweepArgs& a, float* sc, int 
 }
 
 template <int NDIM, int KR, int MODE, bool BATCH>
-__global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
+__global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1)
     sweep_kernel(const __grid_constant__ SweepArgs a) {
   constexpr bool EXT = MODE == kExt, SCORE = MODE == kScore;
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
+  constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
   constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
   // the pooled attempts (32 per warp), then the warps' queues
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_list[2][kListSmem];
   __shared__ float s_J[BATCH ? 1 : kMaxTypes * kJPitch];
   __shared__ TypeParams s_type[BATCH ? 1 : kMaxTypes];
-  __shared__ ReplicaCtx s_ctx[BATCH ? sweep_warps<NDIM, MODE, BATCH>() : 1];
+  __shared__ ReplicaCtx s_ctx[BATCH ? sweep_warps<NDIM, KR, MODE, BATCH>() : 1];
   __shared__ int s_ok, s_claim;
   __shared__ unsigned s_cnt[2], s_next[2], s_pool, s_pend[2];
   __shared__ unsigned long long s_tick0;
@@ -179,6 +205,9 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
   const int wpb = blockDim.x >> 5;
   Attempt* const pool = reinterpret_cast<Attempt*>(smem_raw);
   Attempt* const queue = pool + wpb * 32 + warp * QLEN;
+  RowChange* const changes = reinterpret_cast<RowChange*>(pool + wpb * (32 + QLEN)) +
+                             warp * kChangeLen;  // (DEFER)
+  int nchange = 0;  // queued row changes
   const uint32_t k0 = (uint32_t)a.seed, k1 = (uint32_t)(a.seed >> 32);
   int* err = reinterpret_cast<int*>(&a.ctl[kCtlErr]);
   // A phase's dirty list: the first kListSmem entries in shared memory, the
@@ -229,26 +258,63 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
     n_eval = n_acc = 0;
   };
 
-  // Deltas of the phase with double-buffer index `prv` into the copy it read:
-  // rows of this block's dirty list (each delta is taken with an exchange, so
-  // a row listed twice is replayed once) and, in act runs, its copies.
+  // Deltas of the phase with double-buffer index `prv` into the copy it read
+  // and, in act runs, its copies.  Where the tables have few rows for the
+  // lattice's sites (a.scan) every row is looked at, one thread each, with
+  // coalesced loads; elsewhere the rows of this block's dirty list, each
+  // delta taken with an exchange, so that a row listed twice is replayed once.
+  // The list costs a shared-memory atomic and stores per batch and three
+  // exchanges per entry, and the busiest cells are on it many times (list /
+  // scan: 256 ragged replicas, 20 MCS 23.1 / 17.4 ms; gradient of 128 x 256^2
+  // 31.5 / 24.8 ms; act on 512^2 2.03 / 1.90 ms; 4096^2 tissue 7.08 / 7.06 ms).
   auto replay_phase = [&](int prv, unsigned first) {
-    const unsigned n = min(s_cnt[prv], (unsigned)a.list_cap);  // see kErrListFull
     unsigned long long* const dap = prv ? a.dap[1] : a.dap[0];
     unsigned long long* const ap = prv ? a.ap[1] : a.ap[0];
     unsigned long long* const dcs =
         reinterpret_cast<unsigned long long*>(prv ? a.dcs[1] : a.dcs[0]);
     unsigned long long* const cs = reinterpret_cast<unsigned long long*>(prv ? a.cs[1] : a.cs[0]);
-    for (unsigned j = first; j < n; j += blockDim.x) {
-      const long long row = j < kListSmem ? s_list[prv][j] : __ldcg(blist(prv) + j);
-      unsigned long long d[NDIM + 1];  // all exchanges issued before any add
-      d[NDIM] = atomicExch(dap + row, 0ull);
+    if (a.scan) {
+      // every row of the launch, each by one thread of the grid (of the block
+      // in replica dispatch)
+      const unsigned n = BATCH ? a.scan_rows : (unsigned)ctx.ncells + 1u;
+      const unsigned row0 = BATCH ? 0u : ctx.cell_off;
+      const bool local = !BATCH && a.block_local;
+      const unsigned stride = local ? blockDim.x : blockDim.x * gridDim.x;
+      for (unsigned j = first + (local ? 0u : blockIdx.x * blockDim.x); j < n; j += stride) {
+        const long long row = row0 + j;
+        unsigned long long d[NDIM + 1];
+        d[NDIM] = __ldcg(dap + row);
+        if constexpr (NDIM == 2) {
+          const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(dcs) + row);
+          d[0] = v.x, d[1] = v.y;
+        } else {
 #pragma unroll
-      for (int k = 0; k < NDIM; ++k) d[k] = atomicExch(dcs + row * NDIM + k, 0ull);
-      if (d[NDIM]) atomicAdd(ap + row, d[NDIM]);
+          for (int k = 0; k < NDIM; ++k) d[k] = __ldcg(dcs + row * NDIM + k);
+        }
+        if (d[NDIM]) {
+          __stcg(dap + row, 0ull);
+          atomicAdd(ap + row, d[NDIM]);
+        }
 #pragma unroll
-      for (int k = 0; k < NDIM; ++k)
-        if (d[k]) atomicAdd(cs + row * NDIM + k, d[k]);
+        for (int k = 0; k < NDIM; ++k)
+          if (d[k]) {
+            __stcg(dcs + row * NDIM + k, 0ull);
+            atomicAdd(cs + row * NDIM + k, d[k]);
+          }
+      }
+    } else {
+      const unsigned n = min(s_cnt[prv], (unsigned)a.list_cap);  // see kErrListFull
+      for (unsigned j = first; j < n; j += blockDim.x) {
+        const long long row = j < kListSmem ? s_list[prv][j] : __ldcg(blist(prv) + j);
+        unsigned long long d[NDIM + 1];  // all exchanges issued before any add
+        d[NDIM] = atomicExch(dap + row, 0ull);
+#pragma unroll
+        for (int k = 0; k < NDIM; ++k) d[k] = atomicExch(dcs + row * NDIM + k, 0ull);
+        if (d[NDIM]) atomicAdd(ap + row, d[NDIM]);
+#pragma unroll
+        for (int k = 0; k < NDIM; ++k)
+          if (d[k]) atomicAdd(cs + row * NDIM + k, d[k]);
+      }
     }
     if (EXT && a.act_on) {
       // the copies went into the other lattice copy when they were made;
@@ -286,11 +352,39 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
     const uint32_t* const act_r = cur ? a.act2 : a.act;
     uint32_t* const act_w = cur ? a.act : a.act2;
 
+    // Changed rows (0xFFFFFFFF: none) of the lanes onto the block's dirty list:
+    // one shared-memory atomic per batch.
+    auto push_rows = [&](const unsigned push_s, const unsigned push_t) {
+      const unsigned bs = __ballot_sync(kFull, push_s != 0xFFFFFFFFu);
+      const unsigned bt = __ballot_sync(kFull, push_t != 0xFFFFFFFFu);
+      if ((bs | bt) && !a.scan) {  // warp-uniform
+        const unsigned npush = (unsigned)(__popc(bs) + __popc(bt));
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&s_cnt[cur], npush);
+        at = __shfl_sync(kFull, at, 0);
+        // The host sizes the lists for two rows per attempt; a list that
+        // would still overflow is reported, never written past its end.
+        if ((long long)at + npush > a.list_cap) {
+          if (lane == 0) atomicOr(err, kErrListFull);
+        } else {
+          auto put = [&](unsigned i, unsigned row) {
+            if (i < kListSmem)
+              s_list[cur][i] = row;
+            else
+              blist(cur)[i] = row;
+          };
+          if (push_s != 0xFFFFFFFFu) put(at + __popc(bs & lanemask_lt()), push_s);
+          if (push_t != 0xFFFFFFFFu) put(at + __popc(bs) + __popc(bt & lanemask_lt()), push_t);
+        }
+      }
+    };
+
     // ---- evaluate: n <= 32 attempts, one per lane -------------------------------
     auto evaluate = [&](const Attempt* q, const int n) {
       const uint32_t* const L = lat_r + ctx.lat_off;
       bool accepted = false;
       unsigned push_s = 0xFFFFFFFFu, push_t = 0xFFFFFFFFu;  // table rows this lane changed
+      uint32_t at_site = 0, area_s = 0, area_t = 0, change = 0;  // (DEFER)
       if (lane < n) {
         const uint4 e = *reinterpret_cast<const uint4*>(q + lane);
         const uint32_t site = e.x, s = e.z, t = e.w;
@@ -304,10 +398,10 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
           const unsigned rs = ctx.cell_off + is, rt = ctx.cell_off + it;
           // (the medium's row exists; its values are not used)
           const unsigned long long aps = __ldcg(pt.rap + rs), apt = __ldcg(pt.rap + rt);
-          // centroid sums, needed only on acceptance: in 2D fetched with the
-          // row so that an accepted attempt waits on one L2 round trip; in 3D
-          // (three words a side) on acceptance
-          constexpr bool kEarlyCs = NDIM == 2 && KR < 4;
+          // centroid sums, needed only on acceptance: fetched with the row
+          // where many attempts are accepted and registers allow (batches,
+          // scores: 256 ragged replicas 17.4 ms, on acceptance 18.1)
+          constexpr bool kEarlyCs = NDIM == 2 && (BATCH || MODE != kPlain);
           long long cs_s[NDIM], cs_t[NDIM];
           if constexpr (kEarlyCs) {
             const longlong2 vs = __ldcg(reinterpret_cast<const longlong2*>(pt.rcs) + rs);
@@ -327,9 +421,9 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
           const int zl = NDIM == 3 ? (z ? -(int)plane : (nz - 1) * (int)plane) : 0;
           const int zr = NDIM == 3 ? (z + 1 < nz ? (int)plane : -(nz - 1) * (int)plane) : 0;
           uint32_t nb[NBC];
-  #pragma unroll
+#pragma unroll
           for (int p = 0; p < (NDIM == 3 ? 3 : 1); ++p)
-  #pragma unroll
+#pragma unroll
             for (int m = 0; m < 3; ++m) {
               const uint32_t* c = L + site + (NDIM == 3 ? (p == 0 ? zl : p == 1 ? 0 : zr) : 0) +
                                   (m == 0 ? yl : m == 1 ? 0 : yr);
@@ -343,7 +437,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
           int cnt_s = 0, cnt_t = 0;
           unsigned by_new = 0, by_old = 0;  // (scores) neighbours by type, a byte each
           auto adhesion = [&](const float* Jt, const float* Js, auto&& load) {
-  #pragma unroll
+#pragma unroll
             for (int k = 0; k < NBC; ++k) {
               if (k == NB / 2) continue;  // the target itself
               const uint32_t v = nb[k];
@@ -495,7 +589,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
                                                                         (1.0f - 0.25f * xT)))
                                  : 1.0f - ex;  // 1 - exp(-x)
             const float cT = (dH == 0.0f ? -0.5f : (ok ? -1.0f : ex / om)) / T;
-  #pragma unroll
+#pragma unroll
             for (int p = 0; p < kScorePairsMax; ++p) {
               if (p < a.score_spec.n_pairs) {
                 const int pa = a.score_spec.pair_a[p], pb = a.score_spec.pair_b[p];
@@ -534,54 +628,89 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
                 atomicOr(err, kErrListFull);  // reported, never written past the end
               }
             }
-            const int crd[3] = {x, y, z};
-            const int dim[3] = {nx, ny, nz};
-            long long img[NDIM];
-            if (s) {
-  #pragma unroll
-              for (int k = 0; k < NDIM; ++k)
-                img[k] = nearest_image(
-                    crd[k], dim[k], As,
-                    kEarlyCs ? cs_s[k] : __ldcg(pt.rcs + (long long)rs * NDIM + k));
-              add_delta<NDIM>(pt, rs, 1, dps, img, 1);
-              push_s = rs;
-            }
-            if (t) {
-  #pragma unroll
-              for (int k = 0; k < NDIM; ++k)
-                img[k] = nearest_image(
-                    crd[k], dim[k], At,
-                    kEarlyCs ? cs_t[k] : __ldcg(pt.rcs + (long long)rt * NDIM + k));
-              add_delta<NDIM>(pt, rt, -1, dpt, img, -1);
-              push_t = rt;
+            if constexpr (DEFER) {
+              if (s) push_s = rs;
+              if (t) push_t = rt;
+              area_s = (uint32_t)As, area_t = (uint32_t)At;
+              at_site = site;
+              change = (uint32_t)(dps + 64) | ((uint32_t)(dpt + 64) << 16);
+            } else {
+              const int crd[3] = {x, y, z};
+              const int dim[3] = {nx, ny, nz};
+              long long img[NDIM];
+              if (s) {
+    #pragma unroll
+                for (int k = 0; k < NDIM; ++k)
+                  img[k] = nearest_image(
+                      crd[k], dim[k], As,
+                      kEarlyCs ? cs_s[k] : __ldcg(pt.rcs + (long long)rs * NDIM + k));
+                add_delta<NDIM>(pt, rs, 1, dps, img, 1);
+                push_s = rs;
+              }
+              if (t) {
+    #pragma unroll
+                for (int k = 0; k < NDIM; ++k)
+                  img[k] = nearest_image(
+                      crd[k], dim[k], At,
+                      kEarlyCs ? cs_t[k] : __ldcg(pt.rcs + (long long)rt * NDIM + k));
+                add_delta<NDIM>(pt, rt, -1, dpt, img, -1);
+                push_t = rt;
+              }
             }
           }
         }
       }
+      if constexpr (DEFER) {
+        const unsigned bs = __ballot_sync(kFull, push_s != 0xFFFFFFFFu);
+        const unsigned bt = __ballot_sync(kFull, push_t != 0xFFFFFFFFu);
+        uint4* const q = reinterpret_cast<uint4*>(changes) + nchange;
+        if (push_s != 0xFFFFFFFFu)
+          q[__popc(bs & lanemask_lt())] = make_uint4(push_s, at_site, area_s, change & 0xFFFFu);
+        if (push_t != 0xFFFFFFFFu)
+          q[__popc(bs) + __popc(bt & lanemask_lt())] =
+              make_uint4(push_t, at_site, area_t, (change >> 16) | 256u);
+        nchange += __popc(bs) + __popc(bt);
+      }
       n_acc += __popc(__ballot_sync(kFull, accepted));
-      // the changed rows onto the block's dirty list: one shared-memory
-      // atomic per batch
-      const unsigned bs = __ballot_sync(kFull, push_s != 0xFFFFFFFFu);
-      const unsigned bt = __ballot_sync(kFull, push_t != 0xFFFFFFFFu);
-      if (bs | bt) {  // warp-uniform
-        const unsigned npush = (unsigned)(__popc(bs) + __popc(bt));
-        unsigned at = 0;
-        if (lane == 0) at = atomicAdd(&s_cnt[cur], npush);
-        at = __shfl_sync(kFull, at, 0);
-        // The host sizes the lists for two rows per attempt; a list that
-        // would still overflow is reported, never written past its end.
-        if ((long long)at + npush > a.list_cap) {
-          if (lane == 0) atomicOr(err, kErrListFull);
+      if constexpr (!DEFER) push_rows(push_s, push_t);
+    };
+
+    // ---- n <= 32 queued row changes, one per lane ------------------------------
+    auto change_rows = [&](const RowChange* q, const int n) {
+      unsigned row = 0xFFFFFFFFu;
+      if (lane < n) {
+        const uint4 e = *reinterpret_cast<const uint4*>(q + lane);
+        row = e.x;
+        const int lost = (int)(e.w >> 8), area = (int)e.z;
+        const unsigned site = e.y;
+        const int nx = ctx.nx, ny = ctx.ny, nz = NDIM == 3 ? ctx.nz : 1;
+        const int z = NDIM == 3 ? (int)fast_div(site, ctx.div_plane) : 0;
+        const unsigned in_plane =
+            NDIM == 3 ? site - (unsigned)z * ((unsigned)nx * (unsigned)ny) : site;
+        const int y = (int)fast_div(in_plane, ctx.div_nx), x = (int)(in_plane - (unsigned)y * nx);
+        const int crd[3] = {x, y, z};
+        const int dim[3] = {nx, ny, nz};
+        long long cs[NDIM], img[NDIM];
+        if constexpr (NDIM == 2) {
+          const longlong2 v = __ldcg(reinterpret_cast<const longlong2*>(pt.rcs) + row);
+          cs[0] = v.x, cs[1] = v.y;
         } else {
-          auto put = [&](unsigned i, unsigned row) {
-            if (i < kListSmem)
-              s_list[cur][i] = row;
-            else
-              blist(cur)[i] = row;
-          };
-          if (push_s != 0xFFFFFFFFu) put(at + __popc(bs & lanemask_lt()), push_s);
-          if (push_t != 0xFFFFFFFFu) put(at + __popc(bs) + __popc(bt & lanemask_lt()), push_t);
+#pragma unroll
+          for (int k = 0; k < NDIM; ++k) cs[k] = __ldcg(pt.rcs + (long long)row * NDIM + k);
         }
+#pragma unroll
+        for (int k = 0; k < NDIM; ++k) img[k] = nearest_image(crd[k], dim[k], area, cs[k]);
+        add_delta<NDIM>(pt, row, lost ? -1 : 1, (int)(e.w & 0xFFu) - 64, img, lost ? -1 : 1);
+      }
+      push_rows(row, 0xFFFFFFFFu);
+    };
+
+    auto flush_changes = [&](const int least) {  // while at least that many are queued
+      while (nchange >= least) {
+        const int n = min(32, nchange);
+        nchange -= n;
+        change_rows(changes + nchange, n);
+        __syncwarp();
       }
     };
 
@@ -679,6 +808,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
                 nq = 0;
                 break;
               }
+              if constexpr (DEFER) flush_changes(1);
               if (SCORE && r >= 0) flush_scores(a, sc, r, tick);
               flush_counters();
               __syncwarp();
@@ -759,7 +889,9 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
       }
       evaluate(batch, nbatch);
       __syncwarp();  // the queue is rewritten next
+      if constexpr (DEFER) flush_changes(32);
     }
+    if constexpr (DEFER) flush_changes(1);
     if (SCORE && BATCH && r >= 0) flush_scores(a, sc, r, tick);
   };
 
@@ -824,14 +956,14 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, MODE, BATCH>()), 1)
 template <int NDIM, int KR, int MODE, bool BATCH>
 struct SweepFn {
   static const void* fn() { return (const void*)sweep_kernel<NDIM, KR, MODE, BATCH>; }
-  static size_t smem(int warps) { return sizeof(Attempt) * (size_t)warps * (32 + queue_len<KR>()); }
+  static size_t smem(int warps) { return (size_t)warps * warp_smem<NDIM, KR, MODE, BATCH>(); }
 };
 
 template <int NDIM, int KR, int MODE, bool BATCH>
 cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_t s) {
   using F = SweepFn<NDIM, KR, MODE, BATCH>;
-  const int w = warps < sweep_warps<NDIM, MODE, BATCH>() ? warps
-                                                         : sweep_warps<NDIM, MODE, BATCH>();
+  const int w = warps < sweep_warps<NDIM, KR, MODE, BATCH>() ? warps
+                                                         : sweep_warps<NDIM, KR, MODE, BATCH>();
   const size_t smem = F::smem(w);
   const cudaError_t e =
       cudaFuncSetAttribute(F::fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -8,6 +8,7 @@ import pytest
 
 import oracle
 from gpucpm import workloads as W
+from test_gpu_batch import _batch, _batch_state
 from test_gpu_parity import assert_same, finish, make_engine
 from test_gpu_rowtiles import _terms
 
@@ -88,3 +89,38 @@ def test_small_lattices_run_in_a_cluster(engine_lib, shape, ncells, terms, runs)
             (e.run_graph if i % 2 else e.run_mcs)(mcs)
         finish(e)
         assert_same(e, sim)
+
+
+@pytest.mark.parametrize("shape,cells,mcs", [
+    ((64, 50), 399, 20), ((64, 50), 440, 20),        # rows on both sides of sites / 8
+    ((16, 14, 18), 480, 12), ((16, 14, 18), 720, 12),
+    ((1301, 1025), 170000, 1),                       # four rows side by side, listed rows
+])
+@pytest.mark.parametrize("terms", [False, True])
+def test_tables_scanned_and_listed(engine_lib, shape, cells, mcs, terms):
+    """Few rows are replayed by a scan of the tables, many from lists of the
+    changed ones: the oracle's results either way, alone and in a batch of
+    two lattices of different sizes."""
+    import gpucpm
+    w = W.random_small(shape, cells, ntypes=3, seed=33, temperature=14.0)
+    if terms:
+        _terms(w, 5)
+    sim = oracle.OracleSim(w.lattice, w.ncells, **w.oracle_kwargs(), seed=12).run(mcs)
+    e = make_engine(w, seed=12)
+    e.set_fill(gpucpm.FILL_PARITY)
+    e.run_mcs(mcs)
+    finish(e)
+    assert_same(e, sim)
+    if terms or w.lattice.size > 100000:
+        return
+    v = W.random_small(tuple(s + 3 for s in shape), cells, ntypes=3, seed=34, temperature=14.0)
+    b = _batch([w, v], seed=12, stream0=0)
+    b.set_dispatch(gpucpm.DISPATCH_GRID)
+    b.run_mcs(mcs)
+    for r, (x, (lat, a, p, c, cnt)) in enumerate(zip([w, v], _batch_state(b, 2))):
+        o = oracle.OracleSim(x.lattice, x.ncells, **x.oracle_kwargs(), seed=12, stream=r).run(mcs)
+        np.testing.assert_array_equal(lat.view(np.uint32), o.lattice)
+        np.testing.assert_array_equal(a, o.area)
+        np.testing.assert_array_equal(p, o.perim)
+        np.testing.assert_array_equal(c, o.csum)
+        assert cnt["accepted"] == int(o.counters[2])
