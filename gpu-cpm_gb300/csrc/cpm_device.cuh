@@ -151,16 +151,20 @@ __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
 // kernel with an error status instead of a hang.  Block-uniform result.
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;
 
-__device__ __forceinline__ bool grid_barrier(
+// Arrival of the block, by one thread behind a __syncthreads: a release
+// reduction (nothing comes back).
+__device__ __forceinline__ void grid_arrive(uint32_t* ctl) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl[kCtlBarrier]) : "memory");
+}
+
+// The wait of every thread of the block: acquire polls of the counter itself
+// until every block of this episode has arrived.
+__device__ __forceinline__ bool grid_wait(
     uint32_t* ctl, unsigned episode, int* s_ok,
     unsigned long long timeout_ns = kBarrierTimeoutNs) {
-  __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
     const unsigned target = gridDim.x * episode;
-    // arrival: a release reduction (nothing comes back), then acquire polls
-    // of the counter itself until every block of this episode has arrived
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl[kCtlBarrier]) : "memory");
     const unsigned long long t0 = global_timer_ns();
     unsigned spins = 0, nap = 32;
     while (ld_acquire_gpu(&ctl[kCtlBarrier]) < target) {
@@ -184,6 +188,14 @@ __device__ __forceinline__ bool grid_barrier(
   }
   __syncthreads();
   return *s_ok != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(
+    uint32_t* ctl, unsigned episode, int* s_ok,
+    unsigned long long timeout_ns = kBarrierTimeoutNs) {
+  __syncthreads();
+  if (threadIdx.x == 0) grid_arrive(ctl);
+  return grid_wait(ctl, episode, s_ok, timeout_ns);
 }
 
 }  // namespace gpucpm

@@ -44,13 +44,15 @@ constexpr int kWarps2d = 24, kWarpsWide = 20;  // sweep_warps (cpm_sweep.cuh)
 
 // Variant 0.  A slot's 32-column rows of targets are spread over every SM.
 // While a block has at most one row per warp, one row per task: the phase is
-// one warp's chain, and rows side by side would lengthen it.  Up to four rows
-// per warp they are drawn side by side, one task per warp.  Beyond that,
-// 4-row tasks (8-row ones where every warp still gets two or more), claimed
-// until the slot is done.  Measured (us, one / two / four rows side by side):
-// 101 x 75 x 61 box, 20 MCS 2823 / 2827 / 2941; 1001 x 777, 20 MCS 975 / 942 /
-// 1018; 4096^2 tissue, 50 MCS 8755 / 7875 / 7606; 256^3 tissue, 20 MCS 4268 /
-// 3782 / 3658 (8-row tasks: 3614).
+// one warp's chain, and rows side by side would lengthen it.  Up to three rows
+// per warp they are drawn side by side, one task per warp, its draws made
+// before the phase starts.  Beyond that, 4-row tasks (8-row ones where every
+// warp still gets two or more), claimed until the slot is done.  Measured (us,
+// 20 MCS, two / three rows side by side): 800^2 518 / 510; 100^3 1143 / 1123;
+// 1100 x 1000 634 / 584; 128^3 1354 / 1256; (three / four) 1024^2 956 / 1003;
+// (one / two / four) 101 x 75 x 61 box, 20 MCS 2823 / 2827 / 2941;
+// 4096^2 tissue, 50 MCS 8755 / 7875 / 7606; 256^3 tissue, 20 MCS 4268 / 3782 /
+// 3658 (8-row tasks: 3614).
 SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int sms, bool wide) {
   const long long ncx = std::max(1, nx >> 1), ncy = std::max(1, ny >> 1),
                   ncz = ndim == 3 ? std::max(1, nz >> 1) : 1;
@@ -59,16 +61,16 @@ SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int 
   const long long upb = (units + sms - 1) / sms;  // rows of a block
   SweepPlan p;
   switch (variant) {
-    case 1: p.kr = 2, p.rows = 8; break;
+    case 1: p.kr = 4, p.rows = 8; break;
     case 2: p.kr = 4, p.rows = 16; break;
     case 3: p.kr = 1, p.rows = 1; break;
     default:
-      p.kr = upb <= W ? 1 : (upb <= 2 * W ? 2 : 4);
+      p.kr = upb <= W ? 1 : (upb <= 3 * W ? 3 : 4);
       p.rows = upb > 16 * W ? 8 : p.kr;
   }
   if (wide) {
     p.kr = 2;
-    p.rows = std::max(p.rows, 2);
+    p.rows = variant == 0 && upb <= 2 * W ? 2 : std::max(p.rows, 2);
   }
   const long long tasks = tnx * ((ncy + p.rows - 1) / p.rows) * ncz;
   p.grid = (int)std::min<long long>(sms, tasks);

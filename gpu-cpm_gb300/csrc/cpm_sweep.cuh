@@ -190,6 +190,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
   constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
+  constexpr bool AHEAD = !BATCH && KR < 4;
   constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
   // the pooled attempts (32 per warp), then the warps' queues
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -328,6 +329,101 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
         const unsigned long long site = (unsigned long long)e.x | ((unsigned long long)e.y << 32);
         lat[site] = e.z;
         act[site] = e.w;
+      }
+    }
+  };
+
+  // ---- the phase at hand: targets, tasks, draws ----------------------------------
+  int cx = 0, cy = 0, cz = 0;    // the slot's parity class
+  unsigned long long phase = 0;
+  const int rows = a.rows;
+  int nx = 0, ny = 0, nz = 1;
+  unsigned r_fixed = 0;  // (batches)
+  int ncx = 0, ncy = 0, tnx = 1, tny = 1, ntasks = 0;
+  int task = 0, j = 0, j1 = -1;  // next target row of the task, its end (-1: no task yet)
+  int x = 0, z = 0;              // the lane's column
+  bool in_x = false;
+  auto enter = [&]() {  // the constants of the replica in ctx
+    r = ctx.rep;
+    nx = ctx.nx;
+    ny = ctx.ny;
+    nz = NDIM == 3 ? ctx.nz : 1;
+    r_fixed = ctx.fixed_mask;
+  };
+  auto task_grid = [&]() {
+    ncx = class_count(nx, cx);
+    ncy = class_count(ny, cy);
+    tnx = (ncx + 31) >> 5;
+    tny = (ncy + rows - 1) / rows;
+  };
+  auto place = [&](const int local) {  // task `local` of the lattice
+    const int rest = local / tnx;
+    const int tx = (local - rest * tnx + rest) % tnx;
+    const int tz = NDIM == 3 ? rest / tny : 0, ty = rest - tz * tny;
+    j = ty * rows;
+    j1 = min(ncy, j + rows);
+    in_x = tx * 32 + lane < ncx;
+    x = in_x ? class_coord(nx, cx, tx * 32 + lane) : 0;
+    z = NDIM == 3 ? class_coord(nz, cz, tz) : 0;
+  };
+  // KR rows of targets from row j on: their sites, their sources' sites and
+  // directions, and the words for acceptance.
+  uint32_t site[KR], source[KR], word[KR];
+  int kd[KR];
+  auto draw_rows = [&](auto&& load_target, auto&& load_source) {
+    const unsigned plane = (unsigned)nx * (unsigned)ny;
+    uint32_t c[KR][4];
+    int ys[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      ys[u] = class_coord(ny, cy, min(j + u, j1 - 1));
+      site[u] = (unsigned)z * plane + (unsigned)ys[u] * (unsigned)nx + (unsigned)x;
+      load_target(u);
+    }
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      c[u][0] = site[u];
+      c[u][1] = (uint32_t)phase;
+      c[u][2] = a.stream0 + (uint32_t)r;
+      c[u][3] = (uint32_t)(phase >> 32);
+      philox4x32_10(c[u][0], c[u][1], c[u][2], c[u][3], k0, k1);
+    }
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      kd[u] = (int)__umulhi(c[u][0], (unsigned)NB);
+      int sx, sy, sz;
+      source_coords<NDIM>(kd[u], x, ys[u], z, nx, ny, nz, sx, sy, sz);
+      source[u] = (NDIM == 3 ? (unsigned)sz * plane : 0u) + (unsigned)sy * (unsigned)nx +
+                  (unsigned)sx;
+      word[u] = c[u][1];
+      load_source(u);
+    }
+  };
+  // The phase of slot `slot` at MCS `tick`; in the kernels of small lattices
+  // (AHEAD) also the draws of this warp's first task, often its only one.
+  // They read no site and no table, so they are made between the block's
+  // arrival at the barrier before the phase and its wait: 101 x 75 x 61 box,
+  // 20 MCS 2.78 -> 2.52 ms; 1001 x 777, 20 MCS 0.98 -> 0.90; 96^3 with
+  // persistence 1.46 -> 1.40; act on 512^2, 50 MCS 1.90 -> 1.82.  With four
+  // rows the held draws spill (4096^2, 50 MCS 7.07 -> 7.80).
+  bool drawn = false;
+  auto begin_phase = [&](const int slot, const unsigned long long tick, const int b, const int G) {
+    cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
+    phase = tick * NSLOTS + (unsigned long long)slot;
+    if (!BATCH || r >= 0) enter();
+    if constexpr (!BATCH) {
+      task_grid();
+      ntasks = tnx * tny * class_count(nz, cz);
+    }
+    task = b + warp * G;
+    j = 0, j1 = -1;
+    x = z = 0;
+    in_x = false;
+    if constexpr (AHEAD) {
+      drawn = task < ntasks;
+      if (drawn) {
+        place(task);
+        draw_rows([](int) {}, [](int) {});
       }
     }
   };
@@ -714,42 +810,16 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       }
     };
 
-    const int cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
-    const unsigned long long phase = tick * NSLOTS + (unsigned long long)slot;
-    const int rows = a.rows;
-    int nx = 0, ny = 0, nz = 1;
-    unsigned fixed_mask = 0;
-    const uint32_t* L = lat_r;
-    auto enter = [&]() {  // the constants of the replica in ctx
-      r = ctx.rep;
-      nx = ctx.nx;
-      ny = ctx.ny;
-      nz = NDIM == 3 ? ctx.nz : 1;
-      fixed_mask = ctx.fixed_mask;
-      L = lat_r + ctx.lat_off;
-    };
-    if (!BATCH || r >= 0) enter();
-    int ncx = 0, ncy = 0, tnx = 1, tny = 1, ntasks;
-    auto task_grid = [&]() {
-      ncx = class_count(nx, cx);
-      ncy = class_count(ny, cy);
-      tnx = (ncx + 31) >> 5;
-      tny = (ncy + rows - 1) / rows;
-    };
+    if constexpr (!AHEAD) begin_phase(slot, tick, b, G);
+    const uint32_t* L = lat_r + (!BATCH || r >= 0 ? ctx.lat_off : 0);
     const int* pre = nullptr;  // (batches) tasks of the slot before each replica
     if constexpr (BATCH) {
       pre = a.task_prefix + slot * (a.nrep + 1);
       ntasks = __ldg(pre + a.nrep);
-    } else {
-      task_grid();
-      ntasks = tnx * tny * class_count(nz, cz);
     }
     unsigned* ctr = &s_next[step & 1];
     if (tid == 0) s_next[(step + 1) & 1] = 0u;
-    int nq = 0, task = b + warp * G;
-    int j = 0, j1 = -1;  // next target row of the task, its end (-1: no task yet)
-    int x = 0, z = 0;    // the lane's column
-    bool in_x = false;
+    int nq = 0;
     int next_rep = -1;       // (batches) the replica of the task at hand
     bool rep_ready = !BATCH;  // its constants are loaded
     int pool_at = -1, pool_n = 0;  // pooled stage: this warp's next batch, all attempts
@@ -815,47 +885,22 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
               if (lane == 0) load_replica(rep);
               __syncwarp();
               enter();
+              L = lat_r + ctx.lat_off;
             }
             task_grid();
             rep_ready = true;
             j1 = 0;
           }
         }
-        if (j1 == 0) {  // the task's place
-          const int local = BATCH ? task - __ldg(pre + next_rep) : task;
-          const int rest = local / tnx;
-          const int tx = (local - rest * tnx + rest) % tnx;
-          const int tz = NDIM == 3 ? rest / tny : 0, ty = rest - tz * tny;
-          j = ty * rows;
-          j1 = min(ncy, j + rows);
-          in_x = tx * 32 + lane < ncx;
-          x = in_x ? class_coord(nx, cx, tx * 32 + lane) : 0;
-          z = NDIM == 3 ? class_coord(nz, cz, tz) : 0;
-        }
-        const unsigned plane = (unsigned)nx * (unsigned)ny;
-        uint32_t c[KR][4], site[KR], tv[KR], sv[KR];
-        int ys[KR], kd[KR];
+        if (j1 == 0) place(BATCH ? task - __ldg(pre + next_rep) : task);
+        uint32_t tv[KR], sv[KR];
+        const unsigned fixed_mask = BATCH ? r_fixed : ctx.fixed_mask;
+        if (AHEAD && drawn) {
+          drawn = false;
 #pragma unroll
-        for (int u = 0; u < KR; ++u) {
-          ys[u] = class_coord(ny, cy, min(j + u, j1 - 1));
-          site[u] = (unsigned)z * plane + (unsigned)ys[u] * (unsigned)nx + (unsigned)x;
-          tv[u] = L[site[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < KR; ++u) {
-          c[u][0] = site[u];
-          c[u][1] = (uint32_t)phase;
-          c[u][2] = a.stream0 + (uint32_t)r;
-          c[u][3] = (uint32_t)(phase >> 32);
-          philox4x32_10(c[u][0], c[u][1], c[u][2], c[u][3], k0, k1);
-        }
-#pragma unroll
-        for (int u = 0; u < KR; ++u) {
-          kd[u] = (int)__umulhi(c[u][0], (unsigned)NB);
-          int sx, sy, sz;
-          source_coords<NDIM>(kd[u], x, ys[u], z, nx, ny, nz, sx, sy, sz);
-          sv[u] = L[(NDIM == 3 ? (unsigned)sz * plane : 0u) + (unsigned)sy * (unsigned)nx +
-                    (unsigned)sx];
+          for (int u = 0; u < KR; ++u) tv[u] = L[site[u]], sv[u] = L[source[u]];
+        } else {
+          draw_rows([&](int u) { tv[u] = L[site[u]]; }, [&](int u) { sv[u] = L[source[u]]; });
         }
 #pragma unroll
         for (int u = 0; u < KR; ++u) {
@@ -874,7 +919,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           const unsigned ball = __ballot_sync(kFull, keep);
           if (keep)
             *reinterpret_cast<uint4*>(queue + nq + __popc(ball & lanemask_lt())) =
-                make_uint4(site[u], (c[u][1] & 0xFFFFFF00u) | (uint32_t)kd[u], s, tv[u]);
+                make_uint4(site[u], (word[u] & 0xFFFFFF00u) | (uint32_t)kd[u], s, tv[u]);
           nq += __popc(ball);
           n_eval += __popc(ball);
         }
@@ -920,6 +965,8 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       __syncthreads();
     }
     int step = 0;
+    if constexpr (AHEAD)
+      if (a.mcs > 0) begin_phase(a.slots[0], s_tick0, b, G);
     for (int m = 0; m < a.mcs; ++m) {
       const unsigned long long tick = s_tick0 + (unsigned long long)m;
       for (int si = 0; si < a.nslot_active; ++si, ++step) {
@@ -931,10 +978,16 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
         if (tid == 0) {
           s_cnt[prv] = s_pend[prv] = 0;
           s_pool = 0;
+          if (!local) grid_arrive(a.ctl);
+        }
+        if constexpr (AHEAD) {
+          const bool wrap = si + 1 == a.nslot_active;
+          if (!wrap || m + 1 < a.mcs)
+            begin_phase(a.slots[wrap ? 0 : si + 1], tick + (wrap ? 1 : 0), b, G);
         }
         if (local)
           __syncthreads();
-        else if (!grid_barrier(a.ctl, ++episode, &s_ok))
+        else if (!grid_wait(a.ctl, ++episode, &s_ok))
           return;
       }
       if (SCORE && !BATCH) flush_scores(a, sc, r, tick);
@@ -972,8 +1025,8 @@ cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_
   return cudaLaunchCooperativeKernel(F::fn(), dim3(grid), dim3(32 * w), args, smem, s);
 }
 
-// One kernel per mode and rows drawn side by side (a.kr; the extended, score
-// and batch kernels have two).
+// One kernel per mode and rows drawn side by side (a.kr: one, three or four;
+// the extended, score and batch kernels have two).
 template <int NDIM>
 cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
                             cudaStream_t s) {
@@ -992,7 +1045,7 @@ cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int gri
   switch (a.kr) {
     case 1: return launch_sweep_as<NDIM, 1, kPlain, false>(a, grid, warps, s);
     case 4: return launch_sweep_as<NDIM, 4, kPlain, false>(a, grid, warps, s);
-    default: return launch_sweep_as<NDIM, 2, kPlain, false>(a, grid, warps, s);
+    default: return launch_sweep_as<NDIM, 3, kPlain, false>(a, grid, warps, s);
   }
 }
 

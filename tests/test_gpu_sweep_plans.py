@@ -1,5 +1,5 @@
 """The sweep at the sizes where its plan changes, against the oracle bit for
-bit: one, two and four rows of targets drawn side by side, several tasks per
+bit: one, three and four rows of targets drawn side by side, several tasks per
 warp, one target per task, lattices one task wide or a few rows high, odd
 sides, every tile variant; and targets so large that a constraint's integers
 no longer fit FP32."""
@@ -35,10 +35,10 @@ def test_narrow_and_odd_shapes(engine_lib, shape, ncells, mcs, variant):
 
 
 @pytest.mark.parametrize("shape,mcs", [
-    ((570, 1024), 3),        # two rows side by side
+    ((570, 1024), 3),        # three rows side by side
     ((1301, 1025), 2),       # four rows, one task per warp, odd sides
     ((4000, 2000), 1),       # 8-row tasks, several per warp
-    ((135, 136, 64), 2),     # 3D, two rows
+    ((135, 136, 64), 2),     # 3D, three rows
     ((200, 201, 63), 1),     # 3D, four rows, odd
     ((312, 314, 128), 1),    # 3D, 8-row tasks
 ])
