@@ -81,7 +81,11 @@ SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int 
 }
 
 // Long tasks fill a warp's batches (attempts of different replicas are not
-// evaluated together); small batches need every warp to get a task.
+// evaluated together: with queues of two replicas' attempts 256 ragged
+// replicas took 3 % longer, their constants no longer being the warp's); small
+// batches need every warp to get a task.  Measured (ms): 128 x 256^2 with
+// scores 8 rows 24.1, 4 rows 28.1, 16 rows 28.0; 256 ragged replicas 16 rows
+// 16.4, 8 rows 19.0; 64 x 64^2 2 rows 0.52, 4 rows 0.59.
 int gpucpm::batch_rows(int variant, long long total_units, int sms) {
   switch (variant) {
     case 1: return 8;
@@ -487,7 +491,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     if (n > 1) {
       // Grid dispatch: tasks dealt one at a time, at most ceil(tasks / grid)
       // per block, each attempt touching at most two table rows.
-      c.plan.kr = 2;
+      c.plan.kr = rows >= 4 ? 4 : 2;
       c.plan.rows = rows;
       c.plan.warps = 20;
       c.plan.grid = (int)std::min<long long>(sms, max_tasks);

@@ -73,7 +73,19 @@ constexpr int kErrListFull = 32;      // a dirty list would overflow (not writte
 
 // Per-replica parameters, kept in global memory (read through the
 // read-only cache; a replica's few hundred used bytes stay L1-resident).
-struct DevParams {
+// The scalars of a parameter record, read as words by one warp.
+struct ParamHead {
+  float temperature;
+  int perim_on;         // any lam_perim != 0
+  unsigned fixed_mask;  // bit t: cells of type t never move (src/kernels2d.cu:280-290)
+  int stick_on;         // any stickiness != 0
+  int chemo_on;         // any chemo != 0
+  int act_on;           // any act_lambda != 0
+  int persist_on;       // any persist_lambda != 0
+  int small_targets;    // all target areas and perimeters within (-2^21, 2^21)
+};
+
+struct DevParams : ParamHead {
   float J[kMaxTypes * kMaxTypes];      // J[own type][neighbour type]
   // stickiness S[own type][neighbour type]: added to the adhesion of the
   // configuration before the copy only (src/kernels2d.cu:399-400)
@@ -82,20 +94,12 @@ struct DevParams {
   int tgt_area[kMaxTypes];
   float lam_perim[kMaxTypes];
   int tgt_perim[kMaxTypes];
-  float temperature;
-  int perim_on;         // any lam_perim != 0
-  unsigned fixed_mask;  // bit t: cells of type t never move (src/kernels2d.cu:280-290)
-  int stick_on;         // any stickiness != 0
   // chemotaxis lambda per type: dH -= lambda (d . field at the source), d the
   // unit copy direction (src/kernels2d.cu:302-334, src/kernels3d.cu:275-324)
   float chemo[kMaxTypes];
-  int chemo_on;         // any chemo != 0
-  // act model (src/kernels2d.cu:312-473): lambda and max_act per type
-  int act_on;           // any act_lambda != 0
+  // act model (src/kernels2d.cu:312-473): lambda and max_act per type;
   // persistence (3D, src/kernels3d.cu:327-343, src/kernels.cu:159-212):
   // lambda and diffusion per type
-  int persist_on;       // any persist_lambda != 0
-  int small_targets;    // all target areas and perimeters within (-2^21, 2^21)
   float act_lambda[kMaxTypes];
   int act_max[kMaxTypes];
   float persist_lambda[kMaxTypes];

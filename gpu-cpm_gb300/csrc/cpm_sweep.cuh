@@ -111,16 +111,9 @@ constexpr unsigned kListSmem = 2048;
 
 // What attempts need of their replica, in shared memory (one for the block,
 // in batches one per warp): kept in registers it made every kernel spill.
-struct ReplicaCtx {
+struct ReplicaCtx : DevReplica, ParamHead {
   const DevParams* P;
-  long long lat_off;
-  int rep, ncells;
-  unsigned cell_off;  // (table rows and a replica's sites < 2^31)
-  int nx, ny, nz;
-  FastDiv div_nx, div_plane;
-  float T;
-  unsigned fixed_mask;
-  int stick_on, chemo_on, perim_on, small_targets, act_on, persist_on;
+  int rep;
 };
 
 __device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& d) {
@@ -229,27 +222,22 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   // ---- the replica at hand ------------------------------------------------
   ReplicaCtx& ctx = s_ctx[BATCH ? warp : 0];
   int r = -1;
-  auto load_replica = [&](int rep) {  // one lane of the warps that share ctx
-    const DevReplica* R = a.reps + rep;
-    const DevParams* P = a.params + __ldg(&R->pset);
-    ctx.P = P;
-    ctx.lat_off = __ldg(&R->lat_off);
-    ctx.rep = rep;
-    ctx.ncells = __ldg(&R->ncells);
-    ctx.cell_off = (unsigned)__ldg(&R->cell_off);
-    ctx.nx = __ldg(&R->nx);
-    ctx.ny = __ldg(&R->ny);
-    ctx.nz = NDIM == 3 ? __ldg(&R->nz) : 1;
-    ctx.div_nx = {__ldg(&R->div_nx.mul), __ldg(&R->div_nx.shift)};
-    ctx.div_plane = {__ldg(&R->div_plane.mul), __ldg(&R->div_plane.shift)};
-    ctx.T = __ldg(&P->temperature);
-    ctx.fixed_mask = __ldg(&P->fixed_mask);
-    ctx.stick_on = __ldg(&P->stick_on);
-    ctx.chemo_on = __ldg(&P->chemo_on);
-    ctx.perim_on = __ldg(&P->perim_on);
-    ctx.small_targets = __ldg(&P->small_targets);
-    ctx.act_on = __ldg(&P->act_on);
-    ctx.persist_on = __ldg(&P->persist_on);
+  // by a whole warp, a word per lane: every task of a batch begins with it,
+  // and one lane's loads of the fields took ~60 instructions and as many
+  // trips as fields (with the search below and four rows side by side: 256
+  // ragged replicas, 20 MCS 17.4 -> 16.4 ms; 128 of 128^2 to 512^2 5.72 -> 5.29)
+  auto load_replica = [&](int rep) {
+    constexpr int kRep = sizeof(DevReplica) / 4, kHead = sizeof(ParamHead) / 4;
+    const uint32_t v =
+        lane < kRep ? __ldg(reinterpret_cast<const uint32_t*>(a.reps + rep) + lane) : 0u;
+    const DevParams* P = a.params + __shfl_sync(kFull, v, offsetof(DevReplica, pset) / 4);
+    const uint32_t h =
+        lane < kHead
+            ? __ldg(reinterpret_cast<const uint32_t*>(static_cast<const ParamHead*>(P)) + lane)
+            : 0u;
+    if (lane < kRep) reinterpret_cast<uint32_t*>(static_cast<DevReplica*>(&ctx))[lane] = v;
+    if (lane < kHead) reinterpret_cast<uint32_t*>(static_cast<ParamHead*>(&ctx))[lane] = h;
+    if (lane == 0) ctx.P = P, ctx.rep = rep;
   };
   auto flush_counters = [&]() {
     if (lane == 0 && r >= 0) {
@@ -278,7 +266,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       // every row of the launch, each by one thread of the grid (of the block
       // in replica dispatch)
       const unsigned n = BATCH ? a.scan_rows : (unsigned)ctx.ncells + 1u;
-      const unsigned row0 = BATCH ? 0u : ctx.cell_off;
+      const unsigned row0 = BATCH ? 0u : (unsigned)ctx.cell_off;
       const bool local = !BATCH && a.block_local;
       const unsigned stride = local ? blockDim.x : blockDim.x * gridDim.x;
       for (unsigned j = first + (local ? 0u : blockIdx.x * blockDim.x); j < n; j += stride) {
@@ -340,6 +328,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   int nx = 0, ny = 0, nz = 1;
   unsigned r_fixed = 0;  // (batches)
   int ncx = 0, ncy = 0, tnx = 1, tny = 1, ntasks = 0;
+  unsigned inv_tnx = 0;
   int task = 0, j = 0, j1 = -1;  // next target row of the task, its end (-1: no task yet)
   int x = 0, z = 0;              // the lane's column
   bool in_x = false;
@@ -355,15 +344,33 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     ncy = class_count(ny, cy);
     tnx = (ncx + 31) >> 5;
     tny = (ncy + rows - 1) / rows;
+    inv_tnx = 0xFFFFFFFFu / (unsigned)tnx;
+  };
+  // n / tnx and the remainder, n < 2^31: with inv = floor((2^32 - 1) / tnx),
+  // n * inv / 2^32 lies in (n / tnx - 1/2, n / tnx], so the product's high word
+  // is the quotient or one less.  (Two divisions per task were part of what
+  // made tasks of 4 rows no better than ones of 8: 4096^2, 50 MCS 7.09 -> 7.05.)
+  auto by_tnx = [&](const unsigned n, unsigned& rem) {
+    unsigned q = __umulhi(n, inv_tnx);
+    rem = n - q * (unsigned)tnx;
+    if (rem >= (unsigned)tnx) {
+      rem -= (unsigned)tnx;
+      ++q;
+    }
+    return q;
   };
   auto place = [&](const int local) {  // task `local` of the lattice
-    const int rest = local / tnx;
-    const int tx = (local - rest * tnx + rest) % tnx;
+    unsigned tx, turn;
+    const int rest = (int)by_tnx((unsigned)local, tx);
+    by_tnx((unsigned)rest, turn);
+    tx += turn;
+    if (tx >= (unsigned)tnx) tx -= (unsigned)tnx;
     const int tz = NDIM == 3 ? rest / tny : 0, ty = rest - tz * tny;
     j = ty * rows;
     j1 = min(ncy, j + rows);
-    in_x = tx * 32 + lane < ncx;
-    x = in_x ? class_coord(nx, cx, tx * 32 + lane) : 0;
+    const int i = (int)tx * 32 + lane;
+    in_x = i < ncx;
+    x = in_x ? class_coord(nx, cx, i) : 0;
     z = NDIM == 3 ? class_coord(nz, cz, tz) : 0;
   };
   // KR rows of targets from row j on: their sites, their sources' sites and
@@ -491,7 +498,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           const int kdir = (int)(e.y & 0xFFu);
           const int ts = (int)(s >> 24) & (kMaxTypes - 1);
           const int tt = (int)(t >> 24) & (kMaxTypes - 1);
-          const unsigned rs = ctx.cell_off + is, rt = ctx.cell_off + it;
+          const unsigned rs = (unsigned)ctx.cell_off + is, rt = (unsigned)ctx.cell_off + it;
           // (the medium's row exists; its values are not used)
           const unsigned long long aps = __ldcg(pt.rap + rs), apt = __ldcg(pt.rap + rt);
           // centroid sums, needed only on acceptance: fetched with the row
@@ -661,7 +668,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           }
           dH = s ? __fmaf_rn(ps.lam_area, qas, dH) : dH;
           dH = t ? __fmaf_rn(pr.lam_area, qat, dH) : dH;
-          const float T = ctx.T;
+          const float T = ctx.temperature;
           bool ok;
           float ex = 1.0f;  // exp(-dH/T) when 0 <= dH and T > 0
           if (dH < 0.0f) {
@@ -820,6 +827,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     unsigned* ctr = &s_next[step & 1];
     if (tid == 0) s_next[(step + 1) & 1] = 0u;
     int nq = 0;
+    int first = 0;           // (batches) its replica's first task
     int next_rep = -1;       // (batches) the replica of the task at hand
     bool rep_ready = !BATCH;  // its constants are loaded
     int pool_at = -1, pool_n = 0;  // pooled stage: this warp's next batch, all attempts
@@ -859,10 +867,15 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
             break;
           }
           if constexpr (BATCH) {
-            int lo = 0, hi = a.nrep - 1;  // the largest with pre[lo] <= task
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (__ldg(pre + mid) <= task) lo = mid; else hi = mid - 1;
+            // the largest with pre[lo] <= task, 32 probes at a time
+            int lo = 0, n = a.nrep;
+            while (n > 1) {
+              const int st = (n + 31) >> 5, k = lane * st;
+              const int v = k < n ? __ldg(pre + lo + k) : 0;
+              const int at = __popc(__ballot_sync(kFull, k < n && v <= task)) - 1;
+              first = __shfl_sync(kFull, v, at);
+              lo += at * st;
+              n = min(st, n - at * st);
             }
             next_rep = lo;
             rep_ready = false;
@@ -882,7 +895,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
               if (SCORE && r >= 0) flush_scores(a, sc, r, tick);
               flush_counters();
               __syncwarp();
-              if (lane == 0) load_replica(rep);
+              load_replica(rep);
               __syncwarp();
               enter();
               L = lat_r + ctx.lat_off;
@@ -892,7 +905,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
             j1 = 0;
           }
         }
-        if (j1 == 0) place(BATCH ? task - __ldg(pre + next_rep) : task);
+        if (j1 == 0) place(task - first);
         uint32_t tv[KR], sv[KR];
         const unsigned fixed_mask = BATCH ? r_fixed : ctx.fixed_mask;
         if (AHEAD && drawn) {
@@ -949,9 +962,11 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   if (local && !grid_barrier(a.ctl, ++episode, &s_ok)) return;
   for (;;) {
     if constexpr (!BATCH) {
-      if (tid == 0) {
-        const int qi = local ? (int)atomicAdd(&a.ctl[kCtlQueue], 1u) : 0;
-        s_claim = qi;
+      if (warp == 0) {
+        int qi = 0;
+        if (local && lane == 0) qi = (int)atomicAdd(&a.ctl[kCtlQueue], 1u);
+        qi = __shfl_sync(kFull, qi, 0);
+        if (lane == 0) s_claim = qi;
         if (!local || qi < a.queue_len) load_replica(local ? __ldg(a.rep_order + qi) : 0);
       }
       __syncthreads();
@@ -1025,8 +1040,10 @@ cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_
   return cudaLaunchCooperativeKernel(F::fn(), dim3(grid), dim3(32 * w), args, smem, s);
 }
 
-// One kernel per mode and rows drawn side by side (a.kr: one, three or four;
-// the extended, score and batch kernels have two).
+// One kernel per mode and rows drawn side by side (a.kr): one, three or four;
+// in batches two, and four where tasks have as many rows (more loads in
+// flight: 256 ragged replicas, 20 MCS 17.4 / 16.8 ms, gradient of 128 x 256^2
+// 24.8 / 24.3); two in the extended and single-lattice score kernels.
 template <int NDIM>
 cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
                             cudaStream_t s) {
@@ -1034,9 +1051,12 @@ cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int gri
   if (batch) {
     if (ext) return launch_sweep_as<NDIM, 2, kExt, true>(a, grid, warps, s);
     if constexpr (NDIM == 2) {
-      if (scores) return launch_sweep_as<NDIM, 2, kScore, true>(a, grid, warps, s);
+      if (scores)
+        return a.kr == 4 ? launch_sweep_as<NDIM, 4, kScore, true>(a, grid, warps, s)
+                         : launch_sweep_as<NDIM, 2, kScore, true>(a, grid, warps, s);
     }
-    return launch_sweep_as<NDIM, 2, kPlain, true>(a, grid, warps, s);
+    return a.kr == 4 ? launch_sweep_as<NDIM, 4, kPlain, true>(a, grid, warps, s)
+                     : launch_sweep_as<NDIM, 2, kPlain, true>(a, grid, warps, s);
   }
   if (ext) return launch_sweep_as<NDIM, 2, kExt, false>(a, grid, warps, s);
   if constexpr (NDIM == 2) {

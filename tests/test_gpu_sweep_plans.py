@@ -124,3 +124,51 @@ def test_tables_scanned_and_listed(engine_lib, shape, cells, mcs, terms):
         np.testing.assert_array_equal(p, o.perim)
         np.testing.assert_array_equal(c, o.csum)
         assert cnt["accepted"] == int(o.counters[2])
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+def test_batches_of_many_replicas(engine_lib, ndim, variant):
+    """More replicas than a warp searches at once, of sides from a few columns
+    to several tasks, in tasks of 2 to 32 rows: each as the oracle has it."""
+    import gpucpm
+    g = np.random.default_rng(8)
+    n = 70 if ndim == 2 else 35
+    lo, hi = ((5, 90) if ndim == 2 else (4, 14))
+    ws = [W.random_small(tuple(int(k) for k in g.integers(lo, hi, ndim)), 4 + i % 9,
+                         seed=200 + i, temperature=5.0 + i % 7) for i in range(n)]
+    b = _batch(ws, seed=3, stream0=11)
+    b.set_variant(variant)
+    b.set_dispatch(gpucpm.DISPATCH_GRID)
+    b.run_mcs(4)
+    for r, (x, (lat, a, p, c, cnt)) in enumerate(zip(ws, _batch_state(b, n))):
+        o = oracle.OracleSim(x.lattice, x.ncells, **x.oracle_kwargs(), seed=3,
+                             stream=11 + r).run(4)
+        np.testing.assert_array_equal(lat.view(np.uint32), o.lattice)
+        np.testing.assert_array_equal(a, o.area)
+        np.testing.assert_array_equal(p, o.perim)
+        np.testing.assert_array_equal(c, o.csum)
+        assert cnt["accepted"] == int(o.counters[2])
+
+
+def test_scores_of_long_and_short_tasks(engine_lib):
+    """Scores over tasks of 8 rows (four side by side) and of 2 (two): the same
+    lattices, and sums that differ by their order only (FP32)."""
+    import torch
+
+    import gpucpm
+    ws = [W.sorting_2d(n=40 + 8 * i, ncells=20 + 5 * i, seed=60 + i) for i in range(4)]
+    spec = gpucpm.ScoreSpec.make(((1, 1), (2, 2), (1, 2)), lambda_perim=True)
+    res = []
+    for variant in (1, 3):
+        b = _batch(ws, seed=4, stream0=0)
+        b.set_variant(variant)
+        b.set_dispatch(gpucpm.DISPATCH_GRID)
+        sc = torch.zeros((len(ws), 6, gpucpm.SCORE_MAX), device="cuda")
+        torch.cuda.synchronize()
+        b.run_scores(6, sc.data_ptr(), 0, 6, spec)
+        res.append((_batch_state(b, len(ws)), sc.cpu().numpy()))
+    for r in range(len(ws)):
+        np.testing.assert_array_equal(res[0][0][r][0], res[1][0][r][0])
+    scale = np.abs(res[0][1]).max(axis=(0, 1)) + 1e-6
+    assert (np.abs(res[0][1] - res[1][1]) / scale).max() < 1e-4
