@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -1701,25 +1702,13 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   const DevReplica& R = h->reps[r];
   const int nd = h->ndim;
   const int n[3] = {R.nx, R.ny, R.nz};
-  for (int k = 0; k < npoints; ++k) {
-    for (int a = 0; a < nd; ++a) {
-      const double p = points[(size_t)k * nd + a];
-      if (!(p >= 0.0 && p < (double)n[a]))
-        return h->fail(CPM_ERR_INVALID, "cpm_seed_voronoi_r: point %d lies outside [0, n)", k);
-    }
-    const uint32_t v = values[k], id = v & 0xFFFFFFu, ty = v >> 24;
-    if ((int)id > R.ncells || ty >= (uint32_t)kMaxTypes || (id == 0 && ty != 0))
-      return h->fail(CPM_ERR_INVALID,
-                     "cpm_seed_voronoi_r: value %d is not id <= ncells | type < 32 << 24 "
-                     "(id 0 with type 0)", k);
-  }
   // Bucket grid with about two points per bucket.
   VoronoiGrid vg;
   vg.ndim = nd;
   const double sites = (double)n[0] * n[1] * n[2];
   const double side = std::pow(2.0 * sites / npoints, 1.0 / nd);
   long long G = 1;
-  double wmin = 1e300, wmax = 0.0, w[3];
+  double wmin = 1e300, wmax = 0.0, inv_w[3];
   vg.rmax = 0;
   int nmax = 1;
   for (int a = 0; a < 3; ++a) {
@@ -1727,12 +1716,13 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
     int g = a < nd ? (int)std::lround((double)n[a] / side) : 1;
     g = std::max(1, std::min(g, n[a]));
     vg.g[a] = g;
-    w[a] = (double)n[a] / g;
-    vg.wf[a] = (float)w[a];
-    vg.inv_w[a] = (float)(1.0 / w[a]);
+    const double w = (double)n[a] / g;
+    inv_w[a] = (double)g / n[a];
+    vg.wf[a] = (float)w;
+    vg.inv_w[a] = (float)(1.0 / w);
     if (a < nd) {
-      wmin = std::min(wmin, w[a]);
-      wmax = std::max(wmax, w[a]);
+      wmin = std::min(wmin, w);
+      wmax = std::max(wmax, w);
       nmax = std::max(nmax, n[a]);
     }
     vg.rmax = std::max(vg.rmax, g / 2 + 1);
@@ -1743,20 +1733,31 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   // 2^-24): at most 8 roundings per axis, up to sqrt(3) of it in a distance,
   // and a few more of the squares and the square root.
   vg.ferr = (float)(24.0 * nmax * 0x1p-24);
+  // One pass over the points checks them and finds their buckets (a point at
+  // a bucket's edge may be rounded into the next one: ferr covers it).  The
+  // host side of seeding 2048^2 sites from 42,000 points is passes over the
+  // points: no divisions, no buffers cleared before they are filled.
+  const std::unique_ptr<int[]> bucket_of(new int[npoints]);
+  for (int k = 0; k < npoints; ++k) {
+    const double* p = points + (size_t)k * nd;
+    long long b = 0;
+    for (int a = nd - 1; a >= 0; --a) {
+      if (!(p[a] >= 0.0 && p[a] < (double)n[a]))
+        return h->fail(CPM_ERR_INVALID, "cpm_seed_voronoi_r: point %d lies outside [0, n)", k);
+      b = b * vg.g[a] + std::min((int)(p[a] * inv_w[a]), vg.g[a] - 1);
+    }
+    bucket_of[k] = (int)b;
+    const uint32_t v = values[k], id = v & 0xFFFFFFu, ty = v >> 24;
+    if ((int)id > R.ncells || ty >= (uint32_t)kMaxTypes || (id == 0 && ty != 0))
+      return h->fail(CPM_ERR_INVALID,
+                     "cpm_seed_voronoi_r: value %d is not id <= ncells | type < 32 << 24 "
+                     "(id 0 with type 0)", k);
+  }
   if (G > (1LL << 30))
     return h->fail(CPM_ERR_INVALID, "cpm_seed_voronoi_r: too many buckets");
   // Counting sort of the points by bucket (host; O(npoints)).
-  std::vector<int> bucket_of(npoints), start(G + 1, 0);
-  for (int k = 0; k < npoints; ++k) {
-    long long b = 0;
-    for (int a = nd - 1; a >= 0; --a) {
-      int ba = (int)std::floor(points[(size_t)k * nd + a] / w[a]);
-      ba = std::max(0, std::min(ba, vg.g[a] - 1));
-      b = b * vg.g[a] + ba;
-    }
-    bucket_of[k] = (int)b;
-    ++start[b + 1];
-  }
+  std::vector<int> start(G + 1, 0);
+  for (int k = 0; k < npoints; ++k) ++start[bucket_of[k] + 1];
   for (long long b = 0; b < G; ++b) start[b + 1] += start[b];
   // Work bound.  A site's search ends within about (d + 1) sqrt(ndim)
   // max(w) / min(w) + 1 rings, d the Chebyshev distance (in buckets, wrapped)
@@ -1767,22 +1768,24 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   // refused instead of launched.
   {
     std::vector<int> dist(G, -1), frontier, next;
-    auto neighbours = [&](int b, auto&& f) {  // f(b2) for the wrapped neighbours
-      const int bx = b % vg.g[0], by = (b / vg.g[0]) % vg.g[1], bz = b / (vg.g[0] * vg.g[1]);
+    // f(b2) for the wrapped neighbours, until it returns true
+    auto neighbours = [&](int b, auto&& f) {
+      const int gx = vg.g[0], gy = vg.g[1], gz = vg.g[2];
+      const int bx = b % gx, by = (b / gx) % gy, bz = b / (gx * gy);
+      auto wrap = [](int i, int g) { return i < 0 ? i + g : (i < g ? i : i - g); };
       for (int dz = (nd == 3 ? -1 : 0); dz <= (nd == 3 ? 1 : 0); ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-          for (int dx = -1; dx <= 1; ++dx) {
-            const int x2 = (bx + dx + vg.g[0]) % vg.g[0], y2 = (by + dy + vg.g[1]) % vg.g[1],
-                      z2 = (bz + dz + vg.g[2]) % vg.g[2];
-            f((z2 * vg.g[1] + y2) * vg.g[0] + x2);
-          }
+        for (int dy = -1; dy <= 1; ++dy) {
+          const int row = (wrap(bz + dz, gz) * gy + wrap(by + dy, gy)) * gx;
+          for (int dx = -1; dx <= 1; ++dx)
+            if (f(row + wrap(bx + dx, gx))) return;
+        }
     };
     for (long long b = 0; b < G; ++b)
       if (start[b + 1] > start[b]) dist[b] = 0;
     for (long long b = 0; b < G; ++b) {
       if (dist[b] >= 0) continue;
       bool near = false;
-      neighbours((int)b, [&](int b2) { near = near || dist[b2] == 0; });
+      neighbours((int)b, [&](int b2) { return near = dist[b2] == 0; });
       if (near) frontier.push_back((int)b);
     }
     for (int b : frontier) dist[b] = 1;
@@ -1794,6 +1797,7 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
             dist[b2] = d;
             next.push_back(b2);
           }
+          return false;
         });
       frontier.swap(next);
     }
@@ -1817,37 +1821,36 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
                      "search (about %.3g distance evaluations); spread them more evenly or "
                      "label the lattice on the host", work);
   }
-  // One upload: FP32 points, double points, original indices, values, starts.
+  // Up go the caller's points and values as they are, and the order of the
+  // points by bucket with the buckets' starts; a kernel lays the points out in
+  // that order.  (Laid out here, 44 bytes a point in a fresh buffer, they took
+  // 0.45 of the 0.88 ms of seeding 2048^2 sites from 42,000 points.)
   const size_t np = (size_t)npoints;
-  const size_t off_p = sizeof(float4) * np, off_i = off_p + sizeof(double) * 3 * np,
-               off_v = off_i + sizeof(int) * np, off_s = off_v + sizeof(uint32_t) * np,
-               bytes = off_s + sizeof(int) * (size_t)(G + 1);
-  std::vector<char> up(bytes);
-  float4* fpts = reinterpret_cast<float4*>(up.data());
-  double* pts = reinterpret_cast<double*>(up.data() + off_p);
-  int* idx = reinterpret_cast<int*>(up.data() + off_i);
-  std::vector<int> fill(start.begin(), start.end() - 1);
-  for (int k = 0; k < npoints; ++k) {
-    const int slot = fill[bucket_of[k]]++;
-    double c[3] = {0.0, 0.0, 0.0};
-    for (int a = 0; a < nd; ++a) c[a] = points[(size_t)k * nd + a];
-    for (int a = 0; a < 3; ++a) pts[(size_t)slot * 3 + a] = c[a];
-    fpts[slot] = make_float4((float)c[0], (float)c[1], (float)c[2], 0.0f);
-    idx[slot] = k;
-  }
-  std::memcpy(up.data() + off_v, values, sizeof(uint32_t) * np);
-  std::memcpy(up.data() + off_s, start.data(), sizeof(int) * (size_t)(G + 1));
+  const size_t off_p = sizeof(float4) * np, off_r = off_p + sizeof(double) * 3 * np,
+               off_i = off_r + sizeof(double) * nd * np, off_s = off_i + sizeof(int) * np,
+               off_v = off_s + sizeof(int) * (size_t)(G + 1),
+               bytes = off_v + sizeof(uint32_t) * np;
+  const std::unique_ptr<int[]> up(new int[np + G + 1]);  // order, starts
+  std::copy(start.begin(), start.end(), up.get() + np);
+  for (int k = 0; k < npoints; ++k) up[start[bucket_of[k]]++] = k;
   if (int rc = ensure_scratch(h, bytes)) return rc;
   char* dev = h->d_scratch;
-  cudaError_t e = cudaMemcpyAsync(dev, up.data(), bytes, cudaMemcpyHostToDevice, h->stream);
+  cudaError_t e = cudaMemcpyAsync(dev + off_r, points, sizeof(double) * nd * np,
+                                  cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess)
-    e = launch_voronoi(h->d_lat + R.lat_off, vg, reinterpret_cast<const double*>(dev + off_p),
-                       reinterpret_cast<const float4*>(dev),
+    e = cudaMemcpyAsync(dev + off_i, up.get(), off_v - off_i, cudaMemcpyHostToDevice, h->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dev + off_v, values, sizeof(uint32_t) * np, cudaMemcpyHostToDevice,
+                        h->stream);
+  if (e == cudaSuccess)
+    e = launch_voronoi(h->d_lat + R.lat_off, vg, npoints,
+                       reinterpret_cast<const double*>(dev + off_r),
+                       reinterpret_cast<double*>(dev + off_p), reinterpret_cast<float4*>(dev),
                        reinterpret_cast<const int*>(dev + off_i),
                        reinterpret_cast<const uint32_t*>(dev + off_v),
                        reinterpret_cast<const int*>(dev + off_s), h->stream);
-  h->launches += 1;
-  // the host buffer is read by the copy: wait before it goes
+  h->launches += 2;
+  // the host buffers are read by the copies: wait before they go
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_seed_voronoi_r");
   if (e2 != cudaSuccess) return h->cuda_fail(e2, "cpm_seed_voronoi_r");

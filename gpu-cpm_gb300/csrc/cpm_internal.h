@@ -286,10 +286,11 @@ struct VoronoiGrid {
   int ndim;
   int rmax;         // rings to scan at most (covers every bucket)
 };
-cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, const double* pts,
-                           const float4* fpts, const int* idx, const uint32_t* values,
-                           const int* start,
-                           cudaStream_t s);
+// raw: the points as given; idx: their order by bucket; pts, fpts: room for
+// them in that order (filled here); start: first place of each bucket.
+cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, int npoints, const double* raw,
+                           double* pts, float4* fpts, const int* idx, const uint32_t* values,
+                           const int* start, cudaStream_t s);
 // Boundary counts per replica and unordered type pair: Moore pairs (each
 // once) of sites with different values, counts[r*T*T + a*T + b] for a <= b
 // (types >= T are skipped).  tile_start: per replica the first of its tiles
