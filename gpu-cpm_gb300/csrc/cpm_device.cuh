@@ -121,6 +121,10 @@ __device__ __forceinline__ long long nearest_image(int xc, int n, long long a,
   return xc;
 }
 
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& d) {
+  return __umulhi(n, d.mul) >> d.shift;
+}
+
 __device__ __forceinline__ unsigned long long global_timer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -116,10 +116,6 @@ struct ReplicaCtx : DevReplica, ParamHead {
   int rep;
 };
 
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& d) {
-  return __umulhi(n, d.mul) >> d.shift;
-}
-
 // Act model (src/kernels2d.cu:338-473, src/kernels3d.cu:347-470): the
 // geometric mean of max(amax + act[i] - tick, 0) over site (x, y, z) and
 // those of its neighbours that hold `id`, as exp2 of the mean log2 (own

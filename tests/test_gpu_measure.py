@@ -51,3 +51,25 @@ def test_voronoi_near_ties(engine_lib, shape, gap):
     e.seed_voronoi(0, pts, vals)
     e.pull_from_gpu()
     np.testing.assert_array_equal(e.lattice(0).view(np.uint32), oracle.voronoi(shape, pts, vals))
+
+
+@pytest.mark.parametrize("shape", [(3, (1 << 24) + 5), (40, 64), (7, 33), (5, 6, 67)])
+@pytest.mark.parametrize("width", [1, 5, 400])
+def test_recount_sums_runs_of_sites(engine_lib, shape, width):
+    """Tables of cells that are runs of `width` sites in raster order (across
+    rows, warps and blocks, medium between them), also where a side is too
+    long for 32-bit sums: those of the oracle."""
+    import gpucpm
+    sites = int(np.prod(shape))
+    run = np.arange(sites) // (width if sites < 10**6 else sites // 50 * width // 400 + 1)
+    ids = run % 7 * (1 + run // 7 % 40)
+    ncells = int(ids.max())
+    lat = (ids | np.where(ids > 0, 1 + ids % 3, 0) << 24).astype(np.uint32).reshape(shape)
+    dims = shape[::-1] + ((1,) if len(shape) == 2 else ())
+    e = gpucpm.create_box(*dims, len(shape), ncells, 5.0)
+    e.lattice(0)[...] = lat.view(np.int32)
+    e.push_to_gpu()
+    e.synchronize()
+    sim = oracle.OracleSim(lat, ncells, np.zeros((4, 4), np.float32), [0] * 4, [0] * 4)
+    for got, want in zip(e.tables(0), (sim.area, sim.perim, sim.csum)):
+        np.testing.assert_array_equal(got, want)
