@@ -68,8 +68,8 @@ def parse_args():
                    help="tile variant instead of the autotuner's choice (profiling runs: "
                         "timing under a profiler can change the tuner's pick)")
     p.add_argument("--fill", choices=["parity", "vector", "tma", "cluster"], default=None,
-                   help="single 2D lattices: how tiles are staged instead of the engine's "
-                        "default (see cpm_set_fill)")
+                   help="single 2D lattices: the cluster sweep, or (any other) the grid sweep, "
+                        "instead of the engine's default (see cpm_set_fill)")
     p.add_argument("--dispatch", choices=["grid", "replica", "hybrid"], default=None,
                    help="batches: dispatch instead of the autotuner's choice")
     p.add_argument("--no-cpu-baseline", action="store_true")
@@ -585,12 +585,9 @@ def run_ours(args, world, rank, local, emit=True):
                 "frac": achieved / peak, "peak_source": f"{peak_kind} HBM copy (burst)",
                 "traffic": tpa * attempts_per_launch if tpa is not None else None,
                 "algorithmic_bytes_per_launch": BYTES_PER_ATTEMPT * attempts_per_launch,
-                "kernel": {"parity": "sweep_kernel (one cooperative launch per step)",
-                           "cluster": "sweep2d_kernel, cluster mode (one launch of one "
-                                      "thread-block cluster per step)"}.get(
-                    sim.sweep_config()["fill"],
-                    ("sweep2d_kernel" if w.ndim == 2 else "sweep3d_kernel")
-                    + " (one cooperative launch per step)")}
+                "kernel": ("cluster_sweep_kernel (one launch of one thread-block cluster per "
+                           "step)" if sim.sweep_config()["fill"] == "cluster" else
+                           "sweep_kernel (one cooperative launch per step)")}
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

@@ -14,15 +14,17 @@
 //                                        flight alternate)
 //   dlist  : uint32 [grid * 2 * list_cap] two dirty lists per sweep block:
 //                                        rows changed in a phase (a row may
-//                                        appear more than once)
-//   ctl    : uint32 [64]                 barrier counter / release flag,
-//                                        replica queue, sticky error bits
+//                                        appear more than once); used where
+//                                        rows are many (SweepArgs::scan)
+//   ctl    : uint32 [64]                 barrier counter, replica queue,
+//                                        sticky error bits
 //   (optional) field (chemotaxis, float), act stamps (uint32 per site),
 //   prefdir [rows][3] and the persistence ring [history][rows][3] (double)
 // Table double buffering: phase k reads copy k % 2 and adds its deltas both
 // into the other copy and into dap/dcs[k % 2]; phase k + 1 replays those
-// deltas into copy k % 2, which missed them (each delta is taken with an
-// exchange, so a row listed twice is replayed once).  So every phase reads
+// deltas into copy k % 2, which missed them (every row looked at by one thread,
+// or each delta of a listed row taken with an exchange, so that a row listed
+// twice is replayed once).  So every phase reads
 // tables as they stood when it began, with one grid barrier per phase.  The
 // tables are
 // small next to the lattice (4096^2 at 100 sites per cell: 67 MB of lattice,
@@ -41,8 +43,9 @@ constexpr int kInitThreads = 256;
 // How the slots of a sweep are cut into warp tasks of 32 target columns x
 // `rows` target rows, `kr` of them drawn side by side.  The sweep's result
 // does not depend on it.  Four variants; the autotuner (cpm_autotune) picks
-// one per engine.  Variant 0 follows from the size (plan_sweep, plan_batch),
-// 1 has 8-row tasks, 2 16-row tasks, 3 one-row tasks.
+// one per engine.  Variant 0 follows from the size (plan_sweep, batch_rows),
+// 1 has 8-row tasks, 2 16-row tasks, 3 one-row tasks (batches
+// 8, 32 and 2).
 constexpr int kTileVariants = 4;
 struct SweepPlan {
   int kr, rows;

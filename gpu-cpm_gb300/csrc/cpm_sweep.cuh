@@ -36,8 +36,8 @@
 // 3.61 ms; 4096^2 tissue, 50 MCS, 8.44 -> 7.65 ms; a 101 x 75 x 61 box, 20
 // MCS, 5.09 -> 2.84 ms.
 //
-// Bound: instruction issue on large lattices (7 warp instructions per
-// attempt in 2D), the chain of one warp through a phase on small ones: draw,
+// Bound: instruction issue on large lattices (6 warp instructions per
+// attempt in 2D, 10 in 3D), the chain of one warp through a phase on small ones: draw,
 // two L2 round trips, ~400 instructions, the grid barrier (2,600 cycles, 3,200
 // with reductions outstanding).
 //

@@ -280,7 +280,7 @@ int cpm_run(cpm_handle* h, int mcs);
 int cpm_run_graph(cpm_handle* h, int mcs);
 
 /* Dispatch of a sweep launch over the replicas of a batch:
- *   CPM_DISPATCH_GRID     the tiles of a slot, over all replicas, go to all
+ *   CPM_DISPATCH_GRID     the tasks of a slot, over all replicas, go to all
  *                         warps of the grid; one grid barrier per phase
  *                         (one large lattice, or a few);
  *   CPM_DISPATCH_REPLICA  each block claims whole replicas, largest first,
@@ -301,8 +301,8 @@ int cpm_run_graph(cpm_handle* h, int mcs);
 #define CPM_DISPATCH_REPLICA 1
 #define CPM_DISPATCH_HYBRID 2
 
-/* Project autotuner: times `probe_mcs` MCS of every compiled tile variant
- * (warp tile shape and warps per block), under each dispatch for a batch
+/* Project autotuner: times `probe_mcs` MCS of every variant (rows of targets
+ * per warp task), under each dispatch for a batch
  * (grid, replica, and hybrid where it splits the batch into two parts),
  * three times each (the fastest run counts: a first launch also loads its
  * module; a GPU coming out of idle should be warmed up first),
@@ -314,9 +314,9 @@ int cpm_run_graph(cpm_handle* h, int mcs);
  * (src/python_wrapper.cpp:182-227). */
 int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs);
 
-/* Select a tile variant (0 to 3) or a dispatch explicitly / describe the
- * current launch: warp tile extent in targets, warps per block, grid size
- * and dispatch. */
+/* Select a variant (0: rows per warp task from the size, 1 to 3: fixed) or a
+ * dispatch explicitly / describe the current launch: extent of a warp's task
+ * in targets, warps per block, grid size and dispatch. */
 int cpm_set_variant(cpm_handle* h, int variant);
 int cpm_set_dispatch(cpm_handle* h, int dispatch);
 int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
