@@ -179,7 +179,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
   constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
-  constexpr bool AHEAD = !BATCH && KR < 4;
+  constexpr bool AHEAD = !BATCH;
   constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
   // the pooled attempts (32 per warp), then the warps' queues
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -402,13 +402,14 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       load_source(u);
     }
   };
-  // The phase of slot `slot` at MCS `tick`; in the kernels of small lattices
-  // (AHEAD) also the draws of this warp's first task, often its only one.
-  // They read no site and no table, so they are made between the block's
-  // arrival at the barrier before the phase and its wait: 101 x 75 x 61 box,
-  // 20 MCS 2.78 -> 2.52 ms; 1001 x 777, 20 MCS 0.98 -> 0.90; 96^3 with
-  // persistence 1.46 -> 1.40; act on 512^2, 50 MCS 1.90 -> 1.82.  With four
-  // rows the held draws spill (4096^2, 50 MCS 7.07 -> 7.80).
+  // The phase of slot `slot` at MCS `tick`, and (one lattice) the draws of this
+  // warp's first task, in small lattices its only one.  They read no site and
+  // no table, so they are made between the block's arrival at the barrier before
+  // the phase and its wait, and are kept in the warp's queue, empty then: 101 x
+  // 75 x 61 box, 20 MCS 2.78 -> 2.51 ms; 1001 x 777, 20 MCS 0.98 -> 0.86; 96^3
+  // with persistence 1.46 -> 1.33; act on 512^2, 50 MCS 1.90 -> 1.80; 4096^2, 50
+  // MCS 6.97 -> 6.70; 256^3, 20 MCS 3.54 -> 3.28.  (Held in registers they made
+  // every kernel spill: 4096^2 7.80.)
   bool drawn = false;
   auto begin_phase = [&](const int slot, const unsigned long long tick, const int b, const int G) {
     cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
@@ -427,6 +428,10 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       if (drawn) {
         place(task);
         draw_rows([](int) {}, [](int) {});
+        uint4* const q = reinterpret_cast<uint4*>(queue);
+#pragma unroll
+        for (int u = 0; u < KR; ++u)
+          q[32 * u + lane] = make_uint4(site[u], source[u], word[u], (uint32_t)kd[u]);
       }
     }
   };
@@ -906,6 +911,13 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
         const unsigned fixed_mask = BATCH ? r_fixed : ctx.fixed_mask;
         if (AHEAD && drawn) {
           drawn = false;
+          const uint4* const q = reinterpret_cast<const uint4*>(queue);
+#pragma unroll
+          for (int u = 0; u < KR; ++u) {
+            const uint4 e = q[32 * u + lane];
+            site[u] = e.x, source[u] = e.y, word[u] = e.z, kd[u] = (int)e.w;
+          }
+          __syncwarp();  // the queue is written next
 #pragma unroll
           for (int u = 0; u < KR; ++u) tv[u] = L[site[u]], sv[u] = L[source[u]];
         } else {
