@@ -179,7 +179,6 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
   constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
-  constexpr bool AHEAD = !BATCH;
   constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
   // the pooled attempts (32 per warp), then the warps' queues
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -412,37 +411,68 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       load_source(u);
     }
   };
-  // The phase of slot `slot` at MCS `tick`, and (one lattice) the draws of this
-  // warp's first task, in small lattices its only one.  They read no site and
-  // no table, so they are made between the block's arrival at the barrier before
-  // the phase and its wait, and are kept in the warp's queue, empty then: 101 x
-  // 75 x 61 box, 20 MCS 2.78 -> 2.51 ms; 1001 x 777, 20 MCS 0.98 -> 0.86; 96^3
-  // with persistence 1.46 -> 1.33; act on 512^2, 50 MCS 1.90 -> 1.80; 4096^2, 50
-  // MCS 6.97 -> 6.70; 256^3, 20 MCS 3.54 -> 3.28.  (Held in registers they made
-  // every kernel spill: 4096^2 7.80.)
+  // The phase of slot `slot` at MCS `tick`, and the draws of this warp's first
+  // task, in small lattices its only one.  They read no site and no table, so
+  // they are made between the block's arrival at the barrier before the phase and
+  // its wait, and are kept in the warp's queue, empty then: 101 x 75 x 61 box, 20
+  // MCS 2.78 -> 2.51 ms; 1001 x 777, 20 MCS 0.98 -> 0.86; 96^3 with persistence
+  // 1.46 -> 1.33; act on 512^2, 50 MCS 1.90 -> 1.80; 4096^2, 50 MCS 6.97 -> 6.70;
+  // 256^3, 20 MCS 3.54 -> 3.28; batches of 16 x 64^2, 20 MCS 0.463 -> 0.444, of 32
+  // x 128^2 0.661 -> 0.613, large ones the same.  (Held in registers they made
+  // every kernel spill: 4096^2 7.80.)  Not in batches with scores, which it makes
+  // spill (gradient of 128 x 256^2 24.1 -> 24.4 ms).
+  constexpr bool AHEAD = !(BATCH && SCORE);
   bool drawn = false;
+  int first = 0;             // (batches) first task of the replica at hand
+  auto replica_of = [&](const int t) {
+    // the largest with pre[lo] <= t (tasks of the slot before each replica),
+    // 32 probes at a time
+    const int* pre = a.task_prefix + (cx + 3 * cy + 9 * cz) * (a.nrep + 1);
+    int lo = 0, n = a.nrep;
+    while (n > 1) {
+      const int st = (n + 31) >> 5, k = lane * st;
+      const int v = k < n ? __ldg(pre + lo + k) : 0;
+      const int at = __popc(__ballot_sync(kFull, k < n && v <= t)) - 1;
+      first = __shfl_sync(kFull, v, at);
+      lo += at * st;
+      n = min(st, n - at * st);
+    }
+    return a.rep_map ? __ldg(a.rep_map + lo) : lo;
+  };
+  auto switch_to = [&](const int rep) {
+    flush_counters();
+    __syncwarp();
+    load_replica(rep);
+    __syncwarp();
+    enter();
+  };
   auto begin_phase = [&](const int slot, const unsigned long long tick, const int b, const int G) {
     cx = slot % 3, cy = (slot / 3) % 3, cz = slot / 9;
     phase = tick * NSLOTS + (unsigned long long)slot;
-    if (!BATCH || r >= 0) enter();
-    if constexpr (!BATCH) {
-      task_grid();
-      ntasks = tnx * tny * class_count(nz, cz);
-    }
     task = b + warp * G;
     j = 0, j1 = -1;
     x = z = 0;
     in_x = false;
-    if constexpr (AHEAD) {
-      drawn = task < ntasks;
-      if (drawn) {
-        place(task);
-        draw_rows([](int) {}, [](int) {});
-        uint4* const q = reinterpret_cast<uint4*>(queue);
-#pragma unroll
-        for (int u = 0; u < KR; ++u)
-          q[32 * u + lane] = make_uint4(site[u], source[u], word[u], (uint32_t)kd[u]);
+    if constexpr (BATCH) {
+      ntasks = __ldg(a.task_prefix + slot * (a.nrep + 1) + a.nrep);
+    } else {
+      enter();
+      task_grid();
+      ntasks = tnx * tny * class_count(nz, cz);
+    }
+    if constexpr (AHEAD) drawn = task < ntasks;
+    if (AHEAD && drawn) {
+      if constexpr (BATCH) {
+        const int rep = replica_of(task);
+        if (rep != r) switch_to(rep);
+        task_grid();
       }
+      place(task - first);
+      draw_rows([](int) {}, [](int) {});
+      uint4* const q = reinterpret_cast<uint4*>(queue);
+#pragma unroll
+      for (int u = 0; u < KR; ++u)
+        q[32 * u + lane] = make_uint4(site[u], source[u], word[u], (uint32_t)kd[u]);
     }
   };
 
@@ -824,19 +854,12 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       }
     };
 
-    if constexpr (!AHEAD) begin_phase(slot, tick, b, G);
     const uint32_t* L = lat_r + (!BATCH || r >= 0 ? ctx.lat_off : 0);
-    const int* pre = nullptr;  // (batches) tasks of the slot before each replica
-    if constexpr (BATCH) {
-      pre = a.task_prefix + slot * (a.nrep + 1);
-      ntasks = __ldg(pre + a.nrep);
-    }
     unsigned* ctr = &s_next[step & 1];
     if (tid == 0) s_next[(step + 1) & 1] = 0u;
     int nq = 0;
-    int first = 0;           // (batches) its replica's first task
-    int next_rep = -1;       // (batches) the replica of the task at hand
-    bool rep_ready = !BATCH;  // its constants are loaded
+    int next_rep = -1;      // (batches) the replica of the task at hand
+    bool rep_ready = true;  // its constants are loaded
     int pool_at = -1, pool_n = 0;  // pooled stage: this warp's next batch, all attempts
     for (;;) {
       const Attempt* batch = queue;
@@ -874,25 +897,14 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
             break;
           }
           if constexpr (BATCH) {
-            // the largest with pre[lo] <= task, 32 probes at a time
-            int lo = 0, n = a.nrep;
-            while (n > 1) {
-              const int st = (n + 31) >> 5, k = lane * st;
-              const int v = k < n ? __ldg(pre + lo + k) : 0;
-              const int at = __popc(__ballot_sync(kFull, k < n && v <= task)) - 1;
-              first = __shfl_sync(kFull, v, at);
-              lo += at * st;
-              n = min(st, n - at * st);
-            }
-            next_rep = lo;
+            next_rep = replica_of(task);
             rep_ready = false;
             j1 = 1;  // a task is at hand
           }
         }
         if constexpr (BATCH) {
           if (!rep_ready) {
-            const int rep = a.rep_map ? __ldg(a.rep_map + next_rep) : next_rep;
-            if (rep != r) {
+            if (next_rep != r) {
               if (nq > 0) {  // the last replica's attempts first
                 nbatch = nq;
                 nq = 0;
@@ -900,11 +912,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
               }
               if constexpr (DEFER) flush_changes(1);
               if (SCORE && r >= 0) flush_scores(a, sc, r, tick);
-              flush_counters();
-              __syncwarp();
-              load_replica(rep);
-              __syncwarp();
-              enter();
+              switch_to(next_rep);
               L = lat_r + ctx.lat_off;
             }
             task_grid();
@@ -994,8 +1002,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
       __syncthreads();
     }
     int step = 0;
-    if constexpr (AHEAD)
-      if (a.mcs > 0) begin_phase(a.slots[0], s_tick0, b, G);
+    if (a.mcs > 0) begin_phase(a.slots[0], s_tick0, b, G);
     for (int m = 0; m < a.mcs; ++m) {
       const unsigned long long tick = s_tick0 + (unsigned long long)m;
       for (int si = 0; si < a.nslot_active; ++si, ++step) {
@@ -1009,11 +1016,9 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           s_pool = 0;
           if (!local) grid_arrive(a.ctl);
         }
-        if constexpr (AHEAD) {
-          const bool wrap = si + 1 == a.nslot_active;
-          if (!wrap || m + 1 < a.mcs)
-            begin_phase(a.slots[wrap ? 0 : si + 1], tick + (wrap ? 1 : 0), b, G);
-        }
+        const bool wrap = si + 1 == a.nslot_active;
+        if (!wrap || m + 1 < a.mcs)
+          begin_phase(a.slots[wrap ? 0 : si + 1], tick + (wrap ? 1 : 0), b, G);
         if (local)
           __syncthreads();
         else if (!grid_wait(a.ctl, ++episode, &s_ok))
