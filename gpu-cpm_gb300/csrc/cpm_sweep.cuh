@@ -172,13 +172,15 @@ __device__ __forceinline__ void flush_scores(const SweepArgs& a, float* sc, int 
   for (int k = 0; k < kScoreRegs; ++k) sc[k] = 0.0f;
 }
 
-template <int NDIM, int KR, int MODE, bool BATCH>
+// LOCAL: for replica dispatch, where the kernel differs (see s_pt).
+template <int NDIM, int KR, int MODE, bool BATCH, bool LOCAL>
 __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1)
     sweep_kernel(const __grid_constant__ SweepArgs a) {
   constexpr bool EXT = MODE == kExt, SCORE = MODE == kScore;
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
   constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
+  constexpr bool SHARED_PT = DEFER && !LOCAL;
   constexpr unsigned long long NSLOTS = NDIM == 2 ? 9 : 27;
   // the pooled attempts (32 per warp), then the warps' queues
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -192,8 +194,9 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
   // A phase's table pointers.  Where row changes are queued few instructions use
   // them, and the twelve registers do more for the rest (4096^2, 50 MCS 6.69 ->
   // 6.47 ms).  Elsewhere every accepted copy would wait for them (256 ragged
-  // replicas 16.6 -> 18.9 ms, 1001 x 777 0.87 -> 0.93).
-  __shared__ PhaseTables<NDIM> s_pt[DEFER ? 2 : 1];
+  // replicas 16.6 -> 18.9 ms, 1001 x 777 0.87 -> 0.93), and in replica dispatch a
+  // block's few rows change often (512 x 256^2 of small cells, 50 MCS 34.0 -> 39.1).
+  __shared__ PhaseTables<NDIM> s_pt[SHARED_PT ? 2 : 1];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wpb = blockDim.x >> 5;
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     return {cur ? a.ap[1] : a.ap[0], cur ? a.cs[1] : a.cs[0],   cur ? a.ap[0] : a.ap[1],
             cur ? a.cs[0] : a.cs[1], cur ? a.dap[1] : a.dap[0], cur ? a.dcs[1] : a.dcs[0]};
   };
-  if (DEFER && tid < 2) s_pt[tid] = tables_of(tid);
+  if (SHARED_PT && tid < 2) s_pt[tid] = tables_of(tid);
   // Every block reads *tick_ptr before its first barrier arrival, and block
   // 0 advances it only after its last barrier, so all blocks see one value.
   if (tid == 0) s_tick0 = a.tick_ptr ? __ldcg(a.tick_ptr) : a.tick0;
@@ -482,8 +485,8 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
                        const int G) {
     const int cur = step & 1;
     PhaseTables<NDIM> held;
-    if constexpr (!DEFER) held = tables_of(cur);
-    const PhaseTables<NDIM>& pt = DEFER ? s_pt[cur] : held;
+    if constexpr (!SHARED_PT) held = tables_of(cur);
+    const PhaseTables<NDIM>& pt = SHARED_PT ? s_pt[cur] : held;
     // the lattice (act stamps) the phase reads, and the one it writes:
     // another copy in act runs
     const bool two = EXT && a.act_on;
@@ -1040,15 +1043,15 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     *a.tick_ptr = s_tick0 + (unsigned long long)a.mcs;
 }
 
-template <int NDIM, int KR, int MODE, bool BATCH>
+template <int NDIM, int KR, int MODE, bool BATCH, bool LOCAL>
 struct SweepFn {
-  static const void* fn() { return (const void*)sweep_kernel<NDIM, KR, MODE, BATCH>; }
+  static const void* fn() { return (const void*)sweep_kernel<NDIM, KR, MODE, BATCH, LOCAL>; }
   static size_t smem(int warps) { return (size_t)warps * warp_smem<NDIM, KR, MODE, BATCH>(); }
 };
 
-template <int NDIM, int KR, int MODE, bool BATCH>
+template <int NDIM, int KR, int MODE, bool BATCH, bool LOCAL = false>
 cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_t s) {
-  using F = SweepFn<NDIM, KR, MODE, BATCH>;
+  using F = SweepFn<NDIM, KR, MODE, BATCH, LOCAL>;
   const int w = warps < sweep_warps<NDIM, KR, MODE, BATCH>() ? warps
                                                          : sweep_warps<NDIM, KR, MODE, BATCH>();
   const size_t smem = F::smem(w);
@@ -1083,7 +1086,10 @@ cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int gri
   }
   switch (a.kr) {
     case 1: return launch_sweep_as<NDIM, 1, kPlain, false>(a, grid, warps, s);
-    case 4: return launch_sweep_as<NDIM, 4, kPlain, false>(a, grid, warps, s);
+    case 4:
+      if (NDIM == 2 && a.block_local)
+        return launch_sweep_as<NDIM, 4, kPlain, false, NDIM == 2>(a, grid, warps, s);
+      return launch_sweep_as<NDIM, 4, kPlain, false>(a, grid, warps, s);
     default: return launch_sweep_as<NDIM, 3, kPlain, false>(a, grid, warps, s);
   }
 }
