@@ -544,10 +544,15 @@ cudaLaunchConfig_t cluster_config(const ClusterPlan& p, cudaStream_t s,
   return cfg;
 }
 
-cudaError_t cluster_attributes(const ClusterPlan& p) {
+// The largest plan (8 KB are left to the static arrays).  It is also the
+// function's limit, one value for every lattice: the limit belongs to the
+// function on the device, and engines in other threads set it too.
+constexpr int kClusterSmemMax = kSweepSmemMax - 8 * 1024;
+
+cudaError_t cluster_attributes() {
   const void* fn = (const void*)cluster_sweep_kernel;
   cudaError_t e =
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes);
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
@@ -559,10 +564,10 @@ int cluster_sweep_blocks(int nx, int ny, int ncells) {
   if (nx < 4 || nx > 0xFFF || ny > 0xFFF) return 0;  // (12-bit coordinates in messages)
   for (int G : {16, 8}) {
     const ClusterPlan p = make_plan(nx, ny, ncells, G);
-    if (p.bytes > (unsigned)kSweepSmemMax - 8 * 1024) continue;  // (8 KB of static arrays)
+    if (p.bytes > (unsigned)kClusterSmemMax) continue;
     cudaLaunchAttribute attr[1];
     int n = 0;
-    if (cluster_attributes(p) == cudaSuccess) {
+    if (cluster_attributes() == cudaSuccess) {
       const cudaLaunchConfig_t cfg = cluster_config(p, nullptr, attr);
       if (cudaOccupancyMaxActiveClusters(&n, (const void*)cluster_sweep_kernel, &cfg) !=
           cudaSuccess)
@@ -579,7 +584,7 @@ int cluster_sweep_threads() { return kClusterThreads; }
 cudaError_t launch_cluster_sweep(const SweepArgs& a, int nx, int ny, int ncells, int G,
                                  cudaStream_t s) {
   ClusterPlan p = make_plan(nx, ny, ncells, G);
-  const cudaError_t e = cluster_attributes(p);
+  const cudaError_t e = cluster_attributes();
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<SweepArgs*>(&a), &p};
   cudaLaunchAttribute attr[1];

@@ -1052,14 +1052,16 @@ struct SweepFn {
 template <int NDIM, int KR, int MODE, bool BATCH, bool LOCAL = false>
 cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_t s) {
   using F = SweepFn<NDIM, KR, MODE, BATCH, LOCAL>;
-  const int w = warps < sweep_warps<NDIM, KR, MODE, BATCH>() ? warps
-                                                         : sweep_warps<NDIM, KR, MODE, BATCH>();
-  const size_t smem = F::smem(w);
-  const cudaError_t e =
-      cudaFuncSetAttribute(F::fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr int kMaxWarps = sweep_warps<NDIM, KR, MODE, BATCH>();
+  const int w = warps < kMaxWarps ? warps : kMaxWarps;
+  // The limit belongs to the function on the device: every launch sets the
+  // same one, whatever its own size, so that a launch of another engine in
+  // another thread cannot lower it in between.
+  const cudaError_t e = cudaFuncSetAttribute(
+      F::fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem(kMaxWarps));
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<SweepArgs*>(&a)};
-  return cudaLaunchCooperativeKernel(F::fn(), dim3(grid), dim3(32 * w), args, smem, s);
+  return cudaLaunchCooperativeKernel(F::fn(), dim3(grid), dim3(32 * w), args, F::smem(w), s);
 }
 
 // One kernel per mode and rows drawn side by side (a.kr): one, three or four;
