@@ -1705,39 +1705,11 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   const DevReplica& R = h->reps[r];
   const int nd = h->ndim;
   const int n[3] = {R.nx, R.ny, R.nz};
-  // Bucket grid with about two points per bucket.
-  VoronoiGrid vg;
-  vg.ndim = nd;
-  const double sites = (double)n[0] * n[1] * n[2];
-  const double side = std::pow(2.0 * sites / npoints, 1.0 / nd);
-  long long G = 1;
-  double wmin = 1e300, wmax = 0.0, inv_w[3];
-  vg.rmax = 0;
-  int nmax = 1;
-  for (int a = 0; a < 3; ++a) {
-    vg.n[a] = n[a];
-    int g = a < nd ? (int)std::lround((double)n[a] / side) : 1;
-    g = std::max(1, std::min(g, n[a]));
-    vg.g[a] = g;
-    const double w = (double)n[a] / g;
-    inv_w[a] = (double)g / n[a];
-    vg.wf[a] = (float)w;
-    vg.inv_w[a] = (float)(1.0 / w);
-    if (a < nd) {
-      wmin = std::min(wmin, w);
-      wmax = std::max(wmax, w);
-      nmax = std::max(nmax, n[a]);
-    }
-    vg.rmax = std::max(vg.rmax, g / 2 + 1);
-    G *= g;
-  }
-  vg.lb_scale = (float)wmin;
-  // Coordinates and differences of up to nmax, each rounded to FP32 (relative
-  // 2^-24): at most 8 roundings per axis, up to sqrt(3) of it in a distance,
-  // and a few more of the squares and the square root.
-  vg.ferr = (float)(24.0 * nmax * 0x1p-24);
+  const VoronoiGrid vg = voronoi_grid(nd, n, npoints);
+  const double sites = (double)n[0] * n[1] * n[2], wmin = vg.wmin, wmax = vg.wmax;
+  const long long G = (long long)vg.g[0] * vg.g[1] * vg.g[2];
   // One pass over the points checks them and finds their buckets (a point at
-  // a bucket's edge may be rounded into the next one: ferr covers it).  The
+  // a bucket's edge may be rounded into the next one: the scans allow for it).  The
   // host side of seeding 2048^2 sites from 42,000 points is passes over the
   // points: no divisions, no buffers cleared before they are filled.
   const std::unique_ptr<int[]> bucket_of(new int[npoints]);
@@ -1747,7 +1719,7 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
     for (int a = nd - 1; a >= 0; --a) {
       if (!(p[a] >= 0.0 && p[a] < (double)n[a]))
         return h->fail(CPM_ERR_INVALID, "cpm_seed_voronoi_r: point %d lies outside [0, n)", k);
-      b = b * vg.g[a] + std::min((int)(p[a] * inv_w[a]), vg.g[a] - 1);
+      b = b * vg.g[a] + std::min((int)(p[a] * vg.inv[a]), vg.g[a] - 1);
     }
     bucket_of[k] = (int)b;
     const uint32_t v = values[k], id = v & 0xFFFFFFu, ty = v >> 24;

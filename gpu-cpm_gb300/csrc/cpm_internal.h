@@ -31,6 +31,8 @@
 // 4 MB per table copy) and stay L2-resident through a run.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -276,19 +278,65 @@ cudaError_t launch_observe_heterotypic(const uint32_t* lat, const DevReplica* re
 // Periodic Voronoi seeding of one lattice region (nx*ny*nz sites at `lat`):
 // every site takes values[k] of its nearest point (min-image Euclidean
 // distance in double, ties to the lowest k).  Points are binned in a
-// g[0]*g[1]*g[2] bucket grid of widths w[] (bucket-major order: pts[k*3+a],
+// g[0]*g[1]*g[2] bucket grid (bucket-major order: pts[k*3+a],
 // idx[k] their original index, start[b]..start[b+1] bucket b's points; fpts[k]
 // the same coordinates in FP32).
 struct VoronoiGrid {
   int n[3];         // lattice sides (n[2] = 1 in 2D)
   int g[3];         // buckets per axis
-  float inv_w[3];   // buckets per unit length, g / n
-  float wf[3];      // bucket widths n / g
-  float lb_scale;   // min(w): ring r bounds unscanned points at r * min(w)
+  double inv[3];    // buckets per unit length, g / n
+  double wmin, wmax;  // of the bucket widths n / g: ring r bounds unscanned points at r * wmin
+  float inv_w[3];   // the same in FP32
+  float wf[3];      // bucket widths in FP32
+  float lb_scale;   // wmin in FP32
   float ferr;       // bound on the error of a distance (and of a position) in FP32
   int ndim;
   int rmax;         // rings to scan at most (covers every bucket)
+  bool single;      // the rings are scanned in FP32 first
 };
+// Bucket grid with about two points per bucket.
+//
+// single: a scan in FP32 goes on until its lower bound, 3 ferr below the true
+// one, passes the nearest point, 3 ferr / wmin rings longer than one in double;
+// and every point within 2 ferr of the nearest is looked at again.  ferr grows
+// with the longest side (0.006 at 4096, 384 at 2^28), wmin with neither.  Up to
+// one ring more FP32 is the faster (ms of a call, double / FP32: 256^3 sites,
+// 30,000 points 72.8 / 2.7; 2^20 x 8 sites, 80,000 points, half a ring more
+// 23.4 / 6.8).  2^28 x 4 sites of 10^7 points would take 288 rings for 7, some
+// 6 x 10^14 distances, where the bound on a call's work counts 5 x 10^11: all
+// in double there.
+inline VoronoiGrid voronoi_grid(int ndim, const int (&n)[3], int npoints) {
+  VoronoiGrid vg;
+  vg.ndim = ndim;
+  const double sites = (double)n[0] * n[1] * n[2];
+  const double side = std::pow(2.0 * sites / npoints, 1.0 / ndim);
+  vg.wmin = 1e300, vg.wmax = 0.0;
+  vg.rmax = 0;
+  int nmax = 1;
+  for (int a = 0; a < 3; ++a) {
+    vg.n[a] = n[a];
+    int g = a < ndim ? (int)std::lround((double)n[a] / side) : 1;
+    g = std::max(1, std::min(g, n[a]));
+    vg.g[a] = g;
+    const double w = (double)n[a] / g;
+    vg.inv[a] = (double)g / n[a];
+    vg.wf[a] = (float)w;
+    vg.inv_w[a] = (float)(1.0 / w);
+    if (a < ndim) {
+      vg.wmin = std::min(vg.wmin, w);
+      vg.wmax = std::max(vg.wmax, w);
+      nmax = std::max(nmax, n[a]);
+    }
+    vg.rmax = std::max(vg.rmax, g / 2 + 1);
+  }
+  vg.lb_scale = (float)vg.wmin;
+  // Coordinates and differences of up to nmax, each rounded to FP32 (relative
+  // 2^-24): at most 8 roundings per axis, up to sqrt(3) of it in a distance,
+  // and a few more of the squares and the square root.
+  vg.ferr = (float)(24.0 * nmax * 0x1p-24);
+  vg.single = 3.0 * vg.ferr <= vg.wmin;
+  return vg;
+}
 // raw: the points as given; idx: their order by bucket; pts, fpts: room for
 // them in that order (filled here); start: first place of each bucket.
 cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, int npoints, const double* raw,

@@ -10,7 +10,8 @@
 //                              the mean-coordinate ring and the per-run
 //                              direction update (src/kernels.cu:159-212).
 //   lr_backward_kernel         likelihood-ratio gradient from score sums.
-//   voronoi_kernel             periodic Voronoi seeding (bucketed, exact).
+//   voronoi_kernel, voronoi_double_kernel
+//                              periodic Voronoi seeding (bucketed, exact).
 //   observe_heterotypic_kernel, observe_boundaries_kernel
 //                              sorting order parameter and boundary lengths
 //                              by type pair.
@@ -458,10 +459,12 @@ __global__ void __launch_bounds__(256)
 //
 // The rings are scanned in FP32 first, keeping the nearest point and the
 // distance of the second nearest: this chip has 2 FP64 lanes per SM, and a
-// distance takes 11 FP64 operations (all in FP64: 5.96 ms on a 2048^2
-// tissue, the whole seed / recount / measure sequence on it 9.94 ms, now 1.29).  A float distance is off by at most vg.ferr, so a nearest point
+// distance takes 11 FP64 operations (2048^2 sites, 42,000 points: 5.96 ms all
+// in FP64).  A float distance is off by at most vg.ferr, so a nearest point
 // that leads by more than 2 ferr is the answer; only where the lead is
-// smaller (ties, points midway) are the site's rings scanned in double.
+// smaller (ties, points midway) are the site's rings scanned in double.  On
+// lattices so long that ferr is no longer small against a bucket
+// (VoronoiGrid::single) voronoi_double_kernel scans them in double alone.
 __device__ __forceinline__ double min_image(double a, double b, int n) {
   const double d = fabs(__dsub_rn(a, b));
   const double e = __dsub_rn((double)n, d);
@@ -495,6 +498,29 @@ __device__ __forceinline__ void scan_ring(const VoronoiGrid& vg, const int* __re
         visit(__ldg(start + bucket), __ldg(start + bucket + 1));
       }
     }
+  }
+}
+
+// The nearest point so far, in double, ties to the lowest index.
+struct Nearest {
+  double d2 = 1e300;
+  int k = 0x7FFFFFFF;
+};
+template <int NDIM>
+__device__ __forceinline__ void take_nearer(const VoronoiGrid& vg, const double* __restrict__ pts,
+                                            const int* __restrict__ idx, int j, int x, int y,
+                                            int z, Nearest& best) {
+  const double ddx = min_image((double)x, __ldg(pts + 3LL * j), vg.n[0]);
+  const double ddy = min_image((double)y, __ldg(pts + 3LL * j + 1), vg.n[1]);
+  double d2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
+  if (NDIM == 3) {
+    const double ddz = min_image((double)z, __ldg(pts + 3LL * j + 2), vg.n[2]);
+    d2 = __dadd_rn(d2, __dmul_rn(ddz, ddz));
+  }
+  const int k = __ldg(idx + j);
+  if (d2 < best.d2 || (d2 == best.d2 && k < best.k)) {
+    best.d2 = d2;
+    best.k = k;
   }
 }
 
@@ -573,30 +599,47 @@ __global__ void __launch_bounds__(256)
     if (best_j >= 0 && second > lead2) {
       out = __ldg(values + __ldg(idx + best_j));
     } else {  // the points that may be nearest, in double
-      double dbest = 1e300;
-      int best_k = 0x7FFFFFFF;
+      Nearest near;
       for (int q = 0; q <= min(r, vg.rmax); ++q) {
         scan_ring<NDIM>(vg, start, b, q, [&](int k0, int k1) {
-          for (int k = k0; k < k1; ++k) {
-            if (dist2(__ldg(fpts + k)) > lead2) continue;
-            const double ddx = min_image((double)x, __ldg(pts + 3LL * k), vg.n[0]);
-            const double ddy = min_image((double)y, __ldg(pts + 3LL * k + 1), vg.n[1]);
-            double d2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
-            if (NDIM == 3) {
-              const double ddz = min_image((double)z, __ldg(pts + 3LL * k + 2), vg.n[2]);
-              d2 = __dadd_rn(d2, __dmul_rn(ddz, ddz));
-            }
-            const int kk = __ldg(idx + k);
-            if (d2 < dbest || (d2 == dbest && kk < best_k)) {
-              dbest = d2;
-              best_k = kk;
-            }
-          }
+          for (int k = k0; k < k1; ++k)
+            if (dist2(__ldg(fpts + k)) <= lead2)
+              take_nearer<NDIM>(vg, pts, idx, k, x, y, z, near);
         });
       }
-      if (best_k != 0x7FFFFFFF) out = __ldg(values + best_k);
+      if (near.k != 0x7FFFFFFF) out = __ldg(values + near.k);
     }
     lat[s] = out;
+  }
+}
+
+// The same in double alone.
+template <int NDIM>
+__global__ void __launch_bounds__(256)
+    voronoi_double_kernel(uint32_t* lat, const VoronoiGrid vg, const double* __restrict__ pts,
+                          const int* __restrict__ idx, const uint32_t* __restrict__ values,
+                          const int* __restrict__ start) {
+  const unsigned sites = (unsigned)vg.n[0] * vg.n[1] * vg.n[2];  // < 2^31
+  for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < sites;
+       s += gridDim.x * blockDim.x) {
+    const int x = (int)(s % vg.n[0]), yz = (int)(s / vg.n[0]);
+    const int y = NDIM == 3 ? yz % vg.n[1] : yz, z = NDIM == 3 ? yz / vg.n[1] : 0;
+    const int xyz[3] = {x, y, z};
+    int b[3] = {0, 0, 0};
+#pragma unroll
+    for (int a = 0; a < NDIM; ++a)
+      b[a] = min((int)__dmul_rn((double)xyz[a], vg.inv[a]), vg.g[a] - 1);
+    Nearest near;
+    for (int r = 0; r <= vg.rmax; ++r) {
+      scan_ring<NDIM>(vg, start, b, r, [&](int k0, int k1) {
+        for (int k = k0; k < k1; ++k) take_nearer<NDIM>(vg, pts, idx, k, x, y, z, near);
+      });
+      // every bucket not scanned yet lies r * wmin away at least; the margin
+      // covers the rounding of the bucket indices
+      const double lb = __dsub_rn(__dmul_rn((double)r, vg.wmin), 1e-6);
+      if (near.k != 0x7FFFFFFF && lb > 0.0 && near.d2 < __dmul_rn(lb, lb)) break;
+    }
+    lat[s] = near.k != 0x7FFFFFFF ? __ldg(values + near.k) : 0u;
   }
 }
 
@@ -663,7 +706,12 @@ cudaError_t launch_voronoi(uint32_t* lat, const VoronoiGrid& vg, int npoints, co
   const int grid = (int)std::max(1LL, std::min<long long>((sites + 255) / 256, (long long)sms * 16));
   voronoi_order_kernel<<<(npoints + 255) / 256, 256, 0, s>>>(vg.ndim, npoints, raw, idx, pts,
                                                              fpts);
-  if (vg.ndim == 2)
+  if (!vg.single) {
+    if (vg.ndim == 2)
+      voronoi_double_kernel<2><<<grid, 256, 0, s>>>(lat, vg, pts, idx, values, start);
+    else
+      voronoi_double_kernel<3><<<grid, 256, 0, s>>>(lat, vg, pts, idx, values, start);
+  } else if (vg.ndim == 2)
     voronoi_kernel<2><<<grid, 256, 0, s>>>(lat, vg, pts, fpts, idx, values, start);
   else
     voronoi_kernel<3><<<grid, 256, 0, s>>>(lat, vg, pts, fpts, idx, values, start);
