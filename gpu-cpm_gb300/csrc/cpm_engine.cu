@@ -171,15 +171,16 @@ struct cpm_handle {
   } cfg[kTileVariants];
   int variant = 0;
   int dispatch = CPM_DISPATCH_GRID;  // CPM_DISPATCH_*
-  // CPM_FILL_*.  Until the caller or the autotuner chooses one (fill_auto) the
-  // engine runs the cluster sweep (cpm_cluster.cu) on small lattices that fit
-  // it, else the grid sweep (cpm_sweep.cuh); CPM_FILL_CLUSTER asks for the cluster sweep,
-  // the other fills for the grid sweep.  row_ok: the shapes that accept
-  // CPM_FILL_VECTOR and CPM_FILL_TMA; cluster_fill: those that accept
-  // CPM_FILL_CLUSTER.
+  // CPM_FILL_*, as cpm_get_fill tells it.  Until the caller or the autotuner
+  // chooses one (fill_by) the engine runs the cluster sweep (cpm_cluster.cu) on
+  // small lattices that fit it, else the grid sweep (cpm_sweep.cuh);
+  // CPM_FILL_CLUSTER asks for the cluster sweep, the other fills for the grid
+  // sweep.  row_ok: the shapes that accept CPM_FILL_VECTOR and CPM_FILL_TMA;
+  // cluster_shape: those that accept CPM_FILL_CLUSTER even where their tables
+  // do not fit (cluster_blocks = 0) and the grid sweep runs.
   int fill = CPM_FILL_PARITY;
-  bool fill_auto = true;
-  bool row_ok = false, cluster_fill = false;
+  enum { kBySize, kByTuner, kByCaller } fill_by = kBySize;
+  bool row_ok = false, cluster_shape = false;
   int cluster_blocks = 0;  // blocks of the cluster that holds the lattice (0: none)
   std::vector<unsigned long long> attempts;  // per replica, host-counted
 
@@ -279,9 +280,9 @@ void free_all(cpm_handle* h) {
 bool rows_fit(int ndim, int nx, int ny, int nz) {
   return nx % 4 == 0 && nx >= 72 && (ndim == 2 ? ny >= 66 : ny >= 18 && nz >= 18);
 }
-// Shapes that accept CPM_FILL_CLUSTER: about 190 KB of rows per block of a
-// 16-block cluster.
-bool cluster_fits(int nx, int ny) {
+// Shapes whose rows alone fit a cluster, about 190 KB of them per block of 16
+// (cpm_handle::cluster_shape).
+bool cluster_rows_fit(int nx, int ny) {
   if (!rows_fit(2, nx, ny, 1)) return false;
   for (int g : {16, 8}) {
     const long long h = (ny + g - 1) / g;
@@ -417,7 +418,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
   if (n == 1 && rows_fit(ndim, nx[0], ny[0], nz ? nz[0] : 1)) {
     h->row_ok = true;
     h->fill = CPM_FILL_TMA;
-    if (ndim == 2) h->cluster_fill = cluster_fits(nx[0], ny[0]);
+    if (ndim == 2) h->cluster_shape = cluster_rows_fit(nx[0], ny[0]);
   }
   if (n == 1 && ndim == 2) h->cluster_blocks = cluster_sweep_blocks(nx[0], ny[0], ncells[0]);
 
@@ -886,7 +887,7 @@ const SweepPlan& plan_of(const cpm_handle* h, int v, int d, bool scores = false)
 
 int grid_of(const cpm_handle* h, int v, int d) { return plan_of(h, v, d).grid; }
 
-int fill_key(const cpm_handle* h) { return h->fill_auto ? -2 : h->fill; }
+int fill_key(const cpm_handle* h) { return h->fill_by == cpm_handle::kBySize ? -2 : h->fill; }
 
 // Whether plain runs take the cluster sweep.
 // By itself up to the size where the grid sweep, whose phases take 4.8 us
@@ -895,7 +896,8 @@ int fill_key(const cpm_handle* h) { return h->fill_auto ? -2 : h->fill; }
 constexpr long long kClusterAutoSites = 140000;
 bool uses_cluster(const cpm_handle* h) {
   return h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
-         (h->fill_auto ? h->total_sites <= kClusterAutoSites : h->fill == CPM_FILL_CLUSTER);
+         (h->fill_by == cpm_handle::kBySize ? h->total_sites <= kClusterAutoSites
+                                            : h->fill == CPM_FILL_CLUSTER);
 }
 
 // The launches of one sweep run (`a` from sweep_args, times filled in): one
@@ -1566,10 +1568,13 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   // A lattice that one thread-block cluster can hold is also tried in the
   // cluster sweep (which has no tile variants), unless the caller chose the
   // parity fill.
-  const int row_fill = h->fill == CPM_FILL_CLUSTER ? CPM_FILL_TMA : h->fill;
-  const bool fill_auto = h->fill_auto;
-  h->fill_auto = false;
-  if (h->cluster_blocks > 0 && (fill_auto || h->fill != CPM_FILL_PARITY))
+  const int row_fill = h->fill != CPM_FILL_CLUSTER ? h->fill
+                       : h->row_ok                 ? CPM_FILL_TMA
+                                                   : CPM_FILL_PARITY;
+  const auto fill_by = h->fill_by;
+  h->fill_by = cpm_handle::kByTuner;
+  if (h->cluster_blocks > 0 &&
+      (fill_by == cpm_handle::kBySize || h->fill != CPM_FILL_PARITY))
     pairs.emplace_back(h->variant, -1);
   int best_fill = row_fill;
   const int npairs = (int)pairs.size();
@@ -1598,7 +1603,8 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
     }
   }
   h->fill = best_fill;
-  h->fill_auto = fill_auto && h->cluster_blocks == 0;
+  if (fill_by == cpm_handle::kBySize ? h->cluster_blocks == 0 : best_fill == row_fill)
+    h->fill_by = fill_by;
   if (e == cudaSuccess) e = copy(false);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(save);
@@ -1898,21 +1904,31 @@ int cpm_set_fill(cpm_handle* h, int fill) {
       fill != CPM_FILL_CLUSTER)
     return h->fail(CPM_ERR_INVALID, "fill %d is not parity (0), vector (1), tma (2) or "
                                     "cluster (3)", fill);
-  if (fill == CPM_FILL_CLUSTER && !h->cluster_fill)
+  if (fill == CPM_FILL_CLUSTER && h->cluster_blocks == 0 && !h->cluster_shape)
     return h->fail(CPM_ERR_UNSUPPORTED, "no thread-block cluster holds this lattice (one 2D "
-                                        "lattice that fits row tiles and ~190 KB of rows per "
-                                        "block of a 16- or 8-block cluster)");
-  if (fill != CPM_FILL_PARITY && !h->row_ok)
-    return h->fail(CPM_ERR_UNSUPPORTED, "row tiles need one lattice with nx a multiple of 4 "
+                                        "lattice, nx from 4 and sides to 4095, that fits the "
+                                        "shared memory of 16 or 8 blocks with its tables)");
+  if ((fill == CPM_FILL_VECTOR || fill == CPM_FILL_TMA) && !h->row_ok)
+    return h->fail(CPM_ERR_UNSUPPORTED, "vector and tma need one lattice with nx a multiple of 4 "
                                         "and nx >= 72; in 2D ny >= 66, in 3D ny, nz >= 18");
   h->fill = fill;
-  h->fill_auto = false;
+  h->fill_by = cpm_handle::kByCaller;
   return CPM_OK;
 }
 
 int cpm_get_fill(const cpm_handle* h, int* fill) {
   if (!h || !fill) return CPM_ERR_INVALID;
   *fill = h->fill;
+  return CPM_OK;
+}
+
+int cpm_running_fill(const cpm_handle* h, int* fill) {
+  if (!h || !fill) return CPM_ERR_INVALID;
+  if (uses_cluster(h))
+    *fill = CPM_FILL_CLUSTER;
+  else
+    *fill = h->fill_by == cpm_handle::kByCaller && h->fill != CPM_FILL_CLUSTER ? h->fill
+                                                                              : CPM_FILL_PARITY;
   return CPM_OK;
 }
 

@@ -214,6 +214,7 @@ def library():
         "cpm_set_dispatch": [H, ctypes.c_int],
         "cpm_set_fill": [H, ctypes.c_int],
         "cpm_get_fill": [H, ip],
+        "cpm_running_fill": [H, ip],
         "cpm_recount": [H],
         "cpm_set_centroid_sums_r": [H, ctypes.c_int, ctypes.c_void_p],
         "cpm_get_params_r": [H, ctypes.c_int, ctypes.POINTER(StaticParams)],
@@ -548,19 +549,21 @@ class _Engine:
 
     def sweep_config(self):
         """dict(variant, tile, warps_per_block, grid, dispatch, fill) of the
-        launch runs use."""
+        launch runs use; fill is "cluster" where they take the cluster sweep."""
         vals = [ctypes.c_int() for _ in range(7)]
         self._call("cpm_sweep_config", *[ctypes.byref(v) for v in vals])
+        f = ctypes.c_int()
+        self._call("cpm_running_fill", ctypes.byref(f))
         v, tx, ty, tz, w, g, d = (x.value for x in vals)
         return {"variant": v, "tile": (tx, ty, tz), "warps_per_block": w, "grid": g,
                 "dispatch": {DISPATCH_REPLICA: "replica",
                              DISPATCH_HYBRID: "hybrid"}.get(d, "grid"),
-                "fill": FILL_NAMES[self.fill]}
+                "fill": FILL_NAMES[f.value]}
 
     @property
     def fill(self):
-        """The sweep's kernel: FILL_CLUSTER, or FILL_PARITY, FILL_VECTOR or
-        FILL_TMA, which are one (see cpm_set_fill)."""
+        """The fill that was set, FILL_TMA or FILL_PARITY by the shape where
+        none was (see cpm_set_fill); sweep_config() tells which sweep runs."""
         f = ctypes.c_int()
         self._call("cpm_get_fill", ctypes.byref(f))
         return f.value

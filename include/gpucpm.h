@@ -334,9 +334,7 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
  *                    blocks holds the lattice and its tables in its shared
  *                    memory for a whole run, one strip of rows per block with
  *                    copies of its neighbours' edge rows, and the phases end
- *                    at a barrier inside the cluster.  Where lattice and
- *                    tables do not fit (about 400^2), runs take the other
- *                    sweep.
+ *                    at a barrier inside the cluster
  * Until a fill is set (or cpm_autotune picks one) plain runs of a 2D lattice
  * of up to 140,000 sites take the cluster sweep where it fits, all others the
  * sweep over the whole GPU; cpm_get_fill then reports CPM_FILL_TMA or
@@ -344,8 +342,13 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
  * sweep.
  * CPM_FILL_VECTOR and CPM_FILL_TMA need a single lattice with nx a multiple of
  * 4 and nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18), for which
- * CPM_FILL_TMA is reported; CPM_FILL_CLUSTER a 2D one of these with about
- * 190 KB of rows per block of a 16-block cluster at most.
+ * CPM_FILL_TMA is reported.  CPM_FILL_CLUSTER needs a 2D one that fits a
+ * cluster with its tables (up to about 400^2); it is also accepted, and the
+ * sweep over the whole GPU runs, for shapes that VECTOR and TMA accept and whose
+ * rows alone fit (about 190 KB of them per block of 16).
+ * cpm_running_fill tells which sweep plain runs take as things stand:
+ * CPM_FILL_CLUSTER, or for the sweep over the whole GPU the name that was set
+ * for it, CPM_FILL_PARITY where none was.
  * The result does not depend on the fill: it selects the kernel only
  * (CPM_ERR_UNSUPPORTED for a fill the lattice cannot use). */
 #define CPM_FILL_PARITY 0
@@ -354,6 +357,7 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
 #define CPM_FILL_CLUSTER 3
 int cpm_set_fill(cpm_handle* h, int fill);
 int cpm_get_fill(const cpm_handle* h, int* fill);
+int cpm_running_fill(const cpm_handle* h, int* fill);
 
 /* Replaces Cpm::synchronize (src/cpm.cu:653-655).  Waits for the handle's
  * stream and reports device-side errors (CPM_ERR_TIMEOUT, CPM_ERR_CUDA). */
