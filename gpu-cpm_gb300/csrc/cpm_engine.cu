@@ -1567,15 +1567,17 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
         pairs.emplace_back(v, d);
   // A lattice that one thread-block cluster can hold is also tried in the
   // cluster sweep (which has no tile variants), unless the caller chose the
-  // parity fill.
+  // parity fill.  Runs with the act or persistence term never take it: the fill
+  // stays as it is then, as after an error.
   const int row_fill = h->fill != CPM_FILL_CLUSTER ? h->fill
                        : h->row_ok                 ? CPM_FILL_TMA
                                                    : CPM_FILL_PARITY;
   const auto fill_by = h->fill_by;
+  const int fill = h->fill;
+  const bool try_cluster = h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
+                           (fill_by == cpm_handle::kBySize || fill != CPM_FILL_PARITY);
+  if (try_cluster) pairs.emplace_back(h->variant, -1);
   h->fill_by = cpm_handle::kByTuner;
-  if (h->cluster_blocks > 0 &&
-      (fill_by == cpm_handle::kBySize || h->fill != CPM_FILL_PARITY))
-    pairs.emplace_back(h->variant, -1);
   int best_fill = row_fill;
   const int npairs = (int)pairs.size();
   for (int i = 0; i < 3 * npairs && e == cudaSuccess; ++i) {
@@ -1602,9 +1604,8 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
       best_fill = h->fill;
     }
   }
-  h->fill = best_fill;
-  if (fill_by == cpm_handle::kBySize ? h->cluster_blocks == 0 : best_fill == row_fill)
-    h->fill_by = fill_by;
+  h->fill = fill;
+  h->fill_by = fill_by;
   if (e == cudaSuccess) e = copy(false);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   cudaFree(save);
@@ -1616,6 +1617,10 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   if (w) return h->fail(CPM_ERR_TIMEOUT, "autotune: %s", describe_errors(w).c_str());
   h->variant = best_v;
   h->dispatch = best_d;
+  if (try_cluster && (fill_by == cpm_handle::kBySize || best_fill != fill)) {
+    h->fill = best_fill;
+    h->fill_by = cpm_handle::kByTuner;
+  }
   h->tick = tick;
   if (chosen) *chosen = best_v;
   if (ms_per_mcs) *ms_per_mcs = best / (float)probe_mcs;

@@ -68,3 +68,39 @@ def test_act_runs_report_the_grid_sweep(engine_lib):
     e.run_mcs(2)
     assert e.sweep_config()["fill"] == "cluster"
     finish(e)
+
+
+def test_autotune_keeps_the_fill_that_it_did_not_time(engine_lib):
+    """The cluster sweep is no candidate of act runs, so tuning one decides
+    nothing about the runs after it."""
+    import gpucpm
+    w = W.random_small((64, 64), 40, ntypes=3, seed=3, temperature=9.0)
+    w.act_lambda = np.array([0, 10, 0, 0], np.float32)
+    w.act_max = np.array([0, 20, 0, 0], np.int32)
+    for fill in (None, gpucpm.FILL_CLUSTER):
+        e = make_engine(w, seed=8)
+        if fill is not None:
+            e.set_fill(fill)
+        before = e.fill
+        e.autotune(probe_mcs=2)
+        assert e.fill == before
+        e.set_act(0, 1, 0, 0.0)
+        e.run_mcs(2)
+        assert e.fill == before and e.sweep_config()["fill"] == "cluster"
+        finish(e)
+
+
+def test_autotune_keeps_the_fill_after_an_error(engine_lib):
+    """A site of an unknown cell, which the sweep reports and skips, ends the
+    tuning; variant and fill are as before it."""
+    import gpucpm
+    w = W.random_small((64, 64), 40, ntypes=3, seed=3, temperature=9.0)
+    e = make_engine(w, seed=8)
+    before, config = e.fill, e.sweep_config()
+    e.synchronize()
+    e.device_lattice(0)[10, 10] = w.ncells + 5 + (1 << 24)
+    import torch
+    torch.cuda.synchronize()
+    with pytest.raises(gpucpm.CpmError, match="autotune"):
+        e.autotune(probe_mcs=2)
+    assert e.fill == before and e.sweep_config() == config
