@@ -352,20 +352,10 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     ncy = class_count(ny, cy);
     tnx = (ncx + 31) >> 5;
     tny = (ncy + rows - 1) / rows;
-    inv_tnx = 0xFFFFFFFFu / (unsigned)tnx;
+    inv_tnx = task_reciprocal(tnx);
   };
-  // n / tnx and the remainder, n < 2^31: with inv = floor((2^32 - 1) / tnx),
-  // n * inv / 2^32 lies in (n / tnx - 1/2, n / tnx], so the product's high word
-  // is the quotient or one less.  (Two divisions per task were part of what
-  // made tasks of 4 rows no better than ones of 8: 4096^2, 50 MCS 7.09 -> 7.05.)
   auto by_tnx = [&](const unsigned n, unsigned& rem) {
-    unsigned q = __umulhi(n, inv_tnx);
-    rem = n - q * (unsigned)tnx;
-    if (rem >= (unsigned)tnx) {
-      rem -= (unsigned)tnx;
-      ++q;
-    }
-    return q;
+    return task_quotient(n, (unsigned)tnx, inv_tnx, rem);
   };
   auto place = [&](const int local) {  // task `local` of the lattice
     unsigned tx, turn;
