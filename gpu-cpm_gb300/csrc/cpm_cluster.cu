@@ -357,7 +357,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       }
       const int dp = side ? 2 * cnt - 8 : 8 - 2 * cnt;
       float qp, qa, ex;
-      constraint_terms(ap.x, ap.y, dp, side ? -1 : 1, tp, s_ctx.small_targets != 0, qp, qa);
+      if (s_ctx.small_targets && (unsigned)(ap.x | ap.y) < kSmallTable)
+        constraint_terms_small(ap.x, ap.y, dp, side ? -1 : 1, tp, qp, qa);
+      else
+        constraint_terms_wide(ap.x, ap.y, dp, side ? -1 : 1, tp, qp, qa);
       const float dH = pair_energy(mask, side, s != 0, t != 0, en, chemo, qp, qa, tp,
                                    s_ctx.perim_on != 0);
       if (metropolis(dH, s_ctx.T, e.y, ex)) {

@@ -136,18 +136,20 @@ constexpr int kJPitch = 37;
 // The integers that the constraints multiply: dp (2 (P - P*) + dp) for a
 // perimeter that changes by dp, 1 +- 2 (A - A*) for an area that changes by
 // +-1 (`sign`), each rounded once to FP32.  Where the tables and targets are
-// below 2^21 (`small` tells of the targets) all factors are exact in FP32 and
-// so is the rounding of their product; otherwise in 64 bits.
-__device__ __forceinline__ void constraint_terms(int area, int perim, int dp, int sign,
-                                                 const TypeParams& p, bool small, float& qp,
-                                                 float& qa) {
-  if (small && (unsigned)(area | perim) < (1u << 21)) {
-    qp = __fmul_rn((float)dp, (float)(2 * (perim - p.tgt_perim) + dp));
-    qa = (float)(1 + sign * 2 * (area - p.tgt_area));
-  } else {
-    qp = __ll2float_rn((long long)dp * (2LL * ((long long)perim - p.tgt_perim) + dp));
-    qa = __ll2float_rn(1 + sign * 2LL * ((long long)area - p.tgt_area));
-  }
+// below 2^21 (kSmallTable) all factors are exact in FP32 and so is the rounding
+// of their product; otherwise in 64 bits.
+constexpr unsigned kSmallTable = 1u << 21;
+__device__ __forceinline__ void constraint_terms_small(int area, int perim, int dp, int sign,
+                                                       const TypeParams& p, float& qp,
+                                                       float& qa) {
+  qp = __fmul_rn((float)dp, (float)(2 * (perim - p.tgt_perim) + dp));
+  qa = (float)(1 + sign * 2 * (area - p.tgt_area));
+}
+__device__ __forceinline__ void constraint_terms_wide(int area, int perim, int dp, int sign,
+                                                      const TypeParams& p, float& qp,
+                                                      float& qa) {
+  qp = __ll2float_rn((long long)dp * (2LL * ((long long)perim - p.tgt_perim) + dp));
+  qa = __ll2float_rn(1 + sign * 2LL * ((long long)area - p.tgt_area));
 }
 
 // Metropolis test.  `draw`: the attempt's random word; ex receives
