@@ -121,8 +121,8 @@ struct cpm_handle {
   std::vector<double> h_field;
   float* d_field = nullptr;
   // act model (allocated on first use): MCS of the last copy into each site;
-  // (on the first act run) second copies of lattice and stamps, and the
-  // blocks' lists of the copies of two phases (SweepArgs::lat2, act2, pend)
+  // (on the first act run) second copies of lattice and stamps, where they fit,
+  // and the blocks' lists of a phase's copies (SweepArgs::lat2, act2, pend)
   std::vector<uint32_t> h_act;
   uint32_t* d_act = nullptr;
   uint32_t* d_lat2 = nullptr;
@@ -528,7 +528,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     }
   }
   // act runs list one copy per attempt at most, half of a dirty list's
-  // entries, in two lists per block
+  // entries, in two lists per block (one where there is one lattice copy)
   h->pend_entries = pend_entries;
   e = cudaMalloc((void**)&h->d_dlist, sizeof(uint32_t) * dlist_entries);
   if (e != cudaSuccess) {
@@ -731,13 +731,25 @@ int ensure_act(cpm_handle* h) {
   return CPM_OK;
 }
 
-// The act run's second lattice and stamp copies and its lists.
+// The act run's second lattice and stamp copies and its lists; where these do
+// not fit, the lists of a run with one copy alone.
 int ensure_act_run(cpm_handle* h) {
   if (int rc = ensure_act(h)) return rc;
+  if (h->d_pend) return CPM_OK;
   const size_t b = sizeof(uint32_t) * (h->total_sites ? h->total_sites : 1);
-  if (!h->d_lat2) CPM_CUDA(h, cudaMalloc((void**)&h->d_lat2, b));
-  if (!h->d_act2) CPM_CUDA(h, cudaMalloc((void**)&h->d_act2, b));
-  if (!h->d_pend) CPM_CUDA(h, cudaMalloc((void**)&h->d_pend, sizeof(uint4) * h->pend_entries));
+  cudaError_t e = cudaMalloc((void**)&h->d_lat2, b);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_act2, b);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_pend, sizeof(uint4) * h->pend_entries);
+  if (e == cudaSuccess) return CPM_OK;
+  cudaFree(h->d_lat2);
+  cudaFree(h->d_act2);
+  h->d_lat2 = h->d_act2 = nullptr;
+  h->d_pend = nullptr;
+  if (e != cudaErrorMemoryAllocation) return h->cuda_fail(e, "allocation of the act run's copies");
+  cudaGetLastError();  // (not an error of the run)
+  const size_t entries = (size_t)(h->pend_entries + 1) / 2;
+  CPM_CUDA(h, cudaMalloc((void**)&h->d_pend,
+                         (sizeof(unsigned long long) + sizeof(uint32_t)) * entries));
   return CPM_OK;
 }
 
@@ -909,7 +921,7 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
                           int* nlaunch) {
   const cpm_handle::Config& c = h->cfg[v];
   *nlaunch = 0;
-  if (h->act_active) {  // both lattice and stamp copies start equal
+  if (h->act_active && h->d_lat2) {  // both lattice and stamp copies start equal
     const size_t b = sizeof(uint32_t) * h->total_sites;
     cudaError_t e = cudaMemcpyAsync(h->d_lat2, h->d_lat, b, cudaMemcpyDeviceToDevice, h->stream);
     if (e == cudaSuccess)

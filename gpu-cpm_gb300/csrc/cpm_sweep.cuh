@@ -61,6 +61,7 @@ namespace {
 constexpr int kPlain = 0;
 constexpr int kExt = 1;    // act, 3D persistence
 constexpr int kScore = 2;  // likelihood-ratio scores (2D)
+constexpr int kOne = 3;    // kExt with one lattice copy (SweepArgs::lat2 is null)
 
 // Warps per block (one block per SM): 24 at 80 registers for the plain 2D
 // sweep, 20 at 96 for the others, which would spill at 80.  (28 or 32 warps at
@@ -172,11 +173,22 @@ __device__ __forceinline__ void flush_scores(const SweepArgs& a, float* sc, int 
   for (int k = 0; k < kScoreRegs; ++k) sc[k] = 0.0f;
 }
 
+// Entry j of the block's list of the running phase's copies in act runs with
+// one lattice (SweepArgs::pend).
+__device__ __forceinline__ unsigned long long& pend_site(const SweepArgs& a, unsigned j) {
+  return reinterpret_cast<unsigned long long*>(a.pend)[(long long)blockIdx.x * a.pend_cap + j];
+}
+__device__ __forceinline__ uint32_t& pend_value(const SweepArgs& a, unsigned j) {
+  return reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned long long*>(a.pend) +
+                                     (long long)gridDim.x * a.pend_cap)
+      [(long long)blockIdx.x * a.pend_cap + j];
+}
+
 // LOCAL: for replica dispatch, where the kernel differs (see s_pt).
 template <int NDIM, int KR, int MODE, bool BATCH, bool LOCAL>
 __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1)
     sweep_kernel(const __grid_constant__ SweepArgs a) {
-  constexpr bool EXT = MODE == kExt, SCORE = MODE == kScore;
+  constexpr bool ONE = MODE == kOne, EXT = MODE == kExt || ONE, SCORE = MODE == kScore;
   constexpr int NB = NDIM == 2 ? 8 : 26, NBC = NB + 1;
   constexpr int QLEN = queue_len<KR>();
   constexpr bool DEFER = defers<NDIM, KR, MODE, BATCH>();
@@ -313,7 +325,7 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           if (d[k]) atomicAdd(cs + row * NDIM + k, d[k]);
       }
     }
-    if (EXT && a.act_on) {
+    if (EXT && !ONE && a.act_on) {
       // the copies went into the other lattice copy when they were made;
       // sites of different phases differ, so this phase's writes commute
       const unsigned np = min(s_pend[prv], (unsigned)a.pend_cap);
@@ -478,12 +490,12 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
     if constexpr (!SHARED_PT) held = tables_of(cur);
     const PhaseTables<NDIM>& pt = SHARED_PT ? s_pt[cur] : held;
     // the lattice (act stamps) the phase reads, and the one it writes:
-    // another copy in act runs
-    const bool two = EXT && a.act_on;
+    // another copy in act runs that have one
+    const bool two = EXT && !ONE && a.act_on;
     const uint32_t* const lat_r = two && cur ? a.lat2 : a.lat;
     uint32_t* const lat_w = two && !cur ? a.lat2 : a.lat;
-    const uint32_t* const act_r = cur ? a.act2 : a.act;
-    uint32_t* const act_w = cur ? a.act : a.act2;
+    const uint32_t* const act_r = !ONE && cur ? a.act2 : a.act;
+    uint32_t* const act_w = cur ? a.act : a.act2;  // (not in ONE)
 
     // Changed rows (0xFFFFFFFF: none) of the lanes onto the block's dirty list:
     // one shared-memory atomic per batch.
@@ -741,14 +753,19 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
           }
           if (ok) {
             accepted = true;
-            lat_w[ctx.lat_off + site] = s;
-            if (EXT && a.act_on) {  // into this copy in the next phase
-              act_w[ctx.lat_off + site] = (uint32_t)tick;
+            if constexpr (!ONE) lat_w[ctx.lat_off + site] = s;
+            if (EXT && a.act_on) {  // into this copy in the next phase (ONE: after this one)
+              if constexpr (!ONE) act_w[ctx.lat_off + site] = (uint32_t)tick;
               const unsigned j = atomicAdd(&s_pend[cur], 1u);
               if ((long long)j < a.pend_cap) {
                 const unsigned long long g = (unsigned long long)ctx.lat_off + site;
-                a.pend[(2LL * blockIdx.x + cur) * a.pend_cap + j] =
-                    make_uint4((uint32_t)g, (uint32_t)(g >> 32), s, (uint32_t)tick);
+                if constexpr (ONE) {
+                  pend_site(a, j) = g;
+                  pend_value(a, j) = s;
+                } else {
+                  a.pend[(2LL * blockIdx.x + cur) * a.pend_cap + j] =
+                      make_uint4((uint32_t)g, (uint32_t)(g >> 32), s, (uint32_t)tick);
+                }
               } else {
                 atomicOr(err, kErrListFull);  // reported, never written past the end
               }
@@ -996,6 +1013,17 @@ __global__ void __launch_bounds__((32 * sweep_warps<NDIM, KR, MODE, BATCH>()), 1
         if (step > 0) replay_phase(prv, blockDim.x - 1 - tid);
         run_phase(a.slots[si], tick, step, b, G);
         __syncthreads();
+        if constexpr (ONE) {
+          // the phase's copies are made when all its attempts are
+          if (!local && !grid_barrier(a.ctl, ++episode, &s_ok)) return;
+          const unsigned np = min(s_pend[step & 1], (unsigned)a.pend_cap);
+          for (unsigned j = tid; j < np; j += blockDim.x) {
+            const unsigned long long site = pend_site(a, j);
+            a.lat[site] = pend_value(a, j);
+            a.act[site] = (uint32_t)tick;
+          }
+          __syncthreads();
+        }
         if (tid == 0) {
           s_cnt[prv] = s_pend[prv] = 0;
           s_pool = 0;
@@ -1053,8 +1081,9 @@ cudaError_t launch_sweep_as(const SweepArgs& a, int grid, int warps, cudaStream_
 template <int NDIM>
 cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int grid, int warps,
                             cudaStream_t s) {
-  const bool ext = a.act_on || a.prefdir;
+  const bool ext = a.act_on || a.prefdir, one = a.act_on && !a.lat2;
   if (batch) {
+    if (one) return launch_sweep_as<NDIM, 2, kOne, true>(a, grid, warps, s);
     if (ext) return launch_sweep_as<NDIM, 2, kExt, true>(a, grid, warps, s);
     if constexpr (NDIM == 2) {
       if (scores)
@@ -1064,6 +1093,7 @@ cudaError_t launch_sweep_nd(const SweepArgs& a, bool batch, bool scores, int gri
     return a.kr == 4 ? launch_sweep_as<NDIM, 4, kPlain, true>(a, grid, warps, s)
                      : launch_sweep_as<NDIM, 2, kPlain, true>(a, grid, warps, s);
   }
+  if (one) return launch_sweep_as<NDIM, 2, kOne, false>(a, grid, warps, s);
   if (ext) return launch_sweep_as<NDIM, 2, kExt, false>(a, grid, warps, s);
   if constexpr (NDIM == 2) {
     if (scores) return launch_sweep_as<NDIM, 2, kScore, false>(a, grid, warps, s);

@@ -121,8 +121,9 @@ int cpm_set_adhesion_r(cpm_handle* h, int replica, int type, int other,
  * cell (0 for the medium), act being the MCS of the last copy into a site;
  * here computed as exp2 of the mean log2 with this library's own FP32 log2 /
  * exp2.  Runs with an act lambda keep two copies of lattice and
- * stamps, so that every attempt reads the phase's starting state; they cannot
- * accumulate scores. */
+ * stamps, so that every attempt reads the phase's starting state, or, where the
+ * second ones do not fit in memory on the first such run, make a phase's copies
+ * at its end (the same results); they cannot accumulate scores. */
 int cpm_set_act(cpm_handle* h, int type, int max_act, float lambda);
 int cpm_set_act_r(cpm_handle* h, int replica, int type, int max_act, float lambda);
 
