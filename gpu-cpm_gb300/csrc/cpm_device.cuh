@@ -140,11 +140,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   return v;
 }
 
-__device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v)
-               : "memory");
-}
-
 // Grid-wide barrier of a cooperative launch (all blocks co-resident).  The
 // arrival counter ctl[kCtlBarrier] is zeroed before the launch and only
 // grows.  At the e-th barrier (e = 1, 2, ...) each block adds 1 to it with a

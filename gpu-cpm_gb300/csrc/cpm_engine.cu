@@ -403,8 +403,10 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
   al((void**)&h->d_reps, sizeof(DevReplica) * n);
   al((void**)&h->d_params, sizeof(DevParams));
   h->params_cap = 1;
-  al((void**)&h->d_task_prefix, sizeof(int) * kTileVariants * 27 * (n + 1));
-  al((void**)&h->d_hyb_prefix, sizeof(int) * kTileVariants * 27 * (n + 1));
+  if (n > 1) {
+    al((void**)&h->d_task_prefix, sizeof(int) * kTileVariants * 27 * (n + 1));
+    al((void**)&h->d_hyb_prefix, sizeof(int) * kTileVariants * 27 * (n + 1));
+  }
   al((void**)&h->d_rep_order, sizeof(int) * n);
   al((void**)&h->d_tick, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&h->h_lat, sizeof(uint32_t) * (sites ? sites : 1));
@@ -472,12 +474,13 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
       pend_entries = std::max(pend_entries, c.wide.list_cap * c.wide.grid);
     }
     const int rows = n == 1 ? c.plan.rows : batch_rows(v, total_units, sms);
-    c.task_prefix.assign(27 * (n + 1), 0);
+    if (n > 1) c.task_prefix.assign(27 * (n + 1), 0);
     long long max_tasks = 1;
     for (int slot = 0; slot < 27; ++slot) {
       long long acc = 0;
       for (int r = 0; r < n; ++r) {
-        c.task_prefix[slot * (n + 1) + r] = (int)std::min<long long>(acc, INT32_MAX);
+        if (n > 1)
+          c.task_prefix[slot * (n + 1) + r] = (int)std::min<long long>(acc, INT32_MAX);
         acc += units(r, slot, rows);
       }
       if (acc >= (1LL << 31)) {
@@ -486,7 +489,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
         delete h;
         return CPM_ERR_INVALID;
       }
-      c.task_prefix[slot * (n + 1) + n] = (int)acc;
+      if (n > 1) c.task_prefix[slot * (n + 1) + n] = (int)acc;
       if (acc > 0) c.active_slots.push_back(slot);
       max_tasks = std::max(max_tasks, acc);
     }
@@ -512,6 +515,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
         pend_entries = std::max(pend_entries, p.list_cap * p.grid);
       }
     }
+    if (n == 1) continue;
     // Hybrid split: replica dispatch gets whole rounds of the smallest
     // replicas, grid dispatch the rest.
     c.hyb_ng = n - (n / c.local.grid) * c.local.grid;
@@ -551,7 +555,7 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(h->d_rep_order, order.data(), sizeof(int) * n,
                         cudaMemcpyHostToDevice, h->stream);
-  for (int v = 0; v < kTileVariants && e == cudaSuccess; ++v) {
+  for (int v = 0; n > 1 && v < kTileVariants && e == cudaSuccess; ++v) {
     e = cudaMemcpyAsync(h->d_task_prefix + (size_t)v * 27 * (n + 1),
                         h->cfg[v].task_prefix.data(), sizeof(int) * 27 * (n + 1),
                         cudaMemcpyHostToDevice, h->stream);
@@ -881,7 +885,7 @@ SweepArgs sweep_args(const cpm_handle* h, int v) {
   a.counters = h->d_counters;
   a.reps = h->d_reps;
   a.params = h->d_params;
-  a.task_prefix = h->d_task_prefix + (size_t)v * 27 * (h->nrep + 1);
+  if (h->nrep > 1) a.task_prefix = h->d_task_prefix + (size_t)v * 27 * (h->nrep + 1);
   a.seed = h->seed;
   a.nrep = h->nrep;
   a.stream0 = h->stream_id;
@@ -1462,8 +1466,8 @@ int cpm_run(cpm_handle* h, int mcs) {
     const int chunk = std::min(left, kMaxMcsPerLaunch);
     a.tick0 = h->tick;
     a.mcs = chunk;
-    // Barrier counter and release flag start at zero in every launch; the
-    // sticky error word is left alone until cpm_synchronize reads it.
+    // The barrier counter starts at zero in every launch; the sticky error
+    // word is left alone until cpm_synchronize reads it.
     int nl = 0;
     CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, false, &nl));
     h->launches += nl;

@@ -53,8 +53,7 @@ constexpr size_t kOffCtl = kOffList + align256(4 * kListEntries);
 constexpr size_t kOffCounters = kOffCtl + align256(4 * kCtlWords);
 constexpr size_t kOffRep = kOffCounters + align256(16);
 constexpr size_t kOffParams = kOffRep + align256(sizeof(DevReplica));
-constexpr size_t kOffPrefix = kOffParams + align256(sizeof(DevParams));
-constexpr size_t kWorkBytes = kOffPrefix + align256(4 * 27 * 2);
+constexpr size_t kWorkBytes = kOffParams + align256(sizeof(DevParams));
 
 static __device__ __align__(256) unsigned char g_work[kWorkBytes];
 
@@ -191,7 +190,8 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
   // Dirty-list space of one block and phase: two table rows per target of
   // the tasks it is dealt (narrow lattices do not pay for empty columns).
   // Over every shape within CPM_STATIC_MAX_SITES the lists of a launch need
-  // at most 544,768 entries in 2D and 272,384 in 3D on 152 SMs, within kListEntries.
+  // at most 525,312 entries in 2D (66 x 3650) and 272,384 in 3D (66 x 4 x 990)
+  // on 152 SMs, within kListEntries.
   const SweepPlan plan = plan_sweep(ndim, nx, ny, nz, 0, sms, false);
   if (plan.list_cap * 2 * plan.grid > kListEntries)
     return fail(CPM_ERR_INVALID,

@@ -29,8 +29,8 @@ __device__ __forceinline__ int wrap_coord(int v, int n) {
   return v < 0 ? v + n : (v >= n ? v - n : v);
 }
 
-// Coordinates of the source of an attempt: neighbour `kdir` (the order of
-// Stage::nb_offset) of the target (x, y, z), wrapped.
+// Coordinates of the source of an attempt: neighbour `kdir` (in (dz, dy, dx)
+// order, the target itself left out) of the target (x, y, z), wrapped.
 template <int NDIM>
 __device__ __forceinline__ void source_coords(int kdir, int x, int y, int z, int nx, int ny,
                                               int nz, int& sx, int& sy, int& sz) {
