@@ -195,7 +195,7 @@ struct cpm_handle {
 
   // Scratch of the synchronous seeding and measuring calls, grown on demand
   // and freed with the handle (an allocation per call costs more than their
-  // kernels on small lattices).
+  // kernels on small lattices), or at once where it is large (kScratchKept).
   char* d_scratch = nullptr;
   size_t scratch_cap = 0;
 
@@ -670,7 +670,7 @@ int set_adhesion(cpm_handle* h, int r, int type, int other, float J, int sym) {
 }
 
 // At least `bytes` of scratch at h->d_scratch.  Its users wait for the stream
-// before they return, so nothing in flight holds the old one.
+// before they return, so nothing in flight holds the old one, and trim it then.
 int ensure_scratch(cpm_handle* h, size_t bytes) {
   if (bytes <= h->scratch_cap) return CPM_OK;
   cudaFree(h->d_scratch);
@@ -679,6 +679,17 @@ int ensure_scratch(cpm_handle* h, size_t bytes) {
   CPM_CUDA(h, cudaMalloc((void**)&h->d_scratch, bytes));
   h->scratch_cap = bytes;
   return CPM_OK;
+}
+
+// Gives back scratch that is large enough to be missed (256 MB: the points of a
+// seeding from 4 million, calls in which the allocation does not show: 4096^2
+// sites from 4.4 million points 53.7 ms, with the scratch kept 54.7).
+constexpr size_t kScratchKept = (size_t)256 << 20;
+void trim_scratch(cpm_handle* h) {
+  if (h->scratch_cap <= kScratchKept) return;
+  cudaFree(h->d_scratch);
+  h->d_scratch = nullptr;
+  h->scratch_cap = 0;
 }
 
 int read_error_word(cpm_handle* h, uint32_t* word) {
@@ -1716,6 +1727,7 @@ int cpm_observe_heterotypic(cpm_handle* h, float* out_host) {
     e = cudaMemcpyAsync(c.data(), counts, counts_b, cudaMemcpyDeviceToHost, h->stream);
   // (also on an error: the copies read and write this frame's vectors)
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
+  trim_scratch(h);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_observe_heterotypic");
   for (int r = 0; r < h->nrep; ++r)
@@ -1854,6 +1866,7 @@ int cpm_seed_voronoi_r(cpm_handle* h, int r, int npoints, const double* points,
   h->launches += 2;
   // the host buffers are read by the copies: wait before they go
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
+  trim_scratch(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_seed_voronoi_r");
   if (e2 != cudaSuccess) return h->cuda_fail(e2, "cpm_seed_voronoi_r");
   h->pushed = false;  // the tables no longer describe the lattice
@@ -1887,6 +1900,7 @@ int cpm_observe_boundaries(cpm_handle* h, int ntypes, uint64_t* out_host) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out_host, counts, counts_b, cudaMemcpyDeviceToHost, h->stream);
   const cudaError_t e2 = cudaStreamSynchronize(h->stream);
+  trim_scratch(h);
   if (e != cudaSuccess) return h->cuda_fail(e, "cpm_observe_boundaries");
   if (e2 != cudaSuccess) return h->cuda_fail(e2, "cpm_observe_boundaries");
   return CPM_OK;
