@@ -917,9 +917,13 @@ int grid_of(const cpm_handle* h, int v, int d) { return plan_of(h, v, d).grid; }
 int fill_key(const cpm_handle* h) { return h->fill_by == cpm_handle::kBySize ? -2 : h->fill; }
 
 // Whether plain runs take the cluster sweep.
-// By itself up to the size where the grid sweep, whose phases take 4.8 us
-// whatever the size, overtakes its 16 SMs (us per MCS, grid / cluster: 350^2
-// 19.5 / 16.7, 400^2 19.2 / 20.4).
+// By itself up to about the size where the grid sweep, whose phases take 4.6 us
+// whatever the size, overtakes its 16 SMs.  The line is that of the sorting
+// lattice (us per MCS, grid / cluster: 350^2 19.5 / 16.7, 400^2 19.2 / 20.4).
+// Dense tissues cross it earlier, and long lattices, whose rows or columns do
+// not divide evenly over 16 blocks, here and there (tissue of 50 sites a cell:
+// 330^2 18.6 / 19.9, 4000 x 16 18.3 / 20.4, 100 x 1300 18.7 / 21.0, but 16 x 4000
+// 18.0 / 11.8, 2000 x 32 18.4 / 12.4, 4095 x 5 32.2 / 26.1).
 constexpr long long kClusterAutoSites = 140000;
 bool uses_cluster(const cpm_handle* h) {
   return h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
