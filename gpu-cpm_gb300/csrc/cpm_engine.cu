@@ -88,13 +88,13 @@ SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int 
 // scores 8 rows 24.1, 4 rows 28.1, 16 rows 28.0; 256 ragged replicas 16 rows
 // 16.4, 8 rows 19.0; 64 x 64^2 2 rows 0.52, 4 rows 0.59.
 int gpucpm::batch_rows(int variant, long long total_units, int sms) {
+  const long long per_warp = total_units / ((long long)sms * kWarpsWide);
   switch (variant) {
     case 1: return 8;
     case 2: return 32;
     case 3: return 2;
     default: break;
   }
-  const long long per_warp = total_units / ((long long)sms * kWarpsWide);
   return per_warp >= 32 ? 16 : (per_warp >= 8 ? 8 : (per_warp >= 4 ? 4 : 2));
 }
 
@@ -170,6 +170,7 @@ struct cpm_handle {
     std::vector<int> hyb_prefix;
   } cfg[kTileVariants];
   int variant = 0;
+  bool variant_ext = false;  // the autotuner's choice for act or persistence runs
   int dispatch = CPM_DISPATCH_GRID;  // CPM_DISPATCH_*
   // CPM_FILL_*, as cpm_get_fill tells it.  Until the caller or the autotuner
   // chooses one (fill_by) the engine runs the cluster sweep (cpm_cluster.cu) on
@@ -863,6 +864,14 @@ int upload_params(cpm_handle* h) {
 // come, whose rows the lists never see.
 bool scans(const cpm_handle* h) { return 8 * h->rows <= h->total_sites; }
 
+// The variant that runs use.  A caller's choice is one for plain runs and
+// scores: runs with the act or persistence term take variant 0, or what the
+// autotuner timed on such runs (160 small replicas with act, 8 MCS: 0.84 ms, in
+// variant 2 3.80).
+int run_variant(const cpm_handle* h) {
+  return (h->act_active || h->persist_active) && !h->variant_ext ? 0 : h->variant;
+}
+
 // Kernel arguments of a sweep with tile variant v and dispatch d (tick0 /
 // mcs, and what depends on the launch, filled in by the caller).
 SweepArgs sweep_args(const cpm_handle* h, int v) {
@@ -1475,7 +1484,7 @@ int cpm_run(cpm_handle* h, int mcs) {
   if (!h->pushed) return h->fail(CPM_ERR_STATE, "run() before a successful push_to_gpu()");
   if (mcs == 0) return CPM_OK;
   if (int rc = upload_params(h)) return rc;
-  SweepArgs a = sweep_args(h, h->variant);
+  SweepArgs a = sweep_args(h, run_variant(h));
   int left = mcs;
   while (left > 0) {
     const int chunk = std::min(left, kMaxMcsPerLaunch);
@@ -1484,7 +1493,7 @@ int cpm_run(cpm_handle* h, int mcs) {
     // The barrier counter starts at zero in every launch; the sticky error
     // word is left alone until cpm_synchronize reads it.
     int nl = 0;
-    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, false, &nl));
+    CPM_CUDA(h, enqueue_sweep(h, run_variant(h), h->dispatch, a, false, &nl));
     h->launches += nl;
     h->tick += (uint64_t)chunk;
     left -= chunk;
@@ -1502,7 +1511,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
   if (h->stream == nullptr)
     return h->fail(CPM_ERR_STATE, "graph runs need a non-default stream");
   if (int rc = upload_params(h)) return rc;
-  if (!h->graph_exec || h->graph_mcs != mcs || h->graph_variant != h->variant ||
+  if (!h->graph_exec || h->graph_mcs != mcs || h->graph_variant != run_variant(h) ||
       h->graph_dispatch != h->dispatch || h->graph_fill != fill_key(h) ||
       h->graph_stream != h->stream) {
     if (h->graph_exec) {
@@ -1511,13 +1520,13 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     }
     // Capture: reset the barrier words, then the persistent sweep reading
     // its start time from (and advancing) the device tick.
-    SweepArgs a = sweep_args(h, h->variant);
+    SweepArgs a = sweep_args(h, run_variant(h));
     a.tick_ptr = h->d_tick;
     a.mcs = mcs;
     cudaGraph_t g = nullptr;
     CPM_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int nl = 0;
-    cudaError_t e2 = enqueue_sweep(h, h->variant, h->dispatch, a, false, &nl);
+    cudaError_t e2 = enqueue_sweep(h, run_variant(h), h->dispatch, a, false, &nl);
     cudaError_t e3 = cudaStreamEndCapture(h->stream, &g);
     if (e2 != cudaSuccess) return h->cuda_fail(e2, "capture of the sweep launch");
     if (e3 != cudaSuccess) return h->cuda_fail(e3, "cudaStreamEndCapture");
@@ -1526,7 +1535,7 @@ int cpm_run_graph(cpm_handle* h, int mcs) {
     if (e4 != cudaSuccess) return h->cuda_fail(e4, "cudaGraphInstantiate");
     h->graph_mcs = mcs;
     h->graph_launches = nl;
-    h->graph_variant = h->variant;
+    h->graph_variant = run_variant(h);
     h->graph_dispatch = h->dispatch;
     h->graph_fill = fill_key(h);
     h->graph_stream = h->stream;
@@ -1586,7 +1595,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   if (e == cudaSuccess) e = copy(true);
   const uint64_t tick = h->tick;
   float best = -1.0f;
-  int best_v = h->variant, best_d = h->dispatch;
+  int best_v = run_variant(h), best_d = h->dispatch;
   // Every (tile variant, dispatch) pair, replica dispatch only for batches,
   // timed in three rounds (the fastest run counts): a variant's first launch
   // also loads its module, and clocks may still be rising.
@@ -1607,7 +1616,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   const int fill = h->fill;
   const bool try_cluster = h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
                            (fill_by == cpm_handle::kBySize || fill != CPM_FILL_PARITY);
-  if (try_cluster) pairs.emplace_back(h->variant, -1);
+  if (try_cluster) pairs.emplace_back(run_variant(h), -1);
   h->fill_by = cpm_handle::kByTuner;
   int best_fill = row_fill;
   const int npairs = (int)pairs.size();
@@ -1647,6 +1656,7 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   if (int rc = read_error_word(h, &w)) return rc;
   if (w) return h->fail(CPM_ERR_TIMEOUT, "autotune: %s", describe_errors(w).c_str());
   h->variant = best_v;
+  h->variant_ext = h->act_active || h->persist_active;
   h->dispatch = best_d;
   if (try_cluster && (fill_by == cpm_handle::kBySize || best_fill != fill)) {
     h->fill = best_fill;
@@ -1683,7 +1693,7 @@ int cpm_run_scores(cpm_handle* h, int mcs, float* d_scores, uint64_t score_base,
   if (h->act_active || h->persist_active)
     return h->fail(CPM_ERR_UNSUPPORTED, "cpm_run_scores: scores of runs with the act or "
                                         "persistence term are not supported");
-  SweepArgs a = sweep_args(h, h->variant);
+  SweepArgs a = sweep_args(h, run_variant(h));
   a.scores = d_scores;
   a.score_base = score_base;
   a.score_len = score_len;
@@ -1694,7 +1704,7 @@ int cpm_run_scores(cpm_handle* h, int mcs, float* d_scores, uint64_t score_base,
     a.tick0 = h->tick;
     a.mcs = chunk;
     int nl = 0;
-    CPM_CUDA(h, enqueue_sweep(h, h->variant, h->dispatch, a, true, &nl));
+    CPM_CUDA(h, enqueue_sweep(h, run_variant(h), h->dispatch, a, true, &nl));
     h->launches += nl;
     h->tick += (uint64_t)chunk;
     left -= chunk;
@@ -1934,6 +1944,7 @@ int cpm_set_variant(cpm_handle* h, int variant) {
   if (variant < 0 || variant >= kTileVariants)
     return h->fail(CPM_ERR_INVALID, "tile variant %d out of range [0, %d)", variant, kTileVariants);
   h->variant = variant;
+  h->variant_ext = false;
   return CPM_OK;
 }
 
@@ -2119,7 +2130,7 @@ int cpm_info(const cpm_handle* h, int* n_replicas, int* dimensionality,
   if (n_replicas) *n_replicas = h->nrep;
   if (dimensionality) *dimensionality = h->ndim;
   if (sweep_grid)
-    *sweep_grid = uses_cluster(h) ? h->cluster_blocks : grid_of(h, h->variant, h->dispatch);
+    *sweep_grid = uses_cluster(h) ? h->cluster_blocks : grid_of(h, run_variant(h), h->dispatch);
   if (kernel_launches) *kernel_launches = h->launches;
   return CPM_OK;
 }
@@ -2128,12 +2139,12 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x, int* tile_y
                      int* tile_z, int* warps_per_block, int* grid, int* dispatch) {
   if (!h) return CPM_ERR_INVALID;
   if (variant) *variant = h->variant;
-  const SweepPlan& p = plan_of(h, h->variant, h->dispatch);
+  const SweepPlan& p = plan_of(h, run_variant(h), h->dispatch);
   if (tile_x) *tile_x = 32;
   if (tile_y) *tile_y = p.rows;
   if (tile_z) *tile_z = 1;
   if (warps_per_block) *warps_per_block = p.warps;
-  if (grid) *grid = grid_of(h, h->variant, h->dispatch);
+  if (grid) *grid = p.grid;
   if (dispatch) *dispatch = h->dispatch;
   if (uses_cluster(h)) {  // one cluster, targets dealt one per lane
     if (tile_y) *tile_y = 1;

@@ -317,7 +317,8 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs);
 
 /* Select a variant (0: rows per warp task from the size, 1 to 3: fixed) or a
  * dispatch explicitly / describe the current launch: extent of a warp's task
- * in targets, warps per block, grid size and dispatch. */
+ * in targets, warps per block, grid size and dispatch.  Runs with the act or
+ * persistence term use variant 0, or the autotuner's choice for them. */
 int cpm_set_variant(cpm_handle* h, int variant);
 int cpm_set_dispatch(cpm_handle* h, int dispatch);
 int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
