@@ -63,7 +63,7 @@ SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int 
   SweepPlan p;
   switch (variant) {
     case 1: p.kr = 4, p.rows = 8; break;
-    case 2: p.kr = 4, p.rows = 16; break;
+    case 2: p.kr = 4, p.rows = units >= 16LL * sms ? 16 : 8; break;  // (a task per block)
     case 3: p.kr = 1, p.rows = 1; break;
     default:
       p.kr = upb <= W ? 1 : (upb <= 3 * W ? 3 : 4);
@@ -86,12 +86,14 @@ SweepPlan gpucpm::plan_sweep(int ndim, int nx, int ny, int nz, int variant, int 
 // replicas took 3 % longer, their constants no longer being the warp's); small
 // batches need every warp to get a task.  Measured (ms): 128 x 256^2 with
 // scores 8 rows 24.1, 4 rows 28.1, 16 rows 28.0; 256 ragged replicas 16 rows
-// 16.4, 8 rows 19.0; 64 x 64^2 2 rows 0.52, 4 rows 0.59.
+// 16.4, 8 rows 19.0; 64 x 64^2 2 rows 0.52, 4 rows 0.59.  The 32 rows of variant 2
+// likewise only where every warp gets a task of them (two small 3D replicas, 8
+// MCS: 32 rows 3.98 ms, 16 2.67, 8 2.04).
 int gpucpm::batch_rows(int variant, long long total_units, int sms) {
   const long long per_warp = total_units / ((long long)sms * kWarpsWide);
   switch (variant) {
     case 1: return 8;
-    case 2: return 32;
+    case 2: return per_warp >= 32 ? 32 : (per_warp >= 1 ? 16 : 8);
     case 3: return 2;
     default: break;
   }
@@ -504,8 +506,13 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
       c.plan.list_cap = 2LL * 32 * rows * ((max_tasks + c.plan.grid - 1) / c.plan.grid);
       c.wide = c.plan;
       // Replica dispatch: one block per replica at a time.
-      c.local = plan_sweep(ndim, B.nx, B.ny, B.nz, v, 1, false);
-      const SweepPlan w = plan_sweep(ndim, B.nx, B.ny, B.nz, v, 1, true);
+      // Fixed rows only where every warp gets a task of them (200 replicas of up to
+      // 60^2, one MCS in 16-row tasks 178 us, in these 64), one-row tasks only
+      // where that is not what the size gives anyway.
+      const long long fixed = units(biggest, 0, 1) / kWarps2d;  // rows per warp
+      const int lv = fixed < (v == 3 ? 3 : (v == 2 ? 16 : 8)) ? 0 : v;
+      c.local = plan_sweep(ndim, B.nx, B.ny, B.nz, lv, 1, false);
+      const SweepPlan w = plan_sweep(ndim, B.nx, B.ny, B.nz, lv, 1, true);
       c.local.list_cap = std::max(c.local.list_cap, w.list_cap);
       for (int r = 0; r < n; ++r)  // (a narrower replica may have more rows)
         c.local.list_cap = std::max(c.local.list_cap, 2LL * 32 * c.local.rows *

@@ -502,8 +502,9 @@ class _Engine:
 
     def set_variant(self, variant):
         """Target rows of a warp task (32 columns wide): 0 = by the lattice's
-        size, 1 = 8, 2 = 16 (a batch: 32), 3 = 1 (a batch: 2).  The result
-        does not depend on it."""
+        size, 1 = 8, 2 = 16 (a batch: 32), 3 = 1 (a batch: 2); batches of small
+        replicas take fewer, runs with act or persistence those of 0.  The
+        result does not depend on it."""
         self._call("cpm_set_variant", int(variant))
 
     def set_dispatch(self, dispatch):
