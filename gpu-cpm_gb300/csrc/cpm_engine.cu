@@ -956,13 +956,6 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
                           int* nlaunch) {
   const cpm_handle::Config& c = h->cfg[v];
   *nlaunch = 0;
-  if (h->act_active && h->d_lat2) {  // both lattice and stamp copies start equal
-    const size_t b = sizeof(uint32_t) * h->total_sites;
-    cudaError_t e = cudaMemcpyAsync(h->d_lat2, h->d_lat, b, cudaMemcpyDeviceToDevice, h->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h->d_act2, h->d_act, b, cudaMemcpyDeviceToDevice, h->stream);
-    if (e != cudaSuccess) return e;
-  }
   auto one = [&](SweepArgs x, const SweepPlan& p, bool batch) {
     cudaError_t e;
     if (uses_cluster(h) && !scores) {  // (no grid barrier, no queue)
@@ -970,6 +963,13 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
       e = launch_cluster_sweep(x, R.nx, R.ny, R.ncells, h->cluster_blocks, h->stream);
     } else {
       e = cudaMemsetAsync(h->d_ctl, 0, sizeof(uint32_t) * kCtlErr, h->stream);
+      if (x.lat2) {  // both lattice and stamp copies start equal
+        const size_t b = sizeof(uint32_t) * h->total_sites;
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(x.lat2, x.lat, b, cudaMemcpyDeviceToDevice, h->stream);
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(x.act2, x.act, b, cudaMemcpyDeviceToDevice, h->stream);
+      }
       if (e != cudaSuccess) return e;
       x.rows = p.rows;
       x.kr = p.kr;
@@ -999,6 +999,10 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
   if (ng < h->nrep) {  // replica dispatch over the rest
     SweepArgs q = a;
     q.block_local = 1;
+    // Act: one copy, as the second barrier of a phase is only the block's (us,
+    // two copies / one: 40 x 64^2, 10 MCS 363 / 335, 160 x 64^2 621 / 581, and two
+    // almost frozen lattices of 1,700 sites, one MCS 68 / 54).
+    q.lat2 = q.act2 = nullptr;
     q.rep_order = h->d_rep_order + ng;
     q.queue_len = h->nrep - ng;
     if (cudaError_t e = one(q, c.local, false)) return e;

@@ -229,10 +229,11 @@ struct SweepArgs {
   // `pend` (two lists per block: site low, site high, value, stamp); the next
   // phase replays them into the copy they missed.  Both copies are equal
   // before and after a launch.
-  // Where the second copies do not fit in memory (16 bytes a site of copies and
-  // lists in 2D, against 3) lat2 is null: the blocks list their copies in `pend`
-  // (64-bit sites of all blocks, then 32-bit values) and make them after the
-  // phase, behind a second barrier.  Two copies / one (us): 20 MCS of 64^2 598 /
+  // In replica dispatch, whose barriers are a block's, and where the second
+  // copies do not fit in memory (16 bytes a site of copies and lists in 2D,
+  // against 3) lat2 is null: the blocks list their copies in `pend` (64-bit sites
+  // of all blocks, then 32-bit values) and make them after the phase, behind a
+  // second barrier.  Two copies / one in grid dispatch (us): 20 MCS of 64^2 598 /
   // 668, of 1024^2 1175 / 1249, of 64^3 785 / 856; one MCS of 4096^2, where
   // starting with equal copies is more of it, 806 / 742.
   uint32_t* act;
