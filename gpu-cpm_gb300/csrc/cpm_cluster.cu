@@ -24,8 +24,10 @@
 //    (distributed shared memory), its loads in flight over the phase's queueing,
 //    and applies it to the block's tables.  So tables are as they stood when
 //    the phase began when its attempts read them, without a second copy or a
-//    replay.  (Rows dealt over the blocks, read and changed by their owner
-//    only, need a second cluster barrier per phase: 14.8 ms against 11.4.)
+//    replay.  Where whole tables do not fit, their rows are dealt over the
+//    blocks (DEALT), changed by their owner and read from it, which needs a
+//    second cluster barrier per phase: 256^2 of 6,000 rows, 50 MCS 743 us, of
+//    5,000 in whole tables 568.
 //  * Phases end at the cluster's hardware barrier (509 cycles; with the tables
 //    in global memory it waited for the reductions too, 2,019).
 // The block's attempts are queued together and evaluated on two lanes each
@@ -65,17 +67,20 @@ struct ClusterPlan {
   int pitch;        // words of a strip row: nx + 2
   int cap;          // targets of a block in a phase at most
   int rows;         // table rows
+  int dealt;        // log2 G where the rows are dealt over the blocks, else 0
   FastDiv div_pitch;  // by pitch
   unsigned off_cs, off_ap, off_queue, off_out, off_pos, bytes;
 };
 
-ClusterPlan make_plan(int nx, int ny, int ncells, int G) {
+ClusterPlan make_plan(int nx, int ny, int ncells, int G, bool dealt) {
   ClusterPlan p;
   p.G = G;
   p.H = (ny + G - 1) / G;
   p.pitch = nx + 2;
   p.cap = (p.H / 2 + 1) * std::max(1, nx / 2);
   p.rows = ncells + 1;
+  p.dealt = !dealt ? 0 : (G == 16 ? 4 : 3);
+  const unsigned long long here = dealt ? (p.rows + G - 1) / G : p.rows;  // rows of a block
   p.div_pitch = fast_div_of((uint32_t)p.pitch);
   unsigned long long at = 0;
   auto take = [&](unsigned long long n) {
@@ -84,8 +89,8 @@ ClusterPlan make_plan(int nx, int ny, int ncells, int G) {
     return (unsigned)std::min<unsigned long long>(o, 0xFFFFFFF0u);
   };
   take(4ull * (p.H + 2) * p.pitch);
-  p.off_cs = take(16ull * p.rows);
-  p.off_ap = take(8ull * p.rows);
+  p.off_cs = take(16 * here);
+  p.off_ap = take(8 * here);
   p.off_queue = take(16ull * p.cap);
   p.off_out = take(2 * 16ull * p.cap);  // two 8-byte messages a copy
   p.off_pos = take(8ull * p.cap);
@@ -110,6 +115,14 @@ __device__ __forceinline__ uint2 ld_cluster2(uint32_t addr) {
   uint2 v;
   asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];"
                : "=r"(v.x), "=r"(v.y)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ longlong2 ld_cluster2l(uint32_t addr) {
+  longlong2 v;
+  asm volatile("ld.shared::cluster.v2.u64 {%0, %1}, [%2];"
+               : "=l"(v.x), "=l"(v.y)
                : "r"(addr)
                : "memory");
   return v;
@@ -157,6 +170,9 @@ struct ClusterSlot {
   int column;    // the slot's targets are one column (class 2 in x)
 };
 
+// DEALT: row r of the tables is kept by block r % G alone, at r / G, where whole
+// tables do not fit (in 256^2, more than 5,700 rows).
+template <bool DEALT>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     cluster_sweep_kernel(const __grid_constant__ SweepArgs a,
                          const __grid_constant__ ClusterPlan pl) {
@@ -203,11 +219,14 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       strip[i] = __ldcg(L + (long long)gy * nx + gx);
     }
   }
-  for (int c = tid; c < pl.rows; c += kClusterThreads) {
-    const unsigned long long w = __ldcg(a.ap[0] + cell_off + c);
+  // (the block's rows of the tables: local row c is row c * stride + first)
+  const int stride = DEALT ? pl.G : 1, first_row = DEALT ? rank : 0;
+  for (int c = tid; c * stride + first_row < pl.rows; c += kClusterThreads) {
+    const long long row = cell_off + c * stride + first_row;
+    const unsigned long long w = __ldcg(a.ap[0] + row);
     t_ap[c] = make_int2(unpack_area(w), unpack_perim(w));
-    t_cs[c].x = __ldcg(a.cs[0] + 2 * (cell_off + c));
-    t_cs[c].y = __ldcg(a.cs[0] + 2 * (cell_off + c) + 1);
+    t_cs[c].x = __ldcg(a.cs[0] + 2 * row);
+    t_cs[c].y = __ldcg(a.cs[0] + 2 * row + 1);
   }
   for (int i = tid; i < kMaxTypes * kMaxTypes; i += kClusterThreads)
     s_J[(i / kMaxTypes) * kJPitch + i % kMaxTypes] = __ldg(&P->J[i]);
@@ -264,7 +283,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   // 2 bits each), side (1: the cell lost the site).  y: site x (12 bits),
   // site y (12 bits), perimeter change + 8.
   auto apply = [&](const uint2& m) {
-    const unsigned id = m.x & 0xFFFFFFu;
+    unsigned id = m.x & 0xFFFFFFu;
+    if (DEALT) {
+      if ((id & (unsigned)(pl.G - 1)) != (unsigned)rank) return;
+      id >>= pl.dealt;
+    }
     const int sign = (m.x >> 28) & 1u ? -1 : 1;
     atomicAdd(&t_ap[id].x, sign);
     atomicAdd(&t_ap[id].y, (int)(m.y >> 24) - 8);
@@ -312,8 +335,18 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       const uint32_t own = side ? t : s;
       const unsigned id = own & 0xFFFFFFu;
       const int type = (int)(own >> 24) & (kMaxTypes - 1);
-      const int2 ap = t_ap[id];
-      const longlong2 cs = t_cs[id];
+      int2 ap;
+      longlong2 cs;
+      if constexpr (DEALT) {
+        const int owner = (int)(id & (unsigned)(pl.G - 1));
+        const unsigned at = id >> pl.dealt;
+        const uint2 v = ld_cluster2(map_rank(smem_addr(t_ap + at), owner));
+        ap = make_int2((int)v.x, (int)v.y);
+        cs = ld_cluster2l(map_rank(smem_addr(t_cs + at), owner));
+      } else {
+        ap = t_ap[id];
+        cs = t_cs[id];
+      }
       const TypeParams tp = s_type[type];
       uint32_t nb[9];
 #pragma unroll
@@ -481,7 +514,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         }
       }
       if (step > 0) apply_fetched(prv);
-      __syncthreads();  // tables as of the phase's start, queue complete
+      // tables as of the phase's start (DEALT: in every block), queue complete
+      if (DEALT && step > 0)
+        cluster.sync();
+      else
+        __syncthreads();
       const int nq = (int)s_qn[cur];
       for (int b = warp * 16; b < nq; b += kClusterThreads / 2) {
         const int i = b + (lane >> 1);
@@ -520,13 +557,17 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     const int r = i / nx, c = i - r * nx;
     L[(long long)(row0 + r) * nx + c] = strip[(r + 1) * sp + 1 + c];
   }
-  for (int c = rank * kClusterThreads + tid; c < pl.rows; c += pl.G * kClusterThreads) {
+  // (whole tables: each block writes its share of the rows)
+  const int c0 = DEALT ? tid : rank * kClusterThreads + tid;
+  for (int c = c0; c * stride + first_row < pl.rows;
+       c += DEALT ? kClusterThreads : pl.G * kClusterThreads) {
+    const long long row = cell_off + c * stride + first_row;
     const unsigned long long w = pack_delta(t_ap[c].x, t_ap[c].y);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      a.ap[b][cell_off + c] = w;
-      a.cs[b][2 * (cell_off + c)] = t_cs[c].x;
-      a.cs[b][2 * (cell_off + c) + 1] = t_cs[c].y;
+      a.ap[b][row] = w;
+      a.cs[b][2 * row] = t_cs[c].x;
+      a.cs[b][2 * row + 1] = t_cs[c].y;
     }
   }
 }
@@ -552,8 +593,11 @@ cudaLaunchConfig_t cluster_config(const ClusterPlan& p, cudaStream_t s,
 // function on the device, and engines in other threads set it too.
 constexpr int kClusterSmemMax = kSweepSmemMax - 8 * 1024;
 
-cudaError_t cluster_attributes() {
-  const void* fn = (const void*)cluster_sweep_kernel;
+const void* cluster_fn(bool dealt) {
+  return dealt ? (const void*)cluster_sweep_kernel<true> : (const void*)cluster_sweep_kernel<false>;
+}
+
+cudaError_t cluster_attributes(const void* fn) {
   cudaError_t e =
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
   if (e == cudaSuccess)
@@ -563,18 +607,17 @@ cudaError_t cluster_attributes() {
 
 }  // namespace
 
-int cluster_sweep_blocks(int nx, int ny, int ncells) {
+int cluster_sweep_blocks(int nx, int ny, int ncells, bool dealt) {
   if (nx < 4 || nx > 0xFFF || ny > 0xFFF) return 0;  // (12-bit coordinates in messages)
+  const void* fn = cluster_fn(dealt);
   for (int G : {16, 8}) {
-    const ClusterPlan p = make_plan(nx, ny, ncells, G);
+    const ClusterPlan p = make_plan(nx, ny, ncells, G, dealt);
     if (p.bytes > (unsigned)kClusterSmemMax) continue;
     cudaLaunchAttribute attr[1];
     int n = 0;
-    if (cluster_attributes() == cudaSuccess) {
+    if (cluster_attributes(fn) == cudaSuccess) {
       const cudaLaunchConfig_t cfg = cluster_config(p, nullptr, attr);
-      if (cudaOccupancyMaxActiveClusters(&n, (const void*)cluster_sweep_kernel, &cfg) !=
-          cudaSuccess)
-        n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) n = 0;
     }
     cudaGetLastError();  // (a refused size is not an error of the engine)
     if (n >= 1) return G;
@@ -585,14 +628,15 @@ int cluster_sweep_blocks(int nx, int ny, int ncells) {
 int cluster_sweep_threads() { return kClusterThreads; }
 
 cudaError_t launch_cluster_sweep(const SweepArgs& a, int nx, int ny, int ncells, int G,
-                                 cudaStream_t s) {
-  ClusterPlan p = make_plan(nx, ny, ncells, G);
-  const cudaError_t e = cluster_attributes();
+                                 bool dealt, cudaStream_t s) {
+  const void* fn = cluster_fn(dealt);
+  ClusterPlan p = make_plan(nx, ny, ncells, G, dealt);
+  const cudaError_t e = cluster_attributes(fn);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<SweepArgs*>(&a), &p};
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = cluster_config(p, s, attr);
-  return cudaLaunchKernelExC(&cfg, (const void*)cluster_sweep_kernel, args);
+  return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 }  // namespace gpucpm

@@ -185,6 +185,7 @@ struct cpm_handle {
   enum { kBySize, kByTuner, kByCaller } fill_by = kBySize;
   bool row_ok = false, cluster_shape = false;
   int cluster_blocks = 0;  // blocks of the cluster that holds the lattice (0: none)
+  bool cluster_dealt = false;  // with the tables' rows dealt over them
   std::vector<unsigned long long> attempts;  // per replica, host-counted
 
   // Graph-captured run (cpm_run_graph): the captured launch reads and
@@ -425,7 +426,13 @@ int build_engine(int n, int ndim, const int* nx, const int* ny, const int* nz,
     h->fill = CPM_FILL_TMA;
     if (ndim == 2) h->cluster_shape = cluster_rows_fit(nx[0], ny[0]);
   }
-  if (n == 1 && ndim == 2) h->cluster_blocks = cluster_sweep_blocks(nx[0], ny[0], ncells[0]);
+  if (n == 1 && ndim == 2) {
+    h->cluster_blocks = cluster_sweep_blocks(nx[0], ny[0], ncells[0], false);
+    if (h->cluster_blocks == 0) {
+      h->cluster_blocks = cluster_sweep_blocks(nx[0], ny[0], ncells[0], true);
+      h->cluster_dealt = h->cluster_blocks > 0;
+    }
+  }
 
   // One launch configuration per tile variant: warp tasks per slot and
   // replica (prefix over replicas), grid, dirty-list capacity.
@@ -941,10 +948,23 @@ int fill_key(const cpm_handle* h) { return h->fill_by == cpm_handle::kBySize ? -
 // 330^2 18.6 / 19.9, 4000 x 16 18.3 / 20.4, 100 x 1300 18.7 / 21.0, but 16 x 4000
 // 18.0 / 11.8, 2000 x 32 18.4 / 12.4, 4095 x 5 32.2 / 26.1).
 constexpr long long kClusterAutoSites = 140000;
+// Where a block cannot hold whole tables they are dealt over the blocks, at a
+// second cluster barrier per phase: by the autotuner's choice, or where the
+// caller asks for the cluster on lattices so small that it is the faster one
+// (us of 20 MCS, grid / dealt, cells of 2 sites and of 25 with 16,000 rows to
+// spare: 120 x 173 580 / 371, 532 / 334; 160^2 426 / 310, 396 / 254; 200^2 434 /
+// 446, 408 / 310; 256^2 437 / 522, 411 / 421; before, with tables in global memory,
+// 200^2 485 and 373).
+constexpr long long kClusterDealtSites = 45000;
 bool uses_cluster(const cpm_handle* h) {
-  return h->cluster_blocks > 0 && !h->act_active && !h->persist_active &&
-         (h->fill_by == cpm_handle::kBySize ? h->total_sites <= kClusterAutoSites
-                                            : h->fill == CPM_FILL_CLUSTER);
+  if (h->cluster_blocks == 0 || h->act_active || h->persist_active) return false;
+  switch (h->fill_by) {
+    case cpm_handle::kBySize: return !h->cluster_dealt && h->total_sites <= kClusterAutoSites;
+    case cpm_handle::kByTuner: return h->fill == CPM_FILL_CLUSTER;
+    default:
+      return h->fill == CPM_FILL_CLUSTER &&
+             (!h->cluster_dealt || h->total_sites <= kClusterDealtSites);
+  }
 }
 
 // The launches of one sweep run (`a` from sweep_args, times filled in): one
@@ -960,7 +980,8 @@ cudaError_t enqueue_sweep(const cpm_handle* h, int v, int d, const SweepArgs& a,
     cudaError_t e;
     if (uses_cluster(h) && !scores) {  // (no grid barrier, no queue)
       const DevReplica& R = h->reps[0];
-      e = launch_cluster_sweep(x, R.nx, R.ny, R.ncells, h->cluster_blocks, h->stream);
+      e = launch_cluster_sweep(x, R.nx, R.ny, R.ncells, h->cluster_blocks, h->cluster_dealt,
+                               h->stream);
     } else {
       e = cudaMemsetAsync(h->d_ctl, 0, sizeof(uint32_t) * kCtlErr, h->stream);
       if (x.lat2) {  // both lattice and stamp copies start equal
@@ -1669,7 +1690,8 @@ int cpm_autotune(cpm_handle* h, int probe_mcs, int* chosen, float* ms_per_mcs) {
   h->variant = best_v;
   h->variant_ext = h->act_active || h->persist_active;
   h->dispatch = best_d;
-  if (try_cluster && (fill_by == cpm_handle::kBySize || best_fill != fill)) {
+  if (try_cluster && (fill_by == cpm_handle::kBySize || best_fill != fill ||
+                      best_fill == CPM_FILL_CLUSTER)) {
     h->fill = best_fill;
     h->fill_by = cpm_handle::kByTuner;
   }

@@ -277,11 +277,12 @@ cudaError_t launch_sweep2d(const SweepArgs& a, bool batch, bool scores, int grid
                            cudaStream_t s);
 cudaError_t launch_sweep3d(const SweepArgs& a, bool batch, int grid, int warps, cudaStream_t s);
 // Cluster sweep of a small single 2D lattice (cpm_cluster.cu): blocks of the
-// cluster that can hold it with its tables (0: none), and launch.
-int cluster_sweep_blocks(int nx, int ny, int ncells);
+// cluster that can hold it with its tables (0: none), and launch.  dealt: the
+// tables' rows are dealt over the blocks instead of kept by each.
+int cluster_sweep_blocks(int nx, int ny, int ncells, bool dealt);
 int cluster_sweep_threads();
 cudaError_t launch_cluster_sweep(const SweepArgs& a, int nx, int ny, int ncells, int G,
-                                 cudaStream_t s);
+                                 bool dealt, cudaStream_t s);
 // checkpoints: host array of ncheck (<= kMaxCheckpoints) MCS counts.
 cudaError_t launch_lr_backward(const float* scores, const float* dl_do,
                                const float* obs, const int* checkpoints, int nrep,

@@ -345,9 +345,12 @@ int cpm_sweep_config(const cpm_handle* h, int* variant, int* tile_x,
  * CPM_FILL_VECTOR and CPM_FILL_TMA need a single lattice with nx a multiple of
  * 4 and nx >= 72 (in 2D ny >= 66, in 3D ny >= 18 and nz >= 18), for which
  * CPM_FILL_TMA is reported.  CPM_FILL_CLUSTER needs a 2D one that fits a
- * cluster with its tables (up to about 400^2); it is also accepted, and the
- * sweep over the whole GPU runs, for shapes that VECTOR and TMA accept and whose
- * rows alone fit (about 190 KB of them per block of 16).
+ * cluster with its tables, whole ones in every block (up to about 400^2) or dealt
+ * over the blocks; with dealt tables on more than 45,000 sites the sweep over
+ * the whole GPU runs all the same, unless cpm_autotune found the cluster faster.
+ * It is also accepted, and the sweep over the whole GPU runs, for shapes that
+ * VECTOR and TMA accept and whose rows alone fit (about 190 KB of them per block
+ * of 16).
  * cpm_running_fill tells which sweep plain runs take as things stand:
  * CPM_FILL_CLUSTER, or for the sweep over the whole GPU the name that was set
  * for it, CPM_FILL_PARITY where none was.
