@@ -235,10 +235,13 @@ namespace {
 
 // Entry points that touch the GPU make the handle's device current first:
 // the library carries its own CUDA runtime, whose current device is not the
-// one a caller (torch, another library) selected.
+// one a caller (torch, another library) selected.  What an earlier call of this
+// thread failed with (an allocation refused to another engine, say) was
+// reported then and is forgotten: the launchers return cudaGetLastError().
 #define CPM_BIND(h)                                   \
   do {                                                \
     if (!(h)) return CPM_ERR_INVALID;                 \
+    cudaGetLastError();                               \
     CPM_CUDA((h), cudaSetDevice((h)->device));        \
   } while (0)
 
@@ -1962,6 +1965,7 @@ int cpm_lr_backward(const float* scores, const float* dl_do, const float* obs,
     g_create_error = "cpm_lr_backward: bad arguments";
     return CPM_ERR_INVALID;
   }
+  cudaGetLastError();  // (of an earlier call, see CPM_BIND)
   cudaError_t e = launch_lr_backward(scores, dl_do, obs, checkpoints, nrep, len, nparam,
                                      ncheck, obs_total, nrep_total, grad,
                                      (cudaStream_t)stream);

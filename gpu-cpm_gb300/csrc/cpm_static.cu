@@ -180,6 +180,7 @@ extern "C" int cpm_sweep_static(int dimensionality, int nx, int ny, int nz,
       a.slots[a.nslot_active++] = slot;
   }
   int dev = 0, sms = 0;
+  cudaGetLastError();  // (of an earlier call: the launchers return it)
   STATIC_CUDA(cudaGetDevice(&dev));
   STATIC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const bool perim_on = [&] {
